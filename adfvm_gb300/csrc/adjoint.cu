@@ -70,20 +70,20 @@ __device__ __forceinline__ void adj_face(const MeshDev<R>& m, const Phys& P, con
     stage_row<R, FADJ>(row, v);
 }
 
-template <typename R, typename S, bool TAPED>
-__global__ void __launch_bounds__(FLUX_BLOCK, sizeof(R) == 8 ? 3 : 5) k_adj_flux(MeshDev<R> m, Phys P, const R* __restrict__ rec, R coef,
+template <typename R, typename S, bool TAPED, int NT>
+__global__ void __launch_bounds__(NT, (sizeof(R) == 8 ? 3 : 5) * FLUX_BLOCK / NT) k_adj_flux(MeshDev<R> m, Phys P, const R* __restrict__ rec, R coef,
                                                     const S* __restrict__ ar, const S* __restrict__ au,
                                                     const S* __restrict__ ae, R* __restrict__ fadj, int inviscid,
                                                     const R* __restrict__ tape) {
     // the block's 40-value face records are staged here and written out contiguously: one
     // thread's 40 scalar stores at a 40-value stride would touch a new 32-byte sector each and
     // load L2 with eight partial writes per sector
-    __shared__ __align__(16) R stage[FLUX_BLOCK * FADJ];
-    const int f0 = blockIdx.x * FLUX_BLOCK;
+    __shared__ __align__(16) R stage[NT * FADJ];
+    const int f0 = blockIdx.x * NT;
     const int f = f0 + threadIdx.x;
     if (f < m.nF) adj_face<R, S, TAPED>(m, P, rec, coef, ar, au, ae, inviscid, f, stage + threadIdx.x * FADJ, tape);
     __syncthreads();
-    store_staged<R, FADJ, FLUX_BLOCK>(fadj, f0, min(FLUX_BLOCK, m.nF - f0), stage);
+    store_staged<R, FADJ, NT>(fadj, f0, min(NT, m.nF - f0), stage);
 }
 
 // one cell's sum of its faces' adjoint records (and of the ghosts whose gradient is its own)
@@ -113,14 +113,14 @@ __device__ __forceinline__ void adj_cell_gather(const MeshDev<R>& m, const R* __
     stage_row<R, CBAR>(row, acc);
 }
 
-template <typename R>
-__global__ void __launch_bounds__(BLOCK) k_adj_cell1(MeshDev<R> m, const R* __restrict__ fadj, R* __restrict__ cbar) {
-    __shared__ __align__(16) R stage[BLOCK * CBAR];
-    const int c0 = blockIdx.x * BLOCK;
+template <typename R, int NT>
+__global__ void __launch_bounds__(NT) k_adj_cell1(MeshDev<R> m, const R* __restrict__ fadj, R* __restrict__ cbar) {
+    __shared__ __align__(16) R stage[NT * CBAR];
+    const int c0 = blockIdx.x * NT;
     const int c = c0 + threadIdx.x;
     if (c < m.nIC) adj_cell_gather<R>(m, fadj, c, stage + threadIdx.x * CBAR);
     __syncthreads();
-    if (c0 < m.nIC) store_staged<R, CBAR, BLOCK>(cbar, c0, min(BLOCK, m.nIC - c0), stage);
+    if (c0 < m.nIC) store_staged<R, CBAR, NT>(cbar, c0, min(NT, m.nIC - c0), stage);
 }
 
 
@@ -359,7 +359,7 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
     R* fadj = (R*)c->fadj;
     R* cbar = (R*)c->cbar;
     S* sb = (S*)c->sbar;
-    int nbC = nblocks(m.nIC);
+    const Shape gF = shape_for(m.nF, FLUX_BLOCK), gC = shape_for(m.nIC, BLOCK);
     const double beta[3] = {1.0, 1. / 4, 2. / 3};
     // a tape holds the stage's cell records the primal step built (no primitive or gradient
     // launches here) and, in FP64, its face tape
@@ -379,17 +379,23 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
         R coef = (R)(-beta[st] * dt);
         {
             ProfScope ps(c, KID_ADJ_FLUX, s);
-            int nbF = (m.nF + FLUX_BLOCK - 1) / FLUX_BLOCK;
-            if (faceTape)
-                k_adj_flux<R, S, true><<<nbF, FLUX_BLOCK, 0, s>>>(m, P, rec, coef, ain[0], ain[1], ain[2], fadj,
-                                                                  inviscid, faceTape + (size_t)st * TAPE * m.nF);
-            else
-                k_adj_flux<R, S, false><<<nbF, FLUX_BLOCK, 0, s>>>(m, P, rec, coef, ain[0], ain[1], ain[2], fadj,
-                                                                   inviscid, nullptr);
+            const R* ft = faceTape ? faceTape + (size_t)st * TAPE * m.nF : nullptr;
+            auto flux = [&](auto taped, auto nt) {
+                k_adj_flux<R, S, decltype(taped)::value, decltype(nt)::value><<<gF.blocks, decltype(nt)::value, 0, s>>>(
+                    m, P, rec, coef, ain[0], ain[1], ain[2], fadj, inviscid, ft);
+            };
+            using Small = std::integral_constant<int, 32>;
+            using Big = std::integral_constant<int, FLUX_BLOCK>;
+            const bool small = gF.threads == 32;
+            if (ft && small) flux(std::true_type{}, Small{});
+            else if (ft) flux(std::true_type{}, Big{});
+            else if (small) flux(std::false_type{}, Small{});
+            else flux(std::false_type{}, Big{});
         }
         {
             ProfScope ps(c, KID_ADJ_GATHER, s);
-            k_adj_cell1<R><<<nbC, BLOCK, 0, s>>>(m, fadj, cbar);
+            if (gC.threads == 32) k_adj_cell1<R, 32><<<gC.blocks, 32, 0, s>>>(m, fadj, cbar);
+            else k_adj_cell1<R, BLOCK><<<gC.blocks, BLOCK, 0, s>>>(m, fadj, cbar);
         }
         // the stage's share of the mesh / boundary-input gradients (before the cell kernel: the
         // adjoint outputs it writes may alias this stage's input adjoints)
@@ -397,21 +403,21 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
             if (params) launch_param_grads<R, S>(c, *params, rec, coef, ain[0], ain[1], ain[2], st == 1, obja, s);
         ProfScope ps(c, KID_ADJ_GRAD, s);
         if (st == 2)
-            k_adj_cell2<R, S, 2><<<nbC, BLOCK, 0, s>>>(m, P, rec, fadj, cbar, u[0], u[1], u[2], ain[0], ain[1], ain[2],
+            k_adj_cell2<R, S, 2><<<gC.blocks, gC.threads, 0, s>>>(m, P, rec, fadj, cbar, u[0], u[1], u[2], ain[0], ain[1], ain[2],
                                                     A2[0], A2[1], A2[2], rhoa, rhoUa, rhoEa, sb, dt, c->objective,
                                                     c->objStart, c->objN, obja, c->vane, c->objSeed);
         else if (st == 1)
-            k_adj_cell2<R, S, 1><<<nbC, BLOCK, 0, s>>>(m, P, rec, fadj, cbar, u[0], u[1], u[2], ain[0], ain[1], ain[2],
+            k_adj_cell2<R, S, 1><<<gC.blocks, gC.threads, 0, s>>>(m, P, rec, fadj, cbar, u[0], u[1], u[2], ain[0], ain[1], ain[2],
                                                     A1[0], A1[1], A1[2], rhoa, rhoUa, rhoEa, sb, dt, c->objective,
                                                     c->objStart, c->objN, obja, c->vane, c->objSeed);
         else
-            k_adj_cell2<R, S, 0><<<nbC, BLOCK, 0, s>>>(m, P, rec, fadj, cbar, u[0], u[1], u[2], ain[0], ain[1], ain[2],
+            k_adj_cell2<R, S, 0><<<gC.blocks, gC.threads, 0, s>>>(m, P, rec, fadj, cbar, u[0], u[1], u[2], ain[0], ain[1], ain[2],
                                                     nullptr, nullptr, nullptr, rhoa, rhoUa, rhoEa, sb, dt,
                                                     c->objective, c->objStart, c->objN, obja, c->vane, c->objSeed);
     }
     if (Srhoa || SrhoUa || SrhoEa) {
         ProfScope ps(c, KID_ADJ_MISC, s);
-        k_split5<S><<<nbC, BLOCK, 0, s>>>(m.nIC, sb, Srhoa, SrhoUa, SrhoEa);
+        k_split5<S><<<gC.blocks, gC.threads, 0, s>>>(m.nIC, sb, Srhoa, SrhoUa, SrhoEa);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "adjoint step launch");

@@ -433,7 +433,8 @@ int alloc_work(Ctx* c) {
     }
     if ((st = dalloc(c, &c->zeroS, sizeof(S) * n * 5))) return st;
     cudaMemset(c->zeroS, 0, sizeof(S) * n * 5);
-    int np = (int)((std::max(c->nIC, c->nF) + BLOCK - 1) / BLOCK);
+    // one partial sum a block: of the largest grid, or of a small grid's one-warp blocks
+    int np = std::max(nblocks(std::max(c->nIC, c->nF)), SMALL_WARPS);
     c->nPartials = np;
     if ((st = dalloc(c, (void**)&c->partials, sizeof(double) * (size_t)np))) return st;
     if ((st = dalloc(c, (void**)&c->scal, sizeof(double) * 8))) return st;

@@ -18,6 +18,18 @@ constexpr int BLOCK = 256;
 // 0.217 ms, FP32 k_adj_flux 0.471 (4 blocks) -> 0.445 (5) / 0.456 ms (6).
 constexpr int FLUX_BLOCK = 128;
 
+// Small meshes: an FP64 warp instruction takes 64 cycles of its SM sub-partition, so a small
+// grid's time is the instruction chain of one warp times the warps that share a sub-partition,
+// and 256-thread blocks put eight on one SM while others have none (k_grad of 1,000 FP64 cells:
+// 4 blocks, 13 us). Grids of at most SMALL_WARPS warps - eight a sub-partition, 4 x 152 of
+// them - run one-warp blocks, which spread over all SMs. Measured limits of 1, 4, 8 and 16 warps
+// a sub-partition: 40 steps of the 1,000-cell FP64 tube 4.04 / 4.08 / 4.08 / 4.08 ms (5.25 with
+// 128 and 256 threads), the 256x128 cylinder's mixed step and adjoint 297 / 280 / 269 / 271 us
+// (300), ten steps of a 128x64 cylinder's FP64 sweep 6.04 / 6.0 / 5.92 / 5.98 ms (6.82); above
+// the limit nothing changes.
+constexpr int SMALL_WARPS = 8 * 4 * 152;
+static inline bool small_grid(long long n) { return n <= 32LL * SMALL_WARPS; }
+
 // Block-staged record stores. A thread that stores its own W-value record at a W-value stride
 // makes each scalar store a separate L2 write request into a partly written sector; instead
 // each thread writes its record into the block's shared-memory stage (stage_row: 16-byte
@@ -297,6 +309,16 @@ void default_sources(Ctx* c, const S*& Srho, const S*& SrhoU, const S*& SrhoE);
 int host_copy(int32_t device, void* dst, int32_t dstBytes, const void* src, int32_t srcBytes, int64_t count,
               void* stream, bool toDevice, bool syncPinned);
 static inline int nblocks(long long n) { return (int)((n + BLOCK - 1) / BLOCK); }
+
+// Launch shape of a kernel with one thread per item: `big` threads a block, or one warp a block
+// for a small grid.
+struct Shape {
+    int blocks, threads;
+};
+static inline Shape shape_for(long long n, int big) {
+    const int t = small_grid(n) ? 32 : big;
+    return {(int)((n + t - 1) / t), t};
+}
 
 // rows of U (3), T, p with absolute T and p from FP32 records (stride values apart), which
 // hold the gauge offsets of T and p

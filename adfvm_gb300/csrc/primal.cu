@@ -106,7 +106,7 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     __syncthreads();
     double r = 0.0;
     if (threadIdx.x < 32) {
-        r = (threadIdx.x < BLOCK / 32) ? sh[threadIdx.x] : 0.0;
+        r = (threadIdx.x < blockDim.x / 32) ? sh[threadIdx.x] : 0.0;
         for (int off = 16; off > 0; off >>= 1) r += __shfl_down_sync(0xffffffffu, r, off);
     }
     return r;
@@ -215,14 +215,23 @@ __device__ __forceinline__ void grad_cell(const MeshDev<R>& m, const Phys& P, co
 // are rewritten: the rewrite stores the bits already there (each cell's primitives are read
 // from its own record and written back unchanged), so every read sees the same value whether
 // it lands before or after the store.
-template <typename R>
-__global__ void __launch_bounds__(BLOCK) k_grad(MeshDev<R> m, Phys P, R* __restrict__ rec) {
-    __shared__ __align__(16) R stage[BLOCK * REC];
-    const int c0 = blockIdx.x * BLOCK;
+template <typename R, int NT>
+__global__ void __launch_bounds__(NT) k_grad(MeshDev<R> m, Phys P, R* __restrict__ rec) {
+    __shared__ __align__(16) R stage[NT * REC];
+    const int c0 = blockIdx.x * NT;
     const int c = c0 + threadIdx.x;
     if (c < m.nIC) grad_cell<R>(m, P, rec, c, stage + threadIdx.x * REC);
     __syncthreads();
-    if (c0 < m.nIC) store_staged<R, REC, BLOCK>(rec, c0, min(BLOCK, m.nIC - c0), stage);
+    if (c0 < m.nIC) store_staged<R, REC, NT>(rec, c0, min(NT, m.nIC - c0), stage);
+}
+
+template <typename R>
+static void launch_grad(Ctx* c, R* rec, cudaStream_t s) {
+    const MeshDev<R>& m = meshOf<R>(c);
+    ProfScope ps(c, KID_GRAD, s);
+    const Shape g = shape_for(m.nIC, BLOCK);
+    if (g.threads == 32) k_grad<R, 32><<<g.blocks, 32, 0, s>>>(m, c->phys, rec);
+    else k_grad<R, BLOCK><<<g.blocks, BLOCK, 0, s>>>(m, c->phys, rec);
 }
 
 
@@ -376,7 +385,7 @@ __global__ void __launch_bounds__(BLOCK) k_update(MeshDev<R> m, const R* __restr
         if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = d;
         __syncthreads();
         if (threadIdx.x < 32) {
-            d = (threadIdx.x < BLOCK / 32) ? wmax[threadIdx.x] : 0.0;
+            d = (threadIdx.x < blockDim.x / 32) ? wmax[threadIdx.x] : 0.0;
             for (int off = 16; off > 0; off >>= 1) d = nan_max(d, __shfl_down_sync(0xffffffffu, d, off));
             if (threadIdx.x == 0) atomicMax(dtcBits, (unsigned long long)__double_as_longlong(d));
         }
@@ -507,7 +516,8 @@ template <typename R, typename S>
 void launch_prim(Ctx* c, const S* r, const S* ru, const S* re, cudaStream_t s, R* rec) {
     const MeshDev<R>& m = meshOf<R>(c);
     ProfScope ps(c, KID_PRIM, s);
-    k_prim<R, S><<<nblocks(m.nIC + m.nG), BLOCK, 0, s>>>(m, c->phys, r, ru, re, rec ? rec : (R*)c->rec);
+    const Shape g = shape_for((long long)m.nIC + m.nG, BLOCK);
+    k_prim<R, S><<<g.blocks, g.threads, 0, s>>>(m, c->phys, r, ru, re, rec ? rec : (R*)c->rec);
 }
 
 template <typename R, typename S>
@@ -515,10 +525,7 @@ void launch_prim_grad(Ctx* c, const S* r, const S* ru, const S* re, cudaStream_t
     const MeshDev<R>& m = meshOf<R>(c);
     if (!rec) rec = (R*)c->rec;
     launch_prim<R, S>(c, r, ru, re, s, rec);
-    {
-        ProfScope ps(c, KID_GRAD, s);
-        k_grad<R><<<nblocks(m.nIC), BLOCK, 0, s>>>(m, c->phys, rec);
-    }
+    launch_grad<R>(c, rec, s);
 }
 
 // faces -> fluxes, then the gather + stage update u_{st+1} = ... (timestep.py:35-45)
@@ -533,29 +540,30 @@ void launch_flux_update(Ctx* c, int st, double dt, const double* dtDev, const S*
     int inviscid = (P.muModel == AFVM_MU_CONSTANT && P.mu0 == 0.0) ? 1 : 0;
     {
         ProfScope ps(c, KID_FLUX, s);
-        int nbF = (m.nF + FLUX_BLOCK - 1) / FLUX_BLOCK;
+        const Shape g = shape_for(m.nF, FLUX_BLOCK);
+        const int nbF = g.blocks;
         if (tape && st == 1)
-            k_flux<R, true, true><<<nbF, FLUX_BLOCK, 0, s>>>(m, P, rec, ff, inviscid, tape);
+            k_flux<R, true, true><<<nbF, g.threads, 0, s>>>(m, P, rec, ff, inviscid, tape);
         else if (tape)
-            k_flux<R, true, false><<<nbF, FLUX_BLOCK, 0, s>>>(m, P, rec, ff, inviscid, tape);
+            k_flux<R, true, false><<<nbF, g.threads, 0, s>>>(m, P, rec, ff, inviscid, tape);
         else if (st == 1)
-            k_flux<R, false, true><<<nbF, FLUX_BLOCK, 0, s>>>(m, P, rec, ff, inviscid, nullptr);
+            k_flux<R, false, true><<<nbF, g.threads, 0, s>>>(m, P, rec, ff, inviscid, nullptr);
         else
-            k_flux<R, false, false><<<nbF, FLUX_BLOCK, 0, s>>>(m, P, rec, ff, inviscid, nullptr);
+            k_flux<R, false, false><<<nbF, g.threads, 0, s>>>(m, P, rec, ff, inviscid, nullptr);
     }
-    int nb = nblocks(m.nIC);
+    const Shape g = shape_for(m.nIC, BLOCK);
     R* recNext = nextPrims ? (recOut ? recOut : rec) : nullptr;
     ProfScope ps(c, KID_UPDATE, s);
     if (st == 0)
-        k_update<R, S, 0><<<nb, BLOCK, 0, s>>>(m, ff, dt, dtDev, u0[0], u0[1], u0[2], nullptr, nullptr, nullptr, nullptr,
+        k_update<R, S, 0><<<g.blocks, g.threads, 0, s>>>(m, ff, dt, dtDev, u0[0], u0[1], u0[2], nullptr, nullptr, nullptr, nullptr,
                                             nullptr, nullptr, Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P,
                                             recNext, c->objective, recNext ? objPartials : nullptr);
     else if (st == 1)
-        k_update<R, S, 1><<<nb, BLOCK, 0, s>>>(m, ff, dt, dtDev, u0[0], u0[1], u0[2], u1[0], u1[1], u1[2], nullptr,
+        k_update<R, S, 1><<<g.blocks, g.threads, 0, s>>>(m, ff, dt, dtDev, u0[0], u0[1], u0[2], u1[0], u1[1], u1[2], nullptr,
                                             nullptr, nullptr, Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P,
                                             recNext, c->objective, nullptr);
     else
-        k_update<R, S, 2><<<nb, BLOCK, 0, s>>>(m, ff, dt, dtDev, u0[0], u0[1], u0[2], nullptr, nullptr, nullptr, u2[0],
+        k_update<R, S, 2><<<g.blocks, g.threads, 0, s>>>(m, ff, dt, dtDev, u0[0], u0[1], u0[2], nullptr, nullptr, nullptr, u2[0],
                                             u2[1], u2[2], Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P,
                                             recNext, c->objective, nullptr);
 }
@@ -600,8 +608,7 @@ int primal_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double d
             launch_prim_grad<R, S>(c, in[0], in[1], in[2], s, recs[0]);
         } else {
             // the primitives of stages 1 and 2 were written by the previous stage's update
-            ProfScope ps(c, KID_GRAD, s);
-            k_grad<R><<<nblocks(m.nIC), BLOCK, 0, s>>>(m, c->phys, recs[st]);
+            launch_grad<R>(c, recs[st], s);
         }
         if (st == 1 && c->objSink) {
             // the objective stage's primitives U (3), T, p of every cell, ghosts included, for an
@@ -622,17 +629,19 @@ int primal_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double d
         } else if (st == 1 && c->objective != AFVM_OBJ_NONE) {
             int start = 0, n = m.nIC;
             if (c->objective == AFVM_OBJ_DRAG) { start = c->objStart; n = c->objN; }
-            nObjBlocks = nblocks(n);
+            const Shape g = shape_for(n, BLOCK);
+            nObjBlocks = g.blocks;
             if (nObjBlocks > c->nPartials) return fail(c, AFVM_ERR_BAD_ARG, "objective partials overflow");
             // a cell-sum objective's partials were written by the stage-0 update
             if (n > 0 && !cell_sum_objective(c->objective)) {
                 ProfScope ps(c, KID_OBJECTIVE, s);
-                k_objective<R><<<nObjBlocks, BLOCK, 0, s>>>(m, P, (const R*)recs[1], c->objective, start, n,
+                k_objective<R><<<nObjBlocks, g.threads, 0, s>>>(m, P, (const R*)recs[1], c->objective, start, n,
                                                             c->partials);
             }
         }
         S* const* out = st == 0 ? u1 : (st == 1 ? u2 : outN);
-        double* objPartials = (st == 0 && cell_sum_objective(c->objective) && nblocks(m.nIC) <= c->nPartials)
+        double* objPartials = (st == 0 && cell_sum_objective(c->objective) &&
+                               shape_for(m.nIC, BLOCK).blocks <= c->nPartials)
                                   ? c->partials : nullptr;
         if (st == 0 && cell_sum_objective(c->objective) && !objPartials)
             return fail(c, AFVM_ERR_BAD_ARG, "objective partials overflow");

@@ -14,6 +14,7 @@
 //                back-slot weights, the neighbours'), ghost boundary conditions transposed,
 //                objective gradient (stage 1), primitive VJP and the SSP-RK reverse update.
 #include <cuda_runtime.h>
+#include <cmath>
 #include <type_traits>
 #include "facedev.cuh"
 #include "vane.cuh"
@@ -25,65 +26,189 @@ namespace afvm {
 constexpr int FADJ = 40;
 constexpr int CBAR = 20;   // per cell: primitive adjoint (5) then gradient adjoint (15)
 
-// one face's record of k_adj_flux into row[0..39]; TAPED: the forward values of a
-// non-boundary face come from its tape column instead of a re-evaluation of the face flux
-template <typename R, typename S, bool TAPED>
+// A face's adjoint record and forward values where the kernel keeps them.
+// RowStage: the record as a row of 40 values, the forward values read from the tape column in
+// global memory (or held in registers without a tape).
+template <typename R>
+struct RowStage {
+    R* row;
+    __device__ __forceinline__ void store(const R* v) const { stage_row<R, FADJ>(row, v); }
+};
+// ColumnStage: a column of shared memory of the thread's own (value k at col[k stride]) that
+// holds the face's TAPE forward values - copied from the tape while the seeds are gathered, or
+// written by the forward evaluation - and then, over them, the record.
+template <typename R>
+struct ColumnStage {
+    R* col;
+    static constexpr int stride = FLUX_BLOCK + 1;      // (odd: the copy-out reads rows)
+    __device__ __forceinline__ void store(const R* v) const {
+        for (int k = 0; k < FADJ; k++) col[k * stride] = v[k];
+    }
+    __device__ __forceinline__ void fetch(const R* __restrict__ tape, size_t nF) const {
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(col);
+#pragma unroll
+        for (int k = 0; k < TAPE; k++)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8 * k * stride), "l"(tape + k * nF)
+                         : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    __device__ __forceinline__ void fetched() const { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+};
+// the forward values in a ColumnStage
+template <typename R, typename Q>
+struct TapeColumn {
+    static constexpr bool kFull = true;
+    R* p;
+    unsigned* most;                // (TapeLoad)
+    __device__ __forceinline__ void put(int k, Q x) const { p[k * ColumnStage<R>::stride] = raw(x); }
+    __device__ __forceinline__ Q get(int k) const {
+        const R x = p[k * ColumnStage<R>::stride];
+        if constexpr (!std::is_same<R, Q>::value) seen_taped(*most, k, x);
+        return x;
+    }
+};
+
+// one face's record of k_adj_flux into st; TAPED: the forward values of a non-boundary face come
+// from its tape column instead of a re-evaluation of the face flux
+template <typename R, typename S, bool TAPED, typename Q, typename Stage>
 __device__ __forceinline__ void adj_face(const MeshDev<R>& m, const Phys& P, const R* __restrict__ rec, R coef,
                                          const S* __restrict__ ar, const S* __restrict__ au,
-                                         const S* __restrict__ ae, int inviscid, int f, R* row,
-                                         const R* __restrict__ tape) {
+                                         const S* __restrict__ ae, int inviscid, int f, const Stage& st,
+                                         const R* __restrict__ tape, unsigned* most = nullptr) {
+    constexpr bool COLUMN = std::is_same<Stage, ColumnStage<R>>::value;
+    // (mixed contexts keep the order their FP64 adjoints have always rounded in)
+    constexpr bool VFIRST = sizeof(R) == 4 && sizeof(S) == 8;
     int kind = (f < m.nIF) ? FACE_INTERNAL : (int)m.fkind[f - m.nIF];
+    const bool fromTape = TAPED && kind != FACE_BOUNDARY;
+    if constexpr (TAPED && COLUMN)
+        if (fromTape) st.fetch(tape + f, (size_t)m.nF);
     int iP = m.own[f];
     // Fbar = coef (abar_P A/V_L - abar_N A/V_R), coef folded into the two weights
-    R wp = coef * m.wpf[f];
-    R Fb[5];
-    Fb[0] = R(ar[iP]) * wp;
-    for (int k = 0; k < 3; k++) Fb[1 + k] = R(au[3 * iP + k]) * wp;
-    Fb[4] = R(ae[iP]) * wp;
+    Q wp = Q(coef) * Q(m.wpf[f]);
+    R aP[5] = {R(ar[iP]), R(au[3 * iP]), R(au[3 * iP + 1]), R(au[3 * iP + 2]), R(ae[iP])};
+    Q Fb[5];
+    for (int k = 0; k < 5; k++) {
+        if constexpr (!std::is_same<R, Q>::value) soft_seen(*most, aP[k]);
+        Fb[k] = Q(aP[k]) * wp;
+    }
     if (f < m.nIF) {
         int iN = m.nbr[f];
-        R wn = coef * m.wnf[f];
-        Fb[0] = Fb[0] - R(ar[iN]) * wn;
-        for (int k = 0; k < 3; k++) Fb[1 + k] = Fb[1 + k] - R(au[3 * iN + k]) * wn;
-        Fb[4] = Fb[4] - R(ae[iN]) * wn;
+        Q wn = Q(coef) * Q(m.wnf[f]);
+        R aN[5] = {R(ar[iN]), R(au[3 * iN]), R(au[3 * iN + 1]), R(au[3 * iN + 2]), R(ae[iN])};
+        for (int k = 0; k < 5; k++) {
+            if constexpr (!std::is_same<R, Q>::value) soft_seen(*most, aN[k]);
+            Fb[k] = Fb[k] - Q(aN[k]) * wn;
+        }
     }
-    FaceIn<R> in;
-    FaceBar<R> b;
+    FaceIn<Q> in;
+    FaceBar<Q> b;
     zero_bar(b);
-    if (TAPED && kind != FACE_BOUNDARY) {
-        load_face_geometry<R>(m, f, in);
-        face_vjp_t<R>(P, kind, inviscid != 0, in, TapeLoad<R>{tape + f, (size_t)m.nF}, Fb, b);
+    if (fromTape) {
+        load_face_geometry<R, Q>(m, f, in);
+        if constexpr (COLUMN) {
+            st.fetched();
+            face_vjp_t<Q, VFIRST>(P, kind, inviscid != 0, in, TapeColumn<R, Q>{st.col, most}, Fb, b);
+        } else {
+            face_vjp_t<Q, VFIRST>(P, kind, inviscid != 0, in, TapeLoad<R, Q>{tape + f, (size_t)m.nF, most}, Fb, b);
+        }
     } else {
-        load_face<R>(m, rec, f, in);
+        load_face<R, Q>(m, rec, f, in, most);
         if constexpr (kGauge<R>) {
             // the VJP differentiates the absolute-form flux (the same function of the state as
             // the gauge form the forward evaluates)
             in.TP = rec_abs_T<R>(P, in.TP); in.TN = rec_abs_T<R>(P, in.TN);
             in.pP = rec_abs_p<R>(P, in.pP); in.pN = rec_abs_p<R>(P, in.pN);
         }
-        face_vjp<R>(P, kind, inviscid != 0, in, Fb, b);
+        if constexpr (COLUMN && !TAPED) {
+            if (kind != FACE_BOUNDARY) {
+                // the forward's values through the column
+                const TapeColumn<R, Q> t{st.col, most};
+                Q F[5], maxaF;
+                face_flux<Q>(P, kind, inviscid != 0, in, F, maxaF, t);
+                face_vjp_t<Q, VFIRST>(P, kind, inviscid != 0, in, t, Fb, b);
+            } else {
+                face_vjp<Q, VFIRST>(P, kind, inviscid != 0, in, Fb, b);
+            }
+        } else {
+            face_vjp<Q, VFIRST>(P, kind, inviscid != 0, in, Fb, b);
+        }
     }
-    const R* src = &b.UP[0];
+    const Q* src = &b.UP[0];
     R v[FADJ];
-    for (int k = 0; k < 5; k++) { v[k] = src[k]; v[20 + k] = src[5 + k]; }
-    for (int k = 0; k < 15; k++) { v[5 + k] = src[10 + k]; v[25 + k] = src[25 + k]; }
-    stage_row<R, FADJ>(row, v);
+    for (int k = 0; k < 5; k++) { v[k] = raw(src[k]); v[20 + k] = raw(src[5 + k]); }
+    for (int k = 0; k < 15; k++) { v[5 + k] = raw(src[10 + k]); v[25 + k] = raw(src[25 + k]); }
+    st.store(v);
+}
+
+// the face again with the hardware's FP64 operations throughout (soft_flag)
+template <typename R, typename S, bool TAPED>
+__device__ __noinline__ void adj_face_again(const MeshDev<R>& m, const Phys& P, const R* rec, R coef, const S* ar,
+                                            const S* au, const S* ae, int inviscid, int f, ColumnStage<R> st,
+                                            const R* tape) {
+    adj_face<R, S, TAPED, R>(m, P, rec, coef, ar, au, ae, inviscid, f, st, tape);
 }
 
 template <typename R, typename S, bool TAPED, int NT>
-__global__ void __launch_bounds__(NT, (sizeof(R) == 8 ? 3 : 5) * FLUX_BLOCK / NT) k_adj_flux(MeshDev<R> m, Phys P, const R* __restrict__ rec, R coef,
-                                                    const S* __restrict__ ar, const S* __restrict__ au,
-                                                    const S* __restrict__ ae, R* __restrict__ fadj, int inviscid,
-                                                    const R* __restrict__ tape) {
+__global__ void __launch_bounds__(NT, (sizeof(R) == 8 ? 3 : 5) * FLUX_BLOCK / NT)
+    k_adj_flux(MeshDev<R> m, Phys P, const R* __restrict__ rec, R coef, const S* __restrict__ ar,
+               const S* __restrict__ au, const S* __restrict__ ae, R* __restrict__ fadj, int inviscid,
+               const R* __restrict__ tape) {
     // the block's 40-value face records are staged here and written out contiguously: one
     // thread's 40 scalar stores at a 40-value stride would touch a new 32-byte sector each and
     // load L2 with eight partial writes per sector
     __shared__ __align__(16) R stage[NT * FADJ];
     const int f0 = blockIdx.x * NT;
     const int f = f0 + threadIdx.x;
-    if (f < m.nF) adj_face<R, S, TAPED>(m, P, rec, coef, ar, au, ae, inviscid, f, stage + threadIdx.x * FADJ, tape);
+    if (f < m.nF)
+        adj_face<R, S, TAPED, R>(m, P, rec, coef, ar, au, ae, inviscid, f, RowStage<R>{stage + threadIdx.x * FADJ}, tape);
     __syncthreads();
     store_staged<R, FADJ, NT>(fadj, f0, min(NT, m.nF - f0), stage);
+}
+
+// The same with products, reciprocals and square roots on the integer pipes (soft64.cuh), FP64.
+// Of 323 FP64 instructions a face of the taped VJP 233 are left: 3.71 -> 2.86 ms a launch of
+// 6,340,608 faces (the FP64 pipe 67 % busy; 2.3 ms when it never waited). The forward values
+// come through shared memory: read from global memory where they are used, the same kernel takes
+// 3.05 ms at 168 registers and 3.07 ms at 128 (four blocks a SM). Untaped, the forward writes
+// them there instead of holding 61 values in registers: 3 x 521 -> 3 x 310 us for 317,955
+// faces (356 with the hardware's products).
+constexpr size_t COLUMN_BYTES = sizeof(double) * TAPE * ColumnStage<double>::stride;
+template <bool TAPED>
+__global__ void __launch_bounds__(FLUX_BLOCK, 3)
+    k_adj_flux_soft(const __grid_constant__ MeshDev<double> m, const __grid_constant__ Phys P,
+                    const double* __restrict__ rec, double coef, const double* __restrict__ ar,
+                    const double* __restrict__ au, const double* __restrict__ ae, double* __restrict__ fadj,
+                    int inviscid, const double* __restrict__ tape) {
+    extern __shared__ __align__(16) double columns[];
+    constexpr int stride = ColumnStage<double>::stride;
+    const int f0 = blockIdx.x * FLUX_BLOCK;
+    const int f = f0 + threadIdx.x;
+    if (f < m.nF) {
+        const ColumnStage<double> st{columns + threadIdx.x};
+        soft_flag() = 0;
+        unsigned most = 0;
+        adj_face<double, double, TAPED, sd>(m, P, rec, coef, ar, au, ae, inviscid, f, st, tape, &most);
+        if (__builtin_expect(most >= SOFT_LIMIT || soft_flag() != 0, 0))
+            adj_face_again<double, double, TAPED>(m, P, rec, coef, ar, au, ae, inviscid, f, st, tape);
+    }
+    __syncthreads();
+    // records i = j / 20 out of the columns, two values a step
+    const int n = min(FLUX_BLOCK, m.nF - f0) * (FADJ / 2);
+    double2* o = reinterpret_cast<double2*>(fadj + (size_t)f0 * FADJ);
+    for (int j = threadIdx.x; j < n; j += FLUX_BLOCK) {
+        const int i = j / (FADJ / 2), k = 2 * (j % (FADJ / 2));
+        o[j] = make_double2(columns[k * stride + i], columns[(k + 1) * stride + i]);
+    }
+}
+
+// the shared memory of k_adj_flux_soft on the context's device (before the first launch there)
+int prepare_adjoint(Ctx* c) {
+    cudaError_t e = cudaFuncSetAttribute(k_adj_flux_soft<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)COLUMN_BYTES);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_adj_flux_soft<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)COLUMN_BYTES);
+    return e == cudaSuccess ? AFVM_OK : cuda_fail(c, e, "adjoint set-up");
 }
 
 // one cell's sum of its faces' adjoint records (and of the ghosts whose gradient is its own)
@@ -380,14 +505,28 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
         {
             ProfScope ps(c, KID_ADJ_FLUX, s);
             const R* ft = faceTape ? faceTape + (size_t)st * TAPE * m.nF : nullptr;
+            using Small = std::integral_constant<int, 32>;
+            using Big = std::integral_constant<int, FLUX_BLOCK>;
+            const bool small = gF.threads == 32;
             auto flux = [&](auto taped, auto nt) {
                 k_adj_flux<R, S, decltype(taped)::value, decltype(nt)::value><<<gF.blocks, decltype(nt)::value, 0, s>>>(
                     m, P, rec, coef, ain[0], ain[1], ain[2], fadj, inviscid, ft);
             };
-            using Small = std::integral_constant<int, 32>;
-            using Big = std::integral_constant<int, FLUX_BLOCK>;
-            const bool small = gF.threads == 32;
-            if (ft && small) flux(std::true_type{}, Small{});
+            bool done = false;
+            if constexpr (std::is_same<R, double>::value) {
+                if (use_soft(c, m.nF) && std::fabs(coef) < 0x1p64) {
+                    auto soft = [&](auto kernel) {
+                        kernel<<<(m.nF + FLUX_BLOCK - 1) / FLUX_BLOCK, FLUX_BLOCK, COLUMN_BYTES, s>>>(
+                            m, P, rec, coef, ain[0], ain[1], ain[2], fadj, inviscid, ft);
+                    };
+                    if (ft) soft(k_adj_flux_soft<true>);
+                    else soft(k_adj_flux_soft<false>);
+                    done = true;
+                }
+            }
+            if (done) {
+                // (launched)
+            } else if (ft && small) flux(std::true_type{}, Small{});
             else if (ft) flux(std::true_type{}, Big{});
             else if (small) flux(std::false_type{}, Small{});
             else flux(std::false_type{}, Big{});

@@ -448,6 +448,7 @@ int alloc_adjoint(Ctx* c) {
     if (c->fadj) return AFVM_OK;
     int64_t before = c->bytes;
     int st;
+    if ((st = prepare_adjoint(c))) return st;
     size_t n = c->nIC;
     if ((st = dalloc(c, &c->fadj, sizeof(R) * (size_t)c->nF * 40))) return st;
     if ((st = dalloc(c, &c->cbar, sizeof(R) * n * 20))) return st;
@@ -530,6 +531,29 @@ static void set_gauge(Phys& P, double p, double T, double H) {
     finish_phys(P);
 }
 
+// whether the mesh tables the FP64 face kernels read and the gas constants lie below 2^64 (and are
+// finite), as the integer form of their arithmetic takes for granted (soft64.cuh)
+static bool soft_inputs(const HostTables& h, const Phys& P) {
+    auto below = [](const std::vector<double>& v) {
+        double most = 0;
+        bool finite = true;
+#pragma omp parallel for reduction(max : most) reduction(&& : finite)
+        for (size_t i = 0; i < v.size(); i++) {
+            most = std::max(most, std::fabs(v[i]));
+            finite = finite && std::isfinite(v[i]);
+        }
+        return finite && most < 0x1p64;
+    };
+    const PhysR<double>& q = P.d;
+    const double consts[] = {q.gamma, q.gm1, q.Cp, q.Cv, q.kFac, q.mu0, q.muAs, q.muTs, q.small,
+                             q.Rg, q.gRg, q.hgRg, q.muTs15};
+    for (double v : consts)
+        if (!(std::fabs(v) < 0x1p64)) return false;
+    for (double d : h.dlt)
+        if (!(d > 0x1p-64)) return false;              // 1/deltas
+    return below(h.nrm) && below(h.du) && below(h.lw) && below(h.qw) && below(h.wpf) && below(h.wnf);
+}
+
 // the default gauge state: the mean fixed boundary pressure and temperature (the totals of
 // CBC_TOTAL_PT patches) and the mean of Cp T + |U|^2/2 over the ghosts with fixed U and T (Cp T
 // without any); zero where the boundary conditions fix none (a periodic box)
@@ -608,6 +632,7 @@ int afvm_ctx_create(const afvm_mesh_tensors* mesh, const afvm_patch_bc* bcs, con
     HostTables h;
     int st = build_tables(c, mesh, bcs, h);
     if (!st) derive_gauge(h, P);
+    if (!st) c->softInputs = precision == AFVM_FP64 && soft_inputs(h, P);
     if (!st) st = (precision == AFVM_FP64) ? upload_mesh<double>(c, h, c->m64) : upload_mesh<float>(c, h, c->m32);
     if (!st)
         st = dispatch(c, [&](auto r, auto sv) { return alloc_work<decltype(r), decltype(sv)>(c); });

@@ -153,6 +153,7 @@ struct Ctx {
     int objective, objPatch;
     int objStart, objN;       // face range of the objective patch
     int nIC, nIF, nF, nC, nG, nPatches;
+    bool softInputs = false;  // FP64: gas constants and mesh tables within the range of soft64.cuh
     int nBoundaryFlux = 0;    // faces with FACE_BOUNDARY (the physical boundary flux)
     std::vector<int> patchStart, patchN, patchKind, patchCellStart;
     // device allocations
@@ -261,6 +262,7 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
                      const S* rhoNa, const S* rhoUNa, const S* rhoENa, double obja,
                      S* rhoa, S* rhoUa, S* rhoEa, S* Srhoa, S* SrhoUa, S* SrhoEa, cudaStream_t s,
                      const S* stages = nullptr, const R* tape = nullptr, const ParamDev* params = nullptr);
+int prepare_adjoint(Ctx* c);
 // per stage of the reverse sweep, after the face records and cell sums of the stage (fadj,
 // cbar) and before the stage's cell kernel: adds the stage's share of the parameter gradients
 template <typename R, typename S>
@@ -309,6 +311,14 @@ void default_sources(Ctx* c, const S*& Srho, const S*& SrhoU, const S*& SrhoE);
 int host_copy(int32_t device, void* dst, int32_t dstBytes, const void* src, int32_t srcBytes, int64_t count,
               void* stream, bool toDevice, bool syncPinned);
 static inline int nblocks(long long n) { return (int)((n + BLOCK - 1) / BLOCK); }
+
+// Whether the FP64 face kernels over n faces form their products on the integer pipes
+// (soft64.cuh). Those products run beside the FP64 pipe only where other warps of the
+// sub-partition keep it busy: taped flux and VJP of 2.2 warps a sub-partition (box 24^3) 30.9 and
+// 38.7 us against 33.1 and 39.0, of 3.5 (28^3) 53 and 63 against 50 and 56, of 6.8 (a 256x128
+// cylinder) 58 and 91 against 61 and 81, of 10 (40^3) 97 and 126 against 124 and 138. The line
+// is the one of small grids, 8 warps.
+inline bool use_soft(const Ctx* c, long long n) { return c->softInputs && !small_grid(n); }
 
 // Launch shape of a kernel with one thread per item: `big` threads a block, or one warp a block
 // for a small grid.

@@ -2,6 +2,7 @@
 #pragma once
 #include "ctx.cuh"
 #include "face.cuh"
+#include "soft64.cuh"
 
 namespace afvm {
 
@@ -21,10 +22,36 @@ __device__ __forceinline__ void load_vec(const float* __restrict__ p, float* o, 
     }
 }
 
-// the 55 inputs of one face: primitives and gradients of both sides, geometry
-template <typename R>
-__device__ __forceinline__ void load_face(const MeshDev<R>& m, const R* __restrict__ rec, int f, FaceIn<R>& in) {
+// the geometry inputs of a face (what the VJP reads besides the tape). Q: the type the face
+// physics computes with (R, or sd for FP64)
+template <typename R, typename Q>
+__device__ __forceinline__ void load_face_geometry(const MeshDev<R>& m, int f, FaceIn<Q>& in) {
     const size_t nF = m.nF;
+    for (int k = 0; k < 3; k++) {
+        in.N[k] = m.nrm[k * nF + f];
+        in.D[k] = m.du[k * nF + f];
+        in.qw0[k] = m.qw[k * nF + f];
+        in.qw1[k] = m.qw[(3 + k) * nF + f];
+    }
+    in.lw0 = m.lw[f];
+    in.lw1 = m.lw[nF + f];
+    in.rdelta = m.rdlt[f];
+    if constexpr (sizeof(R) == 8) {
+        for (int k = 0; k < 3; k++) in.Nt[k] = m.ntd[k * nF + f];
+        in.ND = m.ntd[3 * nF + f];
+    } else {
+        // FP32 face kernels are bound by their loads, not by their (FP32) arithmetic: formed here
+        in.ND = dot3(in.N, in.D);
+        for (int k = 0; k < 3; k++) in.Nt[k] = in.N[k] - in.ND * in.D[k];
+    }
+}
+
+// the 55 inputs of one face: primitives and gradients of both sides, geometry. most (for Q =
+// sd): the largest magnitude seen among the cell values (soft_seen); the mesh tables are checked
+// when the context is made.
+template <typename R, typename Q>
+__device__ __forceinline__ void load_face(const MeshDev<R>& m, const R* __restrict__ rec, int f, FaceIn<Q>& in,
+                                          unsigned* most = nullptr) {
     int iP = m.own[f], iN = m.nbr[f];
     int iNg = (f < m.nIF) ? iN : m.gsrc[iN - m.nIC];   // ghost gradient = copy of its source
     R rP[REC], rN[REC], rNg[REC];
@@ -35,6 +62,11 @@ __device__ __forceinline__ void load_face(const MeshDev<R>& m, const R* __restri
     } else {
         load_vec(rec + (size_t)iNg * REC, rNg, REC);
     }
+    if constexpr (!std::is_same<R, Q>::value)
+        for (int k = 0; k < REC; k++) {
+            soft_seen(*most, rP[k]);
+            soft_seen(*most, k < R_GU ? rN[k] : rNg[k]);
+        }
     for (int k = 0; k < 3; k++) { in.UP[k] = rP[k]; in.UN[k] = rN[k]; }
     in.TP = rP[R_T]; in.pP = rP[R_P];
     in.TN = rN[R_T]; in.pN = rN[R_P];
@@ -42,60 +74,34 @@ __device__ __forceinline__ void load_face(const MeshDev<R>& m, const R* __restri
     for (int k = 0; k < 3; k++) {
         in.gTP[k] = rP[R_GT + k]; in.gTN[k] = rNg[R_GT + k];
         in.gpP[k] = rP[R_GP + k]; in.gpN[k] = rNg[R_GP + k];
-        in.N[k] = m.nrm[k * nF + f];
-        in.D[k] = m.du[k * nF + f];
-        in.qw0[k] = m.qw[k * nF + f];
-        in.qw1[k] = m.qw[(3 + k) * nF + f];
     }
-    in.lw0 = m.lw[f];
-    in.lw1 = m.lw[nF + f];
-    in.rdelta = m.rdlt[f];
-    if constexpr (sizeof(R) == 8) {
-        for (int k = 0; k < 3; k++) in.Nt[k] = m.ntd[k * nF + f];
-        in.ND = m.ntd[3 * nF + f];
-    } else {
-        // FP32 face kernels are bound by their loads, not by their (FP32) arithmetic: formed here
-        in.ND = dot3(in.N, in.D);
-        for (int k = 0; k < 3; k++) in.Nt[k] = in.N[k] - in.ND * in.D[k];
-    }
+    load_face_geometry<R, Q>(m, f, in);
+}
+
+// soft_seen of a taped value; 1/eps of the entropy fix may be 1e30 (eps is at least `small`), in a
+// uniform flow, and only meets eigenvalues below 2 eps
+__device__ __forceinline__ void seen_taped(unsigned& most, int k, double x) {
+    if (k != T_RE) soft_seen(most, x);
 }
 
 // a face's column of a device tape (value k of face f at tape[k nF + f]; p = tape + f)
-template <typename R>
+template <typename R, typename Q = R>
 struct TapeStore {
     R* p;
     size_t stride;
-    __device__ __forceinline__ void put(int k, R x) const { p[(size_t)k * stride] = x; }
+    __device__ __forceinline__ void put(int k, Q x) const { p[(size_t)k * stride] = raw(x); }
 };
-template <typename R>
+template <typename R, typename Q = R>
 struct TapeLoad {
     static constexpr bool kFull = true;
     const R* p;
     size_t stride;
-    __device__ __forceinline__ R get(int k) const { return __ldg(p + (size_t)k * stride); }
+    unsigned* most = nullptr;      // as load_face
+    __device__ __forceinline__ Q get(int k) const {
+        const R x = __ldg(p + (size_t)k * stride);
+        if constexpr (!std::is_same<R, Q>::value) seen_taped(*most, k, x);
+        return x;
+    }
 };
-
-// the geometry inputs of a face only (what the VJP reads besides the tape)
-template <typename R>
-__device__ __forceinline__ void load_face_geometry(const MeshDev<R>& m, int f, FaceIn<R>& in) {
-    const size_t nF = m.nF;
-    for (int k = 0; k < 3; k++) {
-        in.N[k] = m.nrm[k * nF + f];
-        in.D[k] = m.du[k * nF + f];
-        in.qw0[k] = m.qw[k * nF + f];
-        in.qw1[k] = m.qw[(3 + k) * nF + f];
-    }
-    in.lw0 = m.lw[f];
-    in.lw1 = m.lw[nF + f];
-    in.rdelta = m.rdlt[f];
-    if constexpr (sizeof(R) == 8) {
-        for (int k = 0; k < 3; k++) in.Nt[k] = m.ntd[k * nF + f];
-        in.ND = m.ntd[3 * nF + f];
-    } else {
-        // FP32 face kernels are bound by their loads, not by their (FP32) arithmetic: formed here
-        in.ND = dot3(in.N, in.D);
-        for (int k = 0; k < 3; k++) in.Nt[k] = in.N[k] - in.ND * in.D[k];
-    }
-}
 
 }  // namespace afvm

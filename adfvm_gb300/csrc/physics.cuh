@@ -144,8 +144,14 @@ inline void finish_phys(Phys& P) {
     fill_consts(P, P.f);
 }
 
+// the precision of a working type's constants (a double evaluated otherwise, soft64.cuh, has
+// the double ones)
 template <typename R>
-AFVM_HD const PhysR<R>& consts(const Phys& P);
+struct PhysOf {
+    using type = PhysR<R>;
+};
+template <typename R>
+AFVM_HD const typename PhysOf<R>::type& consts(const Phys& P);
 template <>
 AFVM_HD const PhysR<double>& consts<double>(const Phys& P) { return P.d; }
 template <>
@@ -315,6 +321,10 @@ AFVM_HD float rcp(float x) {
 #endif
 }
 
+// 1/eps of the entropy fix, whose eps may be as small as `small` (1e-30)
+template <typename R>
+AFVM_HD R rcp_eps(R x) { return rcp(x); }
+
 AFVM_HD double rsqrt_(double x) {
 #if defined(__CUDA_ARCH__)
     return rsqrt_nr(x);
@@ -453,7 +463,7 @@ AFVM_HD void roe(const Phys& P, R pL, R pR, R TL, R TR, const R* UL, const R* UR
     R re = R(0);
     bool s1 = lt_twice(lam1, eps), s2 = lt_twice(lam2, eps), s3 = lt_twice(lam3, eps);
     if (s1 || s2 || s3) {
-        re = rcp(eps);
+        re = rcp_eps(eps);
         if (s1) lam1 = R(0.25) * lam1 * lam1 * re + eps;
         // (the acoustic eigenvalues take the fix only near sonic faces: a branch warps skip)
         if (__builtin_expect(s2 || s3, 0)) {

@@ -239,27 +239,56 @@ static void launch_grad(Ctx* c, R* rec, cudaStream_t s) {
 // k_adj_flux<..., true> reads back instead of re-evaluating the forward flux
 // CFL: the stage whose CFL sum is taken (the second, density.py:405-413); the other stages
 // store 0 in the CFL slot and skip its square root
+// one face: Q is the type its physics computes with (R, or sd for FP64)
+template <typename R, typename Q, bool TAPED, bool CFL>
+__device__ __forceinline__ void flux_face(const MeshDev<R>& m, const Phys& P, const R* __restrict__ rec, int f,
+                                          R* __restrict__ fflux, int inviscid, R* __restrict__ tape,
+                                          unsigned* most = nullptr) {
+    int kind = (f < m.nIF) ? FACE_INTERNAL : (int)m.fkind[f - m.nIF];
+    FaceIn<Q> in;
+    load_face<R, Q>(m, rec, f, in, most);
+    Q F[5], maxaF;
+    // (FP32 records hold gauge offsets and their fluxes are the gauge form; only FP64
+    // contexts keep face tapes)
+    if constexpr (TAPED && !kGauge<R>)
+        face_flux<Q>(P, kind, inviscid != 0, in, F, maxaF, TapeStore<R, Q>{tape + f, (size_t)m.nF});
+    else
+        face_flux<Q, kGauge<R>>(P, kind, inviscid != 0, in, F, maxaF);
+    R* out = fflux + (size_t)f * FREC;
+    for (int k = 0; k < 5; k++) out[k] = raw(F[k]);
+    out[5] = CFL ? raw(maxaF) : R(0);
+}
+
+// the face again with the hardware's FP64 operations throughout (soft_flag)
 template <typename R, bool TAPED, bool CFL>
-__global__ void __launch_bounds__(FLUX_BLOCK, sizeof(R) == 8 ? 3 : 8) k_flux(MeshDev<R> m, Phys P, const R* __restrict__ rec,
-                                                R* __restrict__ fflux, int inviscid, R* __restrict__ tape) {
+__device__ __noinline__ void flux_face_again(const MeshDev<R>& m, const Phys& P, const R* rec, int f, R* fflux,
+                                             int inviscid, R* tape) {
+    flux_face<R, R, TAPED, CFL>(m, P, rec, f, fflux, inviscid, tape);
+}
+
+// SOFT (FP64): products, reciprocals and square roots on the integer pipes (soft64.cuh). The FP64
+// pipe binds either form; of 298 FP64 instructions a face (52 DADD, 90 DMUL, 156 DFMA) 183 are
+// left (50 DADD, 133 DFMA): 3.47 -> 2.33 ms a taped launch of 6,340,608 faces, 1.81 ms when the
+// pipe never waited (it is 68 % busy: three warps a sub-partition, whose integer chains are
+// serial; 128 registers for four spill more than they hide, 2.42 ms, 255 for two 2.46).
+template <typename R, bool TAPED, bool CFL, bool SOFT>
+__global__ void __launch_bounds__(FLUX_BLOCK, sizeof(R) == 8 ? 3 : 8)
+    k_flux(const __grid_constant__ MeshDev<R> m, const __grid_constant__ Phys P, const R* __restrict__ rec,
+           R* __restrict__ fflux, int inviscid, R* __restrict__ tape) {
     // (the 6-value face records are stored directly: staging them through shared memory, as
     // the 20- and 40-value records are, made this kernel slower - 0.217 -> 0.269 ms at 128^3 in
     // FP32 - the barrier costs more than the six partly coalesced stores)
     int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= m.nF) return;
-    int kind = (f < m.nIF) ? FACE_INTERNAL : (int)m.fkind[f - m.nIF];
-    FaceIn<R> in;
-    load_face<R>(m, rec, f, in);
-    R F[5], maxaF;
-    // (FP32 records hold gauge offsets and their fluxes are the gauge form; only FP64
-    // contexts keep face tapes)
-    if constexpr (TAPED && !kGauge<R>)
-        face_flux<R>(P, kind, inviscid != 0, in, F, maxaF, TapeStore<R>{tape + f, (size_t)m.nF});
-    else
-        face_flux<R, kGauge<R>>(P, kind, inviscid != 0, in, F, maxaF);
-    R* out = fflux + (size_t)f * FREC;
-    for (int k = 0; k < 5; k++) out[k] = F[k];
-    out[5] = CFL ? maxaF : R(0);
+    if constexpr (SOFT) {
+        soft_flag() = 0;
+        unsigned most = 0;
+        flux_face<R, sd, TAPED, CFL>(m, P, rec, f, fflux, inviscid, tape, &most);
+        if (__builtin_expect(most >= SOFT_LIMIT || soft_flag() != 0, 0))
+            flux_face_again<R, TAPED, CFL>(m, P, rec, f, fflux, inviscid, tape);
+    } else {
+        flux_face<R, R, TAPED, CFL>(m, P, rec, f, fflux, inviscid, tape);
+    }
 }
 
 // a 6-value face flux record in three 8- (FP32) or 16-byte (FP64) loads; records start on
@@ -541,15 +570,23 @@ void launch_flux_update(Ctx* c, int st, double dt, const double* dtDev, const S*
     {
         ProfScope ps(c, KID_FLUX, s);
         const Shape g = shape_for(m.nF, FLUX_BLOCK);
-        const int nbF = g.blocks;
-        if (tape && st == 1)
-            k_flux<R, true, true><<<nbF, g.threads, 0, s>>>(m, P, rec, ff, inviscid, tape);
-        else if (tape)
-            k_flux<R, true, false><<<nbF, g.threads, 0, s>>>(m, P, rec, ff, inviscid, tape);
-        else if (st == 1)
-            k_flux<R, false, true><<<nbF, g.threads, 0, s>>>(m, P, rec, ff, inviscid, nullptr);
-        else
-            k_flux<R, false, false><<<nbF, g.threads, 0, s>>>(m, P, rec, ff, inviscid, nullptr);
+        auto flux = [&](auto taped, auto cfl, auto soft) {
+            k_flux<R, decltype(taped)::value, decltype(cfl)::value, decltype(soft)::value>
+                <<<g.blocks, g.threads, 0, s>>>(m, P, rec, ff, inviscid, tape);
+        };
+        auto by_cfl = [&](auto taped, auto soft) {
+            if (st == 1) flux(taped, std::true_type{}, soft);
+            else flux(taped, std::false_type{}, soft);
+        };
+        if constexpr (sizeof(R) == 8) {
+            const bool soft = use_soft(c, m.nF);
+            if (tape && soft) by_cfl(std::true_type{}, std::true_type{});
+            else if (tape) by_cfl(std::true_type{}, std::false_type{});
+            else if (soft) by_cfl(std::false_type{}, std::true_type{});
+            else by_cfl(std::false_type{}, std::false_type{});
+        } else {
+            by_cfl(std::false_type{}, std::false_type{});     // (FP32 contexts keep no face tape)
+        }
     }
     const Shape g = shape_for(m.nIC, BLOCK);
     R* recNext = nextPrims ? (recOut ? recOut : rec) : nullptr;

@@ -68,23 +68,37 @@ struct TapeColumn {
     }
 };
 
+// what a face's adjoint reads of the mesh
+template <typename R, typename Q>
+struct AdjFaceMesh {
+    FaceAt at;
+    FaceIn<Q> in;      // the geometry; the cell values where they are needed
+    R wp, wn;          // A/V_L and, of an internal face, A/V_R
+};
+template <typename R, typename Q>
+__device__ __forceinline__ void load_adj_face_mesh(const MeshDev<R>& m, int f, AdjFaceMesh<R, Q>& a) {
+    a.at = load_face_mesh<R, Q>(m, f, a.in);
+    a.wp = m.wpf[f];
+    a.wn = f < m.nIF ? m.wnf[f] : R(0);
+}
+
 // one face's record of k_adj_flux into st; TAPED: the forward values of a non-boundary face come
 // from its tape column instead of a re-evaluation of the face flux
 template <typename R, typename S, bool TAPED, typename Q, typename Stage>
-__device__ __forceinline__ void adj_face(const MeshDev<R>& m, const Phys& P, const R* __restrict__ rec, R coef,
-                                         const S* __restrict__ ar, const S* __restrict__ au,
-                                         const S* __restrict__ ae, int inviscid, int f, const Stage& st,
-                                         const R* __restrict__ tape, unsigned* most = nullptr) {
+__device__ __forceinline__ void adj_face(const MeshDev<R>& m, const Phys& P, AdjFaceMesh<R, Q>& a,
+                                         const R* __restrict__ rec, R coef, const S* __restrict__ ar,
+                                         const S* __restrict__ au, const S* __restrict__ ae, int inviscid, int f,
+                                         const Stage& st, const R* __restrict__ tape, unsigned* most = nullptr) {
     constexpr bool COLUMN = std::is_same<Stage, ColumnStage<R>>::value;
     // (mixed contexts keep the order their FP64 adjoints have always rounded in)
     constexpr bool VFIRST = sizeof(R) == 4 && sizeof(S) == 8;
-    int kind = (f < m.nIF) ? FACE_INTERNAL : (int)m.fkind[f - m.nIF];
+    const int kind = a.at.kind;
     const bool fromTape = TAPED && kind != FACE_BOUNDARY;
     if constexpr (TAPED && COLUMN)
         if (fromTape) st.fetch(tape + f, (size_t)m.nF);
-    int iP = m.own[f];
     // Fbar = coef (abar_P A/V_L - abar_N A/V_R), coef folded into the two weights
-    Q wp = Q(coef) * Q(m.wpf[f]);
+    const int iP = a.at.own;
+    Q wp = Q(coef) * Q(a.wp);
     R aP[5] = {R(ar[iP]), R(au[3 * iP]), R(au[3 * iP + 1]), R(au[3 * iP + 2]), R(ae[iP])};
     Q Fb[5];
     for (int k = 0; k < 5; k++) {
@@ -92,19 +106,18 @@ __device__ __forceinline__ void adj_face(const MeshDev<R>& m, const Phys& P, con
         Fb[k] = Q(aP[k]) * wp;
     }
     if (f < m.nIF) {
-        int iN = m.nbr[f];
-        Q wn = Q(coef) * Q(m.wnf[f]);
+        const int iN = a.at.nbr;
+        Q wn = Q(coef) * Q(a.wn);
         R aN[5] = {R(ar[iN]), R(au[3 * iN]), R(au[3 * iN + 1]), R(au[3 * iN + 2]), R(ae[iN])};
         for (int k = 0; k < 5; k++) {
             if constexpr (!std::is_same<R, Q>::value) soft_seen(*most, aN[k]);
             Fb[k] = Fb[k] - Q(aN[k]) * wn;
         }
     }
-    FaceIn<Q> in;
+    FaceIn<Q>& in = a.in;
     FaceBar<Q> b;
     zero_bar(b);
     if (fromTape) {
-        load_face_geometry<R, Q>(m, f, in);
         if constexpr (COLUMN) {
             st.fetched();
             face_vjp_t<Q, VFIRST>(P, kind, inviscid != 0, in, TapeColumn<R, Q>{st.col, most}, Fb, b);
@@ -112,7 +125,7 @@ __device__ __forceinline__ void adj_face(const MeshDev<R>& m, const Phys& P, con
             face_vjp_t<Q, VFIRST>(P, kind, inviscid != 0, in, TapeLoad<R, Q>{tape + f, (size_t)m.nF, most}, Fb, b);
         }
     } else {
-        load_face<R, Q>(m, rec, f, in, most);
+        load_face_cells<R, Q>(rec, a.at, in, most);
         if constexpr (kGauge<R>) {
             // the VJP differentiates the absolute-form flux (the same function of the state as
             // the gauge form the forward evaluates)
@@ -145,7 +158,9 @@ template <typename R, typename S, bool TAPED>
 __device__ __noinline__ void adj_face_again(const MeshDev<R>& m, const Phys& P, const R* rec, R coef, const S* ar,
                                             const S* au, const S* ae, int inviscid, int f, ColumnStage<R> st,
                                             const R* tape) {
-    adj_face<R, S, TAPED, R>(m, P, rec, coef, ar, au, ae, inviscid, f, st, tape);
+    AdjFaceMesh<R, R> a;
+    load_adj_face_mesh<R, R>(m, f, a);
+    adj_face<R, S, TAPED, R>(m, P, a, rec, coef, ar, au, ae, inviscid, f, st, tape);
 }
 
 template <typename R, typename S, bool TAPED, int NT>
@@ -159,8 +174,12 @@ __global__ void __launch_bounds__(NT, (sizeof(R) == 8 ? 3 : 5) * FLUX_BLOCK / NT
     __shared__ __align__(16) R stage[NT * FADJ];
     const int f0 = blockIdx.x * NT;
     const int f = f0 + threadIdx.x;
+    AdjFaceMesh<R, R> a;
+    if (f < m.nF) load_adj_face_mesh<R, R>(m, f, a);
+    dep_wait(rec, ar, au, ae, fadj, tape);
     if (f < m.nF)
-        adj_face<R, S, TAPED, R>(m, P, rec, coef, ar, au, ae, inviscid, f, RowStage<R>{stage + threadIdx.x * FADJ}, tape);
+        adj_face<R, S, TAPED, R>(m, P, a, rec, coef, ar, au, ae, inviscid, f, RowStage<R>{stage + threadIdx.x * FADJ},
+                                 tape);
     __syncthreads();
     store_staged<R, FADJ, NT>(fadj, f0, min(NT, m.nF - f0), stage);
 }
@@ -183,11 +202,14 @@ __global__ void __launch_bounds__(FLUX_BLOCK, 3)
     constexpr int stride = ColumnStage<double>::stride;
     const int f0 = blockIdx.x * FLUX_BLOCK;
     const int f = f0 + threadIdx.x;
+    AdjFaceMesh<double, sd> a;
+    if (f < m.nF) load_adj_face_mesh<double, sd>(m, f, a);
+    dep_wait(rec, ar, au, ae, fadj, tape);
     if (f < m.nF) {
         const ColumnStage<double> st{columns + threadIdx.x};
         soft_flag() = 0;
         unsigned most = 0;
-        adj_face<double, double, TAPED, sd>(m, P, rec, coef, ar, au, ae, inviscid, f, st, tape, &most);
+        adj_face<double, double, TAPED, sd>(m, P, a, rec, coef, ar, au, ae, inviscid, f, st, tape, &most);
         if (__builtin_expect(most >= SOFT_LIMIT || soft_flag() != 0, 0))
             adj_face_again<double, double, TAPED>(m, P, rec, coef, ar, au, ae, inviscid, f, st, tape);
     }
@@ -211,17 +233,18 @@ int prepare_adjoint(Ctx* c) {
     return e == cudaSuccess ? AFVM_OK : cuda_fail(c, e, "adjoint set-up");
 }
 
-// one cell's sum of its faces' adjoint records (and of the ghosts whose gradient is its own)
+// one cell's sum of its faces' adjoint records (and of the ghosts whose gradient is its own):
+// e the cell's faces in collate order, ghosts gs0..gs1 of the list
 template <typename R>
-__device__ __forceinline__ void adj_cell_gather(const MeshDev<R>& m, const R* __restrict__ fadj, int c, R* row) {
-    const size_t n = m.nIC;
+__device__ __forceinline__ void adj_cell_gather(const MeshDev<R>& m, const R* __restrict__ fadj, const int* e, int gs0,
+                                                int gs1, R* row) {
     // the first slot initialises the sums: adding it to zeros would cost 20 more adds (FP64
     // pipe issues in double) and changes nothing but the sign of a zero
     R acc[CBAR];
+#pragma unroll
     for (int s = 0; s < 6; s++) {
-        int e = m.accf[s * n + c];
-        bool ownerSide = e >= 0;
-        int f = ownerSide ? e : ~e;
+        bool ownerSide = e[s] >= 0;
+        int f = ownerSide ? e[s] : ~e[s];
         R v[CBAR];
         load_vec(fadj + (size_t)f * FADJ + (ownerSide ? 0 : CBAR), v, CBAR);
         if (s == 0)
@@ -230,7 +253,7 @@ __device__ __forceinline__ void adj_cell_gather(const MeshDev<R>& m, const R* __
             for (int k = 0; k < CBAR; k++) acc[k] += v[k];
     }
     // gradient adjoints of the ghosts whose gradient is a copy of this cell's
-    for (int q = m.gsStart[c]; q < m.gsStart[c + 1]; q++) {
+    for (int q = gs0; q < gs1; q++) {
         int g = m.gsList[q];
         const R* r = fadj + (size_t)(m.nIF + g) * FADJ;
         for (int k = 0; k < 15; k++) acc[5 + k] += r[25 + k];
@@ -243,7 +266,15 @@ __global__ void __launch_bounds__(NT) k_adj_cell1(MeshDev<R> m, const R* __restr
     __shared__ __align__(16) R stage[NT * CBAR];
     const int c0 = blockIdx.x * NT;
     const int c = c0 + threadIdx.x;
-    if (c < m.nIC) adj_cell_gather<R>(m, fadj, c, stage + threadIdx.x * CBAR);
+    int e[6], gs0 = 0, gs1 = 0;
+    if (c < m.nIC) {
+#pragma unroll
+        for (int s = 0; s < 6; s++) e[s] = m.accf[s * (size_t)m.nIC + c];
+        gs0 = m.gsStart[c];
+        gs1 = m.gsStart[c + 1];
+    }
+    dep_wait(fadj, cbar);
+    if (c < m.nIC) adj_cell_gather<R>(m, fadj, e, gs0, gs1, stage + threadIdx.x * CBAR);
     __syncthreads();
     if (c0 < m.nIC) store_staged<R, CBAR, NT>(cbar, c0, min(NT, m.nIC - c0), stage);
 }
@@ -262,12 +293,24 @@ __global__ void __launch_bounds__(BLOCK) k_adj_cell2(MeshDev<R> m, Phys P, const
                                                      const S* __restrict__ ue,
                                                      const S* ainr, const S* ainu, const S* aine,
                                                      S* a1r, S* a1u, S* a1e, S* a0r, S* a0u, S* a0e, S* sb,
-                                                     double dt, int objective, int objStart, int objN, double obja,
+                                                     S* sr, S* su, S* se, double dt, int objective, int objStart, int objN, double obja,
                                                      VaneDev vane, const double* __restrict__ objSeed) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= m.nIC) return;
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const size_t n = m.nIC;
     const size_t nF = m.nF;
+    int nb[6], gs0 = 0, gs1 = 0;
+    R bs[18], A[3];
+    if (c < m.nIC) {
+#pragma unroll
+        for (int s = 0; s < 6; s++) nb[s] = m.gnb[s * n + c];
+#pragma unroll
+        for (int k = 0; k < 18; k++) bs[k] = m.gbs[k * n + c];
+        for (int j = 0; j < 3; j++) A[j] = m.gAv[j * n + c];
+        gs0 = m.gsStart[c];
+        gs1 = m.gsStart[c + 1];
+    }
+    dep_wait(rec, fadj, cbar, ur, uu, ue, ainr, ainu, aine, a1r, a1u, a1e, a0r, a0u, a0e, sb, objSeed);
+    if (c >= m.nIC) return;
     // cell adjoint records in 16-byte loads (a record is 80 / 160 bytes, 16-byte aligned)
     R cb[CBAR];
     load_vec(cbar + (size_t)c * CBAR, cb, CBAR);
@@ -276,23 +319,22 @@ __global__ void __launch_bounds__(BLOCK) k_adj_cell2(MeshDev<R> m, Phys P, const
     const R* G = cb + 5;
     {
         // the cell's own slots at once: sum_s (1 - w'_s) (G . S N'_s) / V = G . gAv
-        R A[3] = {m.gAv[c], m.gAv[n + c], m.gAv[2 * n + c]};
         for (int i = 0; i < 5; i++) pbar[i] += G[3 * i] * A[0] + G[3 * i + 1] * A[1] + G[3 * i + 2] * A[2];
     }
+#pragma unroll
     for (int s = 0; s < 6; s++) {
-        int nb = m.gnb[s * n + c];
-        if (nb < m.nIC) {
+        if (nb[s] < m.nIC) {
             // neighbour's gradient: its slot for this face has S N'' = -S N' and weight gwb;
             // gbs_s = -gwb_s S N'_s / V_nb
-            R b[3] = {m.gbs[(3 * s) * n + c], m.gbs[(3 * s + 1) * n + c], m.gbs[(3 * s + 2) * n + c]};
+            const R* b = bs + 3 * s;
             R cn[CBAR];
-            load_vec(cbar + (size_t)nb * CBAR, cn, CBAR);
+            load_vec(cbar + (size_t)nb[s] * CBAR, cn, CBAR);
             const R* Gn = cn + 5;
             for (int i = 0; i < 5; i++) pbar[i] += Gn[3 * i] * b[0] + Gn[3 * i + 1] * b[1] + Gn[3 * i + 2] * b[2];
         }
     }
     // ghost cells whose boundary value comes from this cell: transpose of the BC
-    for (int q = m.gsStart[c]; q < m.gsStart[c + 1]; q++) {
+    for (int q = gs0; q < gs1; q++) {
         int g = m.gsList[q];
         int f = m.nIF + g;
         int o = m.own[f];
@@ -437,20 +479,15 @@ __global__ void __launch_bounds__(BLOCK) k_adj_cell2(MeshDev<R> m, Phys P, const
         a1r[c] = out[0]; a1u[3 * c] = out[1]; a1u[3 * c + 1] = out[2]; a1u[3 * c + 2] = out[3]; a1e[c] = out[4];
     } else {
         S z[5] = {a0r[c], a0u[3 * c], a0u[3 * c + 1], a0u[3 * c + 2], a0e[c]};
-        for (int k = 0; k < 5; k++) { z[k] += ain[k] + (S)J[k]; sb[k * n + c] += S(dt) * ain[k]; }
+        for (int k = 0; k < 5; k++) z[k] += ain[k] + (S)J[k];
+        // the source adjoint, complete with this stage, in the reference's layout (any part may be
+        // absent; the stages before keep it in rows by component, as the outputs may alias inputs)
+        if (sr) sr[c] = sb[c] + S(dt) * ain[0];
+        if (su)
+            for (int k = 1; k < 4; k++) su[3 * c + k - 1] = sb[k * n + c] + S(dt) * ain[k];
+        if (se) se[c] = sb[4 * n + c] + S(dt) * ain[4];
         a0r[c] = z[0]; a0u[3 * c] = z[1]; a0u[3 * c + 1] = z[2]; a0u[3 * c + 2] = z[3]; a0e[c] = z[4];
     }
-}
-
-// the source adjoint (5 x nIC, one coalesced row per component) into the reference layout
-template <typename R>
-__global__ void k_split5(int n, const R* __restrict__ sb, R* r, R* u, R* e) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    const size_t m = n;
-    if (r) r[c] = sb[c];
-    if (u) { u[3 * c] = sb[m + c]; u[3 * c + 1] = sb[2 * m + c]; u[3 * c + 2] = sb[3 * m + c]; }
-    if (e) e[c] = sb[4 * m + c];
 }
 
 template <typename R, typename S>
@@ -472,7 +509,6 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
         stage_views<S, const S>(stages, m.nIC, u1c, u2c);
     } else {
         // forward recompute of the stage states
-        cudaMemsetAsync(c->dtcBits, 0, sizeof(unsigned long long), s);
         launch_prim_grad<R, S>(c, rho, rhoU, rhoE, s);
         launch_flux_update<R, S>(c, 0, dt, nullptr, u0c, u1c, u2c, Srho, SrhoU, SrhoE, u1, s);
         launch_prim_grad<R, S>(c, u1[0], u1[1], u1[2], s);
@@ -495,7 +531,7 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
         const S* const* u = st == 0 ? u0c : (st == 1 ? u1c : u2c);
         const R* rec = recTape ? recTape + (size_t)st * m.nC * REC : (const R*)c->rec;
         if (!recTape) launch_prim_grad<R, S>(c, u[0], u[1], u[2], s);
-        if (st == 1 && c->objective == AFVM_OBJ_VANE) launch_vane_sums<R>(c, s, nullptr, nullptr, rec);
+        if (st == 1 && c->objective == AFVM_OBJ_VANE) launch_vane_sums<R>(c, s, nullptr, rec);
         // adjoint of this stage's output: a3 = seeds, a2 = A2, a1 = A1
         const S* ain[3];
         if (st == 2) { ain[0] = rhoNa; ain[1] = rhoUNa; ain[2] = rhoENa; }
@@ -509,15 +545,15 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
             using Big = std::integral_constant<int, FLUX_BLOCK>;
             const bool small = gF.threads == 32;
             auto flux = [&](auto taped, auto nt) {
-                k_adj_flux<R, S, decltype(taped)::value, decltype(nt)::value><<<gF.blocks, decltype(nt)::value, 0, s>>>(
-                    m, P, rec, coef, ain[0], ain[1], ain[2], fadj, inviscid, ft);
+                launch_after(k_adj_flux<R, S, decltype(taped)::value, decltype(nt)::value>, gF.blocks, gF.threads, 0, s,
+                             m, P, rec, coef, ain[0], ain[1], ain[2], fadj, inviscid, ft);
             };
             bool done = false;
             if constexpr (std::is_same<R, double>::value) {
                 if (use_soft(c, m.nF) && std::fabs(coef) < 0x1p64) {
                     auto soft = [&](auto kernel) {
-                        kernel<<<(m.nF + FLUX_BLOCK - 1) / FLUX_BLOCK, FLUX_BLOCK, COLUMN_BYTES, s>>>(
-                            m, P, rec, coef, ain[0], ain[1], ain[2], fadj, inviscid, ft);
+                        launch_after(kernel, (m.nF + FLUX_BLOCK - 1) / FLUX_BLOCK, FLUX_BLOCK, COLUMN_BYTES, s, m, P,
+                                     rec, coef, ain[0], ain[1], ain[2], fadj, inviscid, ft);
                     };
                     if (ft) soft(k_adj_flux_soft<true>);
                     else soft(k_adj_flux_soft<false>);
@@ -533,30 +569,19 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
         }
         {
             ProfScope ps(c, KID_ADJ_GATHER, s);
-            if (gC.threads == 32) k_adj_cell1<R, 32><<<gC.blocks, 32, 0, s>>>(m, fadj, cbar);
-            else k_adj_cell1<R, BLOCK><<<gC.blocks, BLOCK, 0, s>>>(m, fadj, cbar);
+            launch_after(gC.threads == 32 ? k_adj_cell1<R, 32> : k_adj_cell1<R, BLOCK>, gC.blocks, gC.threads, 0, s, m,
+                         (const R*)fadj, cbar);
         }
         // the stage's share of the mesh / boundary-input gradients (before the cell kernel: the
         // adjoint outputs it writes may alias this stage's input adjoints)
         if constexpr (std::is_same<R, double>::value && std::is_same<S, double>::value)
             if (params) launch_param_grads<R, S>(c, *params, rec, coef, ain[0], ain[1], ain[2], st == 1, obja, s);
         ProfScope ps(c, KID_ADJ_GRAD, s);
-        if (st == 2)
-            k_adj_cell2<R, S, 2><<<gC.blocks, gC.threads, 0, s>>>(m, P, rec, fadj, cbar, u[0], u[1], u[2], ain[0], ain[1], ain[2],
-                                                    A2[0], A2[1], A2[2], rhoa, rhoUa, rhoEa, sb, dt, c->objective,
-                                                    c->objStart, c->objN, obja, c->vane, c->objSeed);
-        else if (st == 1)
-            k_adj_cell2<R, S, 1><<<gC.blocks, gC.threads, 0, s>>>(m, P, rec, fadj, cbar, u[0], u[1], u[2], ain[0], ain[1], ain[2],
-                                                    A1[0], A1[1], A1[2], rhoa, rhoUa, rhoEa, sb, dt, c->objective,
-                                                    c->objStart, c->objN, obja, c->vane, c->objSeed);
-        else
-            k_adj_cell2<R, S, 0><<<gC.blocks, gC.threads, 0, s>>>(m, P, rec, fadj, cbar, u[0], u[1], u[2], ain[0], ain[1], ain[2],
-                                                    nullptr, nullptr, nullptr, rhoa, rhoUa, rhoEa, sb, dt,
-                                                    c->objective, c->objStart, c->objN, obja, c->vane, c->objSeed);
-    }
-    if (Srhoa || SrhoUa || SrhoEa) {
-        ProfScope ps(c, KID_ADJ_MISC, s);
-        k_split5<S><<<gC.blocks, gC.threads, 0, s>>>(m.nIC, sb, Srhoa, SrhoUa, SrhoEa);
+        S* const* a1 = st == 2 ? A2 : A1;      // (not written by the last stage)
+        launch_after(st == 2 ? k_adj_cell2<R, S, 2> : (st == 1 ? k_adj_cell2<R, S, 1> : k_adj_cell2<R, S, 0>), gC.blocks,
+                     gC.threads, 0, s, m, P, rec, (const R*)fadj, (const R*)cbar, u[0], u[1], u[2], ain[0], ain[1],
+                     ain[2], a1[0], a1[1], a1[2], rhoa, rhoUa, rhoEa, sb, Srhoa, SrhoUa, SrhoEa, dt, c->objective,
+                     c->objStart, c->objN, obja, c->vane, c->objSeed);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "adjoint step launch");

@@ -46,21 +46,41 @@ __device__ __forceinline__ void load_face_geometry(const MeshDev<R>& m, int f, F
     }
 }
 
-// the 55 inputs of one face: primitives and gradients of both sides, geometry. most (for Q =
-// sd): the largest magnitude seen among the cell values (soft_seen); the mesh tables are checked
-// when the context is made.
+// a face's kind, its cells, and the cell whose gradient the neighbour side reads (a ghost's is a
+// copy of its source's)
+struct FaceAt {
+    int kind, own, nbr, grad;
+};
+template <typename R>
+__device__ __forceinline__ FaceAt face_at(const MeshDev<R>& m, int f) {
+    FaceAt a;
+    a.kind = f < m.nIF ? FACE_INTERNAL : (int)m.fkind[f - m.nIF];
+    a.own = m.own[f];
+    a.nbr = m.nbr[f];
+    a.grad = f < m.nIF ? a.nbr : m.gsrc[a.nbr - m.nIC];
+    return a;
+}
+// what a face reads of the mesh
 template <typename R, typename Q>
-__device__ __forceinline__ void load_face(const MeshDev<R>& m, const R* __restrict__ rec, int f, FaceIn<Q>& in,
-                                          unsigned* most = nullptr) {
-    int iP = m.own[f], iN = m.nbr[f];
-    int iNg = (f < m.nIF) ? iN : m.gsrc[iN - m.nIC];   // ghost gradient = copy of its source
+__device__ __forceinline__ FaceAt load_face_mesh(const MeshDev<R>& m, int f, FaceIn<Q>& in) {
+    const FaceAt a = face_at<R>(m, f);
+    load_face_geometry<R, Q>(m, f, in);
+    return a;
+}
+
+// the cell values of one face: primitives and gradients of both sides. most (for Q = sd): the
+// largest magnitude seen among them (soft_seen); the mesh tables are checked when the context is
+// made.
+template <typename R, typename Q>
+__device__ __forceinline__ void load_face_cells(const R* __restrict__ rec, const FaceAt& a, FaceIn<Q>& in,
+                                                unsigned* most = nullptr) {
     R rP[REC], rN[REC], rNg[REC];
-    load_vec(rec + (size_t)iP * REC, rP, REC);
-    load_vec(rec + (size_t)iN * REC, rN, REC);
-    if (iNg == iN) {
+    load_vec(rec + (size_t)a.own * REC, rP, REC);
+    load_vec(rec + (size_t)a.nbr * REC, rN, REC);
+    if (a.grad == a.nbr) {
         for (int k = 0; k < REC; k++) rNg[k] = rN[k];
     } else {
-        load_vec(rec + (size_t)iNg * REC, rNg, REC);
+        load_vec(rec + (size_t)a.grad * REC, rNg, REC);
     }
     if constexpr (!std::is_same<R, Q>::value)
         for (int k = 0; k < REC; k++) {
@@ -75,7 +95,13 @@ __device__ __forceinline__ void load_face(const MeshDev<R>& m, const R* __restri
         in.gTP[k] = rP[R_GT + k]; in.gTN[k] = rNg[R_GT + k];
         in.gpP[k] = rP[R_GP + k]; in.gpN[k] = rNg[R_GP + k];
     }
-    load_face_geometry<R, Q>(m, f, in);
+}
+
+// the 55 inputs of one face
+template <typename R, typename Q>
+__device__ __forceinline__ void load_face(const MeshDev<R>& m, const R* __restrict__ rec, int f, FaceIn<Q>& in,
+                                          unsigned* most = nullptr) {
+    load_face_cells<R, Q>(rec, load_face_mesh<R, Q>(m, f, in), in, most);
 }
 
 // soft_seen of a taped value; 1/eps of the entropy fix may be 1e30 (eps is at least `small`), in a

@@ -148,60 +148,76 @@ __device__ __forceinline__ void ghost_prims(const MeshDev<R>& m, const Phys& P, 
     if (kp == GK_FIXED) v[4] = kGauge<R> ? m.gval[4 * (size_t)m.nG + g] - gP : m.gval[4 * (size_t)m.nG + g];
 }
 
+// dtcBits (may be NULL): the step's CFL maximum, cleared here
 template <typename R, typename S>
 __global__ void __launch_bounds__(BLOCK) k_prim(MeshDev<R> m, Phys P, const S* __restrict__ rho,
                                                 const S* __restrict__ rhoU, const S* __restrict__ rhoE,
-                                                R* __restrict__ rec) {
+                                                R* __restrict__ rec, unsigned long long* dtcBits) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int g = t - m.nIC;
+    const int src = g >= 0 && g < m.nG ? m.gsrc[g] : t;
+    dep_wait(rho, rhoU, rhoE, rec);
+    if (t == 0 && dtcBits) *dtcBits = 0;
     if (t < m.nIC) {
         R v[5];
         load_prim<R, S>(P, rho, rhoU, rhoE, t, v);
         store_prims(rec + (size_t)t * REC, v);
         return;
     }
-    int g = t - m.nIC;
     if (g >= m.nG) return;
     R v[5];
-    load_prim<R, S>(P, rho, rhoU, rhoE, m.gsrc[g], v);
+    load_prim<R, S>(P, rho, rhoU, rhoE, src, v);
     ghost_prims<R>(m, P, g, v);
     store_prims(rec + (size_t)t * REC, v);
 }
 
+// the mesh side of a cell's gradient: the neighbours and the mesh-only products of
+//   sum_s phiF_s S N'_s / V with phiF_s = phi_c (1 - w'_s) + phi_nb w'_s, regrouped as
+//   phi_c sum_s (1 - w'_s) S N'_s / V + sum_s phi_nb (w'_s S N'_s / V)
+// (15 FMAs a slot; the face interpolation and the 1/V scaling were 25)
 template <typename R>
-__device__ __forceinline__ void grad_cell(const MeshDev<R>& m, const Phys& P, const R* __restrict__ rec, int c,
+struct GradSlots {
+    int nb[6];
+    R ws[18], a[3], cl[3];
+};
+template <typename R>
+__device__ __forceinline__ void load_slots(const MeshDev<R>& m, int c, GradSlots<R>& g) {
+    const size_t n = m.nIC;
+#pragma unroll
+    for (int s = 0; s < 6; s++) g.nb[s] = m.gnb[s * n + c];
+#pragma unroll
+    for (int k = 0; k < 18; k++) g.ws[k] = m.gws[k * n + c];
+    for (int j = 0; j < 3; j++) g.a[j] = m.gAv[j * n + c];
+    if constexpr (kGauge<R>)
+        for (int j = 0; j < 3; j++) g.cl[j] = m.gcl[j * n + c];
+}
+
+template <typename R>
+__device__ __forceinline__ void grad_cell(const Phys& P, const R* __restrict__ rec, int c, const GradSlots<R>& t,
                                           R* row) {
     // the five primitives of a record as one 16-byte load and a scalar (records are 16-byte
     // aligned)
     R phic[5];
     load_vec(rec + (size_t)c * REC, phic, 4);
     phic[4] = rec[(size_t)c * REC + 4];
-    // sum_s phiF_s S N'_s / V with phiF_s = phi_c (1 - w'_s) + phi_nb w'_s, regrouped as
-    // phi_c sum_s (1 - w'_s) S N'_s / V + sum_s phi_nb (w'_s S N'_s / V): the mesh-only products
-    // are tables, leaving 15 FMAs a slot (the face interpolation and the 1/V scaling were 25)
-    const size_t n = m.nIC;
     R g[15];
-    {
-        R a[3] = {m.gAv[c], m.gAv[n + c], m.gAv[2 * n + c]};
-        for (int i = 0; i < 5; i++)
-            for (int j = 0; j < 3; j++) g[3 * i + j] = phic[i] * a[j];
-    }
+    for (int i = 0; i < 5; i++)
+        for (int j = 0; j < 3; j++) g[3 * i + j] = phic[i] * t.a[j];
 #pragma unroll
     for (int s = 0; s < 6; s++) {
-        int nb = m.gnb[s * n + c];
-        R ws[3] = {m.gws[(3 * s) * n + c], m.gws[(3 * s + 1) * n + c], m.gws[(3 * s + 2) * n + c]};
+        const R* ws = t.ws + 3 * s;
         R rn[5];
-        load_vec(rec + (size_t)nb * REC, rn, 4);
-        rn[4] = rec[(size_t)nb * REC + 4];
+        load_vec(rec + (size_t)t.nb[s] * REC, rn, 4);
+        rn[4] = rec[(size_t)t.nb[s] * REC + 4];
         for (int i = 0; i < 5; i++)
             for (int j = 0; j < 3; j++) g[3 * i + j] = g[3 * i + j] + rn[i] * ws[j];
     }
     if constexpr (kGauge<R>) {
         // FP32 records hold T - gT, p - gP: the gradient of the constant offsets is the offset
         // times the cell's sum of S N'/V, which warped faces leave nonzero
-        R cl[3] = {m.gcl[c], m.gcl[n + c], m.gcl[2 * n + c]};
         for (int j = 0; j < 3; j++) {
-            g[9 + j] = g[9 + j] + consts<R>(P).gT * cl[j];
-            g[12 + j] = g[12 + j] + consts<R>(P).gP * cl[j];
+            g[9 + j] = g[9 + j] + consts<R>(P).gT * t.cl[j];
+            g[12 + j] = g[12 + j] + consts<R>(P).gP * t.cl[j];
         }
     }
     R v[REC];
@@ -220,7 +236,10 @@ __global__ void __launch_bounds__(NT) k_grad(MeshDev<R> m, Phys P, R* __restrict
     __shared__ __align__(16) R stage[NT * REC];
     const int c0 = blockIdx.x * NT;
     const int c = c0 + threadIdx.x;
-    if (c < m.nIC) grad_cell<R>(m, P, rec, c, stage + threadIdx.x * REC);
+    GradSlots<R> t;
+    if (c < m.nIC) load_slots<R>(m, c, t);
+    dep_wait(rec);
+    if (c < m.nIC) grad_cell<R>(P, rec, c, t, stage + threadIdx.x * REC);
     __syncthreads();
     if (c0 < m.nIC) store_staged<R, REC, NT>(rec, c0, min(NT, m.nIC - c0), stage);
 }
@@ -230,8 +249,7 @@ static void launch_grad(Ctx* c, R* rec, cudaStream_t s) {
     const MeshDev<R>& m = meshOf<R>(c);
     ProfScope ps(c, KID_GRAD, s);
     const Shape g = shape_for(m.nIC, BLOCK);
-    if (g.threads == 32) k_grad<R, 32><<<g.blocks, 32, 0, s>>>(m, c->phys, rec);
-    else k_grad<R, BLOCK><<<g.blocks, BLOCK, 0, s>>>(m, c->phys, rec);
+    launch_after(g.threads == 32 ? k_grad<R, 32> : k_grad<R, BLOCK>, g.blocks, g.threads, 0, s, m, c->phys, rec);
 }
 
 
@@ -241,12 +259,11 @@ static void launch_grad(Ctx* c, R* rec, cudaStream_t s) {
 // store 0 in the CFL slot and skip its square root
 // one face: Q is the type its physics computes with (R, or sd for FP64)
 template <typename R, typename Q, bool TAPED, bool CFL>
-__device__ __forceinline__ void flux_face(const MeshDev<R>& m, const Phys& P, const R* __restrict__ rec, int f,
-                                          R* __restrict__ fflux, int inviscid, R* __restrict__ tape,
-                                          unsigned* most = nullptr) {
-    int kind = (f < m.nIF) ? FACE_INTERNAL : (int)m.fkind[f - m.nIF];
-    FaceIn<Q> in;
-    load_face<R, Q>(m, rec, f, in, most);
+__device__ __forceinline__ void flux_face(const MeshDev<R>& m, const Phys& P, const FaceAt& at, FaceIn<Q>& in,
+                                          const R* __restrict__ rec, int f, R* __restrict__ fflux, int inviscid,
+                                          R* __restrict__ tape, unsigned* most = nullptr) {
+    const int kind = at.kind;
+    load_face_cells<R, Q>(rec, at, in, most);
     Q F[5], maxaF;
     // (FP32 records hold gauge offsets and their fluxes are the gauge form; only FP64
     // contexts keep face tapes)
@@ -263,7 +280,9 @@ __device__ __forceinline__ void flux_face(const MeshDev<R>& m, const Phys& P, co
 template <typename R, bool TAPED, bool CFL>
 __device__ __noinline__ void flux_face_again(const MeshDev<R>& m, const Phys& P, const R* rec, int f, R* fflux,
                                              int inviscid, R* tape) {
-    flux_face<R, R, TAPED, CFL>(m, P, rec, f, fflux, inviscid, tape);
+    FaceIn<R> in;
+    const FaceAt at = load_face_mesh<R, R>(m, f, in);
+    flux_face<R, R, TAPED, CFL>(m, P, at, in, rec, f, fflux, inviscid, tape);
 }
 
 // SOFT (FP64): products, reciprocals and square roots on the integer pipes (soft64.cuh). The FP64
@@ -278,16 +297,21 @@ __global__ void __launch_bounds__(FLUX_BLOCK, sizeof(R) == 8 ? 3 : 8)
     // (the 6-value face records are stored directly: staging them through shared memory, as
     // the 20- and 40-value records are, made this kernel slower - 0.217 -> 0.269 ms at 128^3 in
     // FP32 - the barrier costs more than the six partly coalesced stores)
-    int f = blockIdx.x * blockDim.x + threadIdx.x;
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    using Q = std::conditional_t<SOFT, sd, R>;
+    FaceIn<Q> in;
+    FaceAt at = {};
+    if (f < m.nF) at = load_face_mesh<R, Q>(m, f, in);
+    dep_wait(rec, fflux, tape);
     if (f >= m.nF) return;
     if constexpr (SOFT) {
         soft_flag() = 0;
         unsigned most = 0;
-        flux_face<R, sd, TAPED, CFL>(m, P, rec, f, fflux, inviscid, tape, &most);
+        flux_face<R, Q, TAPED, CFL>(m, P, at, in, rec, f, fflux, inviscid, tape, &most);
         if (__builtin_expect(most >= SOFT_LIMIT || soft_flag() != 0, 0))
             flux_face_again<R, TAPED, CFL>(m, P, rec, f, fflux, inviscid, tape);
     } else {
-        flux_face<R, R, TAPED, CFL>(m, P, rec, f, fflux, inviscid, tape);
+        flux_face<R, Q, TAPED, CFL>(m, P, at, in, rec, f, fflux, inviscid, tape);
     }
 }
 
@@ -308,6 +332,25 @@ __device__ __forceinline__ void load_flux_record(const double* __restrict__ p, d
     }
 }
 
+// StepEnd's work, by one block
+__device__ __forceinline__ void step_end(const StepEnd& e) {
+    __shared__ double sh[BLOCK / 32];
+    double v = 0.0;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < e.nPartials; i += blockDim.x) v += e.partials[i];
+    const double s = block_sum(v, sh);
+    if (threadIdx.x != 0) return;
+    const double dtc = __longlong_as_double((long long)*e.dtcBits);
+    *e.dtcBits = 0;
+    if (e.objOut) *e.objOut = s;
+    if (e.dtcOut) *e.dtcOut = dtc;
+    if (e.dtNext) {
+        const double d = *e.dt;
+        if (e.dtHist) *e.dtHist = d;
+        *e.dtNext = e.fixed ? d : fmin(2 * e.CFL / dtc, d * e.stepFactor);
+    }
+}
+
 // Gather of the face fluxes (op.div / op.absDiv, op.py:12-29, collated in the order of
 // density.py:390-402) and the SSP-RK3 stage update (timestep.py:35-45).
 template <typename R, typename S, int STAGE>
@@ -320,33 +363,47 @@ __global__ void __launch_bounds__(BLOCK) k_update(MeshDev<R> m, const R* __restr
                                                   const S* __restrict__ Se,
                                                   S* outr, S* outu, S* oute,
                                                   unsigned long long* dtcBits, Phys P, R* __restrict__ recNext,
-                                                  int objKind, double* __restrict__ objPartials) {
+                                                  int objKind, double* __restrict__ objPartials, StepEnd end) {
     // the gather (and the CFL sum) in the flux type R, the stage update in the state's type S:
     // under FP32 fluxes with an FP64 state the six fluxes are summed in FP32 (each carries FP32
     // rounding already; summing them in FP64 cost six FP64 conversions, products and sums a
     // cell and component) and the state is updated in FP64
+    const size_t n = m.nIC;
     int c = blockIdx.x * blockDim.x + threadIdx.x;
+    int e[6], gs0 = 0, gs1 = 0;
+    R w[6];
+    if (c < m.nIC) {
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            e[k] = m.accf[k * n + c];
+            w[k] = m.accw[k * n + c];
+        }
+        gs0 = m.gsStart[c];
+        gs1 = m.gsStart[c + 1];
+    }
+    dep_wait(fflux, dtp, u0r, u0u, u0e, u1r, u1u, u1e, u2r, u2u, u2e, Sr, Su, Se, recNext);
+    if (STAGE == 2 && end.dtcBits && blockIdx.x == gridDim.x - 1) {
+        step_end(end);
+        return;
+    }
     R dtc = R(0);
     double objv = 0.0;     // this cell's term of a cell-sum objective (stage 0, objPartials)
     if (c < m.nIC) {
-        const size_t n = m.nIC;
         // the sums start at -0, which the compiler drops from the first term's add (-0 + x is x,
         // while +0 + x is one more add; the values differ at most in the sign of a zero)
         R res[5] = {R(-0.0), R(-0.0), R(-0.0), R(-0.0), R(-0.0)};
 #pragma unroll
         for (int k = 0; k < 6; k++) {
-            int e = m.accf[k * n + c];
-            R w = m.accw[k * n + c];
-            bool ownerSide = e >= 0;
-            int f = ownerSide ? e : ~e;
+            bool ownerSide = e[k] >= 0;
+            int f = ownerSide ? e[k] : ~e[k];
             R F[FREC];
             load_flux_record(fflux + (size_t)f * FREC, F);
             // the side's sign on the weight (one select a face, not one a term); each product
             // rounded before it is added, as the reference's collate sum does, so that equal
             // and opposite terms cancel exactly
-            R ws = ownerSide ? w : -w;
+            R ws = ownerSide ? w[k] : -w[k];
             for (int q = 0; q < 5; q++) res[q] = res[q] + mul_rn(F[q], ws);
-            dtc = dtc + F[5] * w;
+            dtc = dtc + F[5] * w[k];
         }
         S rs[5];
         for (int q = 0; q < 5; q++) rs[q] = S(res[q]);
@@ -388,11 +445,11 @@ __global__ void __launch_bounds__(BLOCK) k_update(MeshDev<R> m, const R* __restr
             prim_values(P, o[0], o[1], o[2], o[3], o[4], v);
             store_prims(recNext + (size_t)c * REC, v);
             if (STAGE == 0 && objPartials) objv = cell_objective<R>(P, objKind, v, m.vol[c]);
-            for (int q = m.gsStart[c]; q < m.gsStart[c + 1]; q++) {
+            for (int q = gs0; q < gs1; q++) {
                 int g = m.gsList[q];
-                R w[5] = {v[0], v[1], v[2], v[3], v[4]};
-                ghost_prims<R>(m, P, g, w);
-                store_prims(recNext + (size_t)(m.nIC + g) * REC, w);
+                R gv[5] = {v[0], v[1], v[2], v[3], v[4]};
+                ghost_prims<R>(m, P, g, gv);
+                store_prims(recNext + (size_t)(m.nIC + g) * REC, gv);
             }
         }
     }
@@ -446,6 +503,7 @@ template <typename R>
 __global__ void __launch_bounds__(BLOCK) k_objective(MeshDev<R> m, Phys P, const R* __restrict__ rec, int kind,
                                                      int start, int n, double* partials) {
     __shared__ double sh[BLOCK / 32];
+    dep_wait(rec, partials);
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     double v = 0.0;
     if (t < n) {
@@ -474,6 +532,7 @@ template <typename R>
 __global__ void __launch_bounds__(BLOCK) k_obj_vane(MeshDev<R> m, Phys P, const R* __restrict__ rec, VaneDev v,
                                                     int nBlocks, double* partials) {
     __shared__ double sh0[BLOCK / 32], sh1[BLOCK / 32], sh2[BLOCK / 32];
+    dep_wait(rec, partials);
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     double l = 0.0, w = 0.0, h = 0.0;
     if (t < v.nPlane) {
@@ -494,10 +553,11 @@ __global__ void __launch_bounds__(BLOCK) k_obj_vane(MeshDev<R> m, Phys P, const 
 }
 
 // fixed-order sums of the vane partials into sums[0..2]; with objOut, also the objective
-// a L/W + b H/sum(A w) and the dtc bits, as k_finish does
-__global__ void k_vane_finish(const double* partials, int nBlocks, VaneDev v, double* sums,
-                              const unsigned long long* dtcBits, double* dtcOut, double* objOut) {
+// a L/W + b H/sum(A w)
+__global__ void __launch_bounds__(BLOCK) k_vane_finish(const double* partials, int nBlocks, VaneDev v, double* sums,
+                                                       double* objOut) {
     __shared__ double sh0[BLOCK / 32], sh1[BLOCK / 32], sh2[BLOCK / 32];
+    dep_wait(partials);
     double a = 0.0, b = 0.0, c = 0.0;
     for (int i = threadIdx.x; i < nBlocks; i += BLOCK) {
         a += partials[i];
@@ -510,43 +570,27 @@ __global__ void k_vane_finish(const double* partials, int nBlocks, VaneDev v, do
         sums[1] = W;
         sums[2] = H;
         if (objOut) *objOut = v.a * (L / W) + v.b * (H * v.rw2);
-        if (dtcOut) *dtcOut = __longlong_as_double((long long)*dtcBits);
     }
 }
 
 template <typename R>
-void launch_vane_sums(Ctx* c, cudaStream_t s, double* dtcOut, double* objOut, const R* rec) {
+void launch_vane_sums(Ctx* c, cudaStream_t s, double* objOut, const R* rec) {
     const MeshDev<R>& m = meshOf<R>(c);
     {
         ProfScope ps(c, KID_OBJECTIVE, s);
-        k_obj_vane<R><<<c->nVaneBlocks, BLOCK, 0, s>>>(m, c->phys, rec ? rec : (const R*)c->rec, c->vane,
-                                                      c->nVaneBlocks, c->vanePartials);
+        launch_after(k_obj_vane<R>, c->nVaneBlocks, BLOCK, 0, s, m, c->phys, rec ? rec : (const R*)c->rec, c->vane,
+                     c->nVaneBlocks, c->vanePartials);
     }
     ProfScope ps(c, KID_FINISH, s);
-    k_vane_finish<<<1, BLOCK, 0, s>>>(c->vanePartials, c->nVaneBlocks, c->vane, c->vaneSums, c->dtcBits, dtcOut,
-                                      objOut);
+    launch_after(k_vane_finish, 1, BLOCK, 0, s, c->vanePartials, c->nVaneBlocks, c->vane, c->vaneSums, objOut);
 }
-
-// fixed-order final sum of the partials (deterministic) and the dtc bits -> double
-__global__ void k_finish(const double* partials, int nPartials, const unsigned long long* dtcBits,
-                         double* dtcOut, double* objOut, int haveObj) {
-    __shared__ double sh[BLOCK / 32];
-    double v = 0.0;
-    for (int i = threadIdx.x; i < nPartials; i += BLOCK) v += partials[i];
-    double s = block_sum(haveObj ? v : 0.0, sh);
-    if (threadIdx.x == 0) {
-        if (objOut) *objOut = haveObj ? s : 0.0;
-        if (dtcOut) *dtcOut = __longlong_as_double((long long)*dtcBits);
-    }
-}
-
 
 template <typename R, typename S>
 void launch_prim(Ctx* c, const S* r, const S* ru, const S* re, cudaStream_t s, R* rec) {
     const MeshDev<R>& m = meshOf<R>(c);
     ProfScope ps(c, KID_PRIM, s);
     const Shape g = shape_for((long long)m.nIC + m.nG, BLOCK);
-    k_prim<R, S><<<g.blocks, g.threads, 0, s>>>(m, c->phys, r, ru, re, rec ? rec : (R*)c->rec);
+    launch_after(k_prim<R, S>, g.blocks, g.threads, 0, s, m, c->phys, r, ru, re, rec ? rec : (R*)c->rec, c->dtcBits);
 }
 
 template <typename R, typename S>
@@ -561,7 +605,7 @@ void launch_prim_grad(Ctx* c, const S* r, const S* ru, const S* re, cudaStream_t
 template <typename R, typename S>
 void launch_flux_update(Ctx* c, int st, double dt, const double* dtDev, const S* const* u0, const S* const* u1,
                         const S* const* u2, const S* Sr, const S* Su, const S* Se, S* const* out, cudaStream_t s,
-                        bool nextPrims, R* tape, R* recIn, R* recOut, double* objPartials) {
+                        bool nextPrims, R* tape, R* recIn, R* recOut, double* objPartials, const StepEnd* end) {
     const MeshDev<R>& m = meshOf<R>(c);
     const Phys& P = c->phys;
     R* rec = recIn ? recIn : (R*)c->rec;
@@ -571,8 +615,8 @@ void launch_flux_update(Ctx* c, int st, double dt, const double* dtDev, const S*
         ProfScope ps(c, KID_FLUX, s);
         const Shape g = shape_for(m.nF, FLUX_BLOCK);
         auto flux = [&](auto taped, auto cfl, auto soft) {
-            k_flux<R, decltype(taped)::value, decltype(cfl)::value, decltype(soft)::value>
-                <<<g.blocks, g.threads, 0, s>>>(m, P, rec, ff, inviscid, tape);
+            launch_after(k_flux<R, decltype(taped)::value, decltype(cfl)::value, decltype(soft)::value>, g.blocks,
+                         g.threads, 0, s, m, P, rec, ff, inviscid, tape);
         };
         auto by_cfl = [&](auto taped, auto soft) {
             if (st == 1) flux(taped, std::true_type{}, soft);
@@ -591,18 +635,20 @@ void launch_flux_update(Ctx* c, int st, double dt, const double* dtDev, const S*
     const Shape g = shape_for(m.nIC, BLOCK);
     R* recNext = nextPrims ? (recOut ? recOut : rec) : nullptr;
     ProfScope ps(c, KID_UPDATE, s);
+    const S* none = nullptr;
+    const StepEnd noEnd = {};
     if (st == 0)
-        k_update<R, S, 0><<<g.blocks, g.threads, 0, s>>>(m, ff, dt, dtDev, u0[0], u0[1], u0[2], nullptr, nullptr, nullptr, nullptr,
-                                            nullptr, nullptr, Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P,
-                                            recNext, c->objective, recNext ? objPartials : nullptr);
+        launch_after(k_update<R, S, 0>, g.blocks, g.threads, 0, s, m, ff, dt, dtDev, u0[0], u0[1], u0[2], none, none,
+                     none, none, none, none, Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P, recNext, c->objective,
+                     recNext ? objPartials : nullptr, noEnd);
     else if (st == 1)
-        k_update<R, S, 1><<<g.blocks, g.threads, 0, s>>>(m, ff, dt, dtDev, u0[0], u0[1], u0[2], u1[0], u1[1], u1[2], nullptr,
-                                            nullptr, nullptr, Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P,
-                                            recNext, c->objective, nullptr);
+        launch_after(k_update<R, S, 1>, g.blocks, g.threads, 0, s, m, ff, dt, dtDev, u0[0], u0[1], u0[2], u1[0], u1[1],
+                     u1[2], none, none, none, Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P, recNext, c->objective,
+                     (double*)nullptr, noEnd);
     else
-        k_update<R, S, 2><<<g.blocks, g.threads, 0, s>>>(m, ff, dt, dtDev, u0[0], u0[1], u0[2], nullptr, nullptr, nullptr, u2[0],
-                                            u2[1], u2[2], Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P,
-                                            recNext, c->objective, nullptr);
+        launch_after(k_update<R, S, 2>, g.blocks + (end ? 1 : 0), g.threads, 0, s, m, ff, dt, dtDev, u0[0], u0[1], u0[2],
+                     none, none, none, u2[0], u2[1], u2[2], Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P, recNext,
+                     c->objective, (double*)nullptr, end ? *end : noEnd);
 }
 
 template <typename S>
@@ -616,7 +662,8 @@ void default_sources(Ctx* c, const S*& Srho, const S*& SrhoU, const S*& SrhoE) {
 template <typename R, typename S>
 int primal_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double dt, const double* dtDev,
                     const S* Srho, const S* SrhoU, const S* SrhoE, S* rhoN, S* rhoUN, S* rhoEN,
-                    double* dtcDev, double* objDev, cudaStream_t s, S* stages, R* tape) {
+                    double* dtcDev, double* objDev, cudaStream_t s, S* stages, R* tape, const StepEnd* rule,
+                    bool primsReady, bool nextStep) {
     const MeshDev<R>& m = meshOf<R>(c);
     const Phys& P = c->phys;
     default_sources<S>(c, Srho, SrhoU, SrhoE);
@@ -627,9 +674,7 @@ int primal_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double d
     const S* u0c[3] = {rho, rhoU, rhoE};
     const S* u1c[3] = {u1[0], u1[1], u1[2]};
     const S* u2c[3] = {u2[0], u2[1], u2[2]};
-    cudaMemsetAsync(c->dtcBits, 0, sizeof(unsigned long long), s);
     int nObjBlocks = 0;
-    bool vaneDone = false;
     if (c->objective == AFVM_OBJ_VANE && !c->vaneSet)
         return fail(c, AFVM_ERR_BAD_ARG, "AFVM_OBJ_VANE needs afvm_set_objective_vane before the first step");
     // with a tape each stage's cell records are built in the tape's record part (kept for the
@@ -641,12 +686,10 @@ int primal_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double d
     for (int st = 0; st < 3; st++) recs[st] = recTape ? recTape + (size_t)st * m.nC * REC : (R*)c->rec;
     for (int st = 0; st < 3; st++) {
         const S* const* in = st == 0 ? u0c : (st == 1 ? u1c : u2c);
-        if (st == 0) {
-            launch_prim_grad<R, S>(c, in[0], in[1], in[2], s, recs[0]);
-        } else {
-            // the primitives of stages 1 and 2 were written by the previous stage's update
-            launch_grad<R>(c, recs[st], s);
-        }
+        // the primitives of stages 1 and 2, and of a step that follows another in primal_run_dev,
+        // were written by the update before
+        if (st == 0 && !primsReady) launch_prim<R, S>(c, in[0], in[1], in[2], s, recs[0]);
+        launch_grad<R>(c, recs[st], s);
         if (st == 1 && c->objSink) {
             // the objective stage's primitives U (3), T, p of every cell, ghosts included, for an
             // objective evaluated by the caller (absolute values: FP32 records add their gauge)
@@ -657,12 +700,7 @@ int primal_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double d
                                   cudaMemcpyDeviceToDevice, s);
         }
         if (st == 1 && c->objective == AFVM_OBJ_VANE) {
-            // the partial sums now, while rec holds the stage-1 primitives; combined at the end
-            const MeshDev<R>& mm = meshOf<R>(c);
-            ProfScope ps(c, KID_OBJECTIVE, s);
-            k_obj_vane<R><<<c->nVaneBlocks, BLOCK, 0, s>>>(mm, P, (const R*)recs[1], c->vane, c->nVaneBlocks,
-                                                          c->vanePartials);
-            vaneDone = true;
+            launch_vane_sums<R>(c, s, objDev, (const R*)recs[1]);
         } else if (st == 1 && c->objective != AFVM_OBJ_NONE) {
             int start = 0, n = m.nIC;
             if (c->objective == AFVM_OBJ_DRAG) { start = c->objStart; n = c->objN; }
@@ -672,8 +710,8 @@ int primal_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double d
             // a cell-sum objective's partials were written by the stage-0 update
             if (n > 0 && !cell_sum_objective(c->objective)) {
                 ProfScope ps(c, KID_OBJECTIVE, s);
-                k_objective<R><<<nObjBlocks, g.threads, 0, s>>>(m, P, (const R*)recs[1], c->objective, start, n,
-                                                            c->partials);
+                launch_after(k_objective<R>, nObjBlocks, g.threads, 0, s, m, P, (const R*)recs[1], c->objective, start,
+                             n, c->partials);
             }
         }
         S* const* out = st == 0 ? u1 : (st == 1 ? u2 : outN);
@@ -682,43 +720,44 @@ int primal_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double d
                                   ? c->partials : nullptr;
         if (st == 0 && cell_sum_objective(c->objective) && !objPartials)
             return fail(c, AFVM_ERR_BAD_ARG, "objective partials overflow");
-        launch_flux_update<R, S>(c, st, dt, dtDev, u0c, u1c, u2c, Srho, SrhoU, SrhoE, out, s, st < 2,
+        StepEnd end = {};
+        if (st == 2) {
+            if (rule) end = *rule;
+            end.partials = c->partials;
+            end.nPartials = nObjBlocks;
+            end.dtcBits = c->dtcBits;
+            end.dtcOut = dtcDev;
+            end.objOut = c->objective == AFVM_OBJ_VANE ? nullptr : objDev;    // (k_vane_finish's)
+        }
+        launch_flux_update<R, S>(c, st, dt, dtDev, u0c, u1c, u2c, Srho, SrhoU, SrhoE, out, s, st < 2 || nextStep,
                                  faceTape ? faceTape + (size_t)st * TAPE * m.nF : nullptr, recs[st],
-                                 st < 2 ? recs[st + 1] : nullptr, objPartials);
-    }
-    if (vaneDone) {
-        ProfScope ps(c, KID_FINISH, s);
-        k_vane_finish<<<1, BLOCK, 0, s>>>(c->vanePartials, c->nVaneBlocks, c->vane, c->vaneSums, c->dtcBits, dtcDev,
-                                          objDev);
-    } else {
-        ProfScope ps(c, KID_FINISH, s);
-        k_finish<<<1, BLOCK, 0, s>>>(c->partials, nObjBlocks, c->dtcBits, dtcDev, objDev, nObjBlocks > 0);
+                                 st < 2 ? recs[st + 1] : nullptr, objPartials, st == 2 ? &end : nullptr);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "primal step launch");
     return AFVM_OK;
 }
 
-// time-step rule of the reference loop, dt <- min(2*CFL/dtc, stepFactor*dt)
-// (adFVM/solver.py:365), kept on the device; records the dt each step used
-__global__ void k_next_dt(double* dt, const double* dtc, double CFL, double stepFactor, int fixed, double* dtHist) {
-    double d = *dt;
-    if (dtHist) *dtHist = d;
-    if (!fixed) *dt = fmin(2 * CFL / *dtc, d * stepFactor);
-}
-
 template <typename R, typename S>
 int primal_run_dev(Ctx* c, S* rho, S* rhoU, S* rhoE, int nSteps, double dt0, double CFL, double stepFactor,
                    int fixed, const S* Srho, const S* SrhoU, const S* SrhoE, double* dtHist, double* dtcHist,
                    double* objHist, cudaStream_t s) {
-    double* dtDev = c->scal + 2;
-    cudaMemcpyAsync(dtDev, &dt0, sizeof(double), cudaMemcpyHostToDevice, s);
+    // the step's dt and the next one's in turn; each step's last update writes the next step's
+    // primitives as well
+    double* dtDev[2] = {c->scal + 2, c->scal + 3};
+    cudaMemcpyAsync(dtDev[0], &dt0, sizeof(double), cudaMemcpyHostToDevice, s);
     for (int n = 0; n < nSteps; n++) {
-        double* dtcOut = dtcHist ? dtcHist + n : c->scal;
-        int st = primal_step_dev<R, S>(c, rho, rhoU, rhoE, 0.0, dtDev, Srho, SrhoU, SrhoE, rho, rhoU, rhoE, dtcOut,
-                                    objHist ? objHist + n : c->scal + 1, s);
+        StepEnd rule = {};
+        rule.dt = dtDev[n & 1];
+        rule.dtNext = dtDev[(n + 1) & 1];
+        rule.dtHist = dtHist ? dtHist + n : nullptr;
+        rule.CFL = CFL;
+        rule.stepFactor = stepFactor;
+        rule.fixed = fixed;
+        int st = primal_step_dev<R, S>(c, rho, rhoU, rhoE, 0.0, dtDev[n & 1], Srho, SrhoU, SrhoE, rho, rhoU, rhoE,
+                                    dtcHist ? dtcHist + n : c->scal, objHist ? objHist + n : c->scal + 1, s, nullptr,
+                                    nullptr, &rule, n > 0, n + 1 < nSteps);
         if (st != AFVM_OK) return st;
-        k_next_dt<<<1, 1, 0, s>>>(dtDev, dtcOut, CFL, stepFactor, fixed, dtHist ? dtHist + n : nullptr);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "primal run launch");
@@ -727,20 +766,21 @@ int primal_run_dev(Ctx* c, S* rho, S* rhoU, S* rhoE, int nSteps, double dt0, dou
 
 #define AFVM_PRIMAL_INST(R, S)                                                                                 \
     template int primal_step_dev<R, S>(Ctx*, const S*, const S*, const S*, double, const double*, const S*,       \
-                                       const S*, const S*, S*, S*, S*, double*, double*, cudaStream_t, S*, R*);   \
+                                       const S*, const S*, S*, S*, S*, double*, double*, cudaStream_t, S*, R*,    \
+                                       const StepEnd*, bool, bool);                                                 \
     template int primal_run_dev<R, S>(Ctx*, S*, S*, S*, int, double, double, double, int, const S*, const S*,     \
                                       const S*, double*, double*, double*, cudaStream_t);                         \
     template void launch_prim<R, S>(Ctx*, const S*, const S*, const S*, cudaStream_t, R*);                       \
     template void launch_prim_grad<R, S>(Ctx*, const S*, const S*, const S*, cudaStream_t, R*);                  \
     template void launch_flux_update<R, S>(Ctx*, int, double, const double*, const S* const*, const S* const*,   \
                                            const S* const*, const S*, const S*, const S*, S* const*, cudaStream_t,  \
-                                           bool, R*, R*, R*, double*);
+                                           bool, R*, R*, R*, double*, const StepEnd*);
 AFVM_PRIMAL_INST(double, double)
 AFVM_PRIMAL_INST(float, float)
 AFVM_PRIMAL_INST(float, double)
 template void default_sources<double>(Ctx*, const double*&, const double*&, const double*&);
 template void default_sources<float>(Ctx*, const float*&, const float*&, const float*&);
-template void launch_vane_sums<double>(Ctx*, cudaStream_t, double*, double*, const double*);
-template void launch_vane_sums<float>(Ctx*, cudaStream_t, double*, double*, const float*);
+template void launch_vane_sums<double>(Ctx*, cudaStream_t, double*, const double*);
+template void launch_vane_sums<float>(Ctx*, cudaStream_t, double*, const float*);
 
 }  // namespace afvm

@@ -51,3 +51,26 @@ def test_step_and_adjoint_at_the_edges_of_a_block(name, n):
             assert G.rel_err(a[i].cpu().numpy(), refa[i].numpy()) < 1e-12, (name, n, i)
     assert abs(out[3] - float(ref[3])) <= 1e-12 * abs(float(ref[3]))
     assert abs(out[4] - float(ref[4])) <= 1e-12 * max(abs(float(ref[4])), 1e-300)
+
+
+@pytest.mark.parametrize('name', ['tube', 'box', 'cylinder', 'channel'])
+@pytest.mark.parametrize('steps', [1, 2, 5])
+def test_a_device_run_is_its_steps(name, steps):
+    """RCF.run_device (whose steps write the next one's primitives and its dt on the device) against
+    the same steps one call at a time with the dt rule on the host: the same bits. The histories
+    cover each kind of objective: none, a cell sum, a face sum, the vane's."""
+    case = {'tube': lambda: cases.sod(100), 'box': lambda: cases.box(8), 'cylinder': lambda: cases.cylinder(32, 16),
+            'channel': lambda: cases.vane_channel(32, 12)}[name]()
+    config = dict(case.config, fixedTimeStep=False)
+    rcf = RCF(case.build_mesh(), case.bc, objective=case.objective, **config)
+    x = [torch.as_tensor(a).cuda() for a in cases.conservative(case)]
+    y = [t.clone() for t in x]
+    dt, want = case.dt, []
+    for _ in range(steps):
+        r = rcf.step(*x, dt)
+        x = list(r[:3])
+        want.append((dt, r[3], r[4]))
+        dt = min(2 * rcf.CFL / r[3], dt * rcf.stepFactor)
+    hist = rcf.run_device(*y, steps, case.dt).cpu().numpy()
+    assert all(torch.equal(a, b) for a, b in zip(x, y))
+    assert np.array_equal(hist[:, :steps].T, np.array(want))

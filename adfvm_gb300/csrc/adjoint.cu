@@ -280,22 +280,58 @@ __global__ void __launch_bounds__(NT) k_adj_cell1(MeshDev<R> m, const R* __restr
 }
 
 
+// the split form (CellAt): warp q of a block sums values 4q..4q+3 of 32 cells
+template <typename R>
+__global__ void __launch_bounds__(160) k_adj_cell1_split(MeshDev<R> m, const R* __restrict__ fadj, R* __restrict__ cbar) {
+    __shared__ __align__(16) R stage[32 * CBAR];
+    const CellAt<true> at;
+    const int c = at.c, k0 = 4 * at.q0, c0 = blockIdx.x * 32;
+    int e[6], gs0 = 0, gs1 = 0;
+    if (c < m.nIC) {
+#pragma unroll
+        for (int s = 0; s < 6; s++) e[s] = m.accf[s * (size_t)m.nIC + c];
+        gs0 = m.gsStart[c];
+        gs1 = m.gsStart[c + 1];
+    }
+    dep_wait(fadj, cbar);
+    if (c < m.nIC) {
+        R v[6][4], acc[4];
+#pragma unroll
+        for (int s = 0; s < 6; s++) {
+            const bool ownerSide = e[s] >= 0;
+            load_vec(fadj + (size_t)(ownerSide ? e[s] : ~e[s]) * FADJ + (ownerSide ? 0 : CBAR) + k0, v[s], 4);
+        }
+        for (int k = 0; k < 4; k++) acc[k] = v[0][k];
+#pragma unroll
+        for (int s = 1; s < 6; s++)
+            for (int k = 0; k < 4; k++) acc[k] += v[s][k];
+        for (int q = gs0; q < gs1; q++) {
+            const R* r = fadj + (size_t)(m.nIF + m.gsList[q]) * FADJ + CBAR + k0;
+            for (int k = 0; k < 4; k++)
+                if (k0 + k >= 5) acc[k] += r[k];
+        }
+        for (int k = 0; k < 4; k++) stage[(threadIdx.x & 31) * CBAR + k0 + k] = acc[k];
+    }
+    __syncthreads();
+    if (c0 < m.nIC) store_staged<R, CBAR, 160>(cbar, c0, min(32, m.nIC - c0), stage);
+}
+
 // phiFbar_i = rv * sum_j G[i][j] sn_j  (transpose of grad += phiF (x) S N', scaled by 1/V)
 template <typename R>
 __device__ __forceinline__ void phi_bar(const R* G, const R* sn, R rv, R* pb) {
     for (int i = 0; i < 5; i++) pb[i] = rv * (G[3 * i] * sn[0] + G[3 * i + 1] * sn[1] + G[3 * i + 2] * sn[2]);
 }
 
-template <typename R, typename S, int STAGE>
-__global__ void __launch_bounds__(BLOCK) k_adj_cell2(MeshDev<R> m, Phys P, const R* __restrict__ rec,
-                                                     const R* __restrict__ fadj, const R* __restrict__ cbar,
-                                                     const S* __restrict__ ur, const S* __restrict__ uu,
-                                                     const S* __restrict__ ue,
-                                                     const S* ainr, const S* ainu, const S* aine,
-                                                     S* a1r, S* a1u, S* a1e, S* a0r, S* a0u, S* a0e, S* sb,
-                                                     S* sr, S* su, S* se, double dt, int objective, int objStart, int objN, double obja,
-                                                     VaneDev vane, const double* __restrict__ objSeed) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+template <typename R, typename S, int STAGE, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 160 : BLOCK)
+    k_adj_cell2(MeshDev<R> m, Phys P, const R* __restrict__ rec, const R* __restrict__ fadj,
+                const R* __restrict__ cbar, const S* __restrict__ ur, const S* __restrict__ uu,
+                const S* __restrict__ ue, const S* ainr, const S* ainu, const S* aine, S* a1r, S* a1u, S* a1e, S* a0r,
+                S* a0u, S* a0e, S* sb, S* sr, S* su, S* se, double dt, int objective, int objStart, int objN,
+                double obja, VaneDev vane, const double* __restrict__ objSeed) {
+    const CellAt<SPLIT> at;
+    const int c = at.c;
+    const bool first = !SPLIT || at.q0 == 0;        // the thread that goes on with the whole cell
     const size_t n = m.nIC;
     const size_t nF = m.nF;
     int nb[6], gs0 = 0, gs1 = 0;
@@ -306,187 +342,219 @@ __global__ void __launch_bounds__(BLOCK) k_adj_cell2(MeshDev<R> m, Phys P, const
 #pragma unroll
         for (int k = 0; k < 18; k++) bs[k] = m.gbs[k * n + c];
         for (int j = 0; j < 3; j++) A[j] = m.gAv[j * n + c];
-        gs0 = m.gsStart[c];
-        gs1 = m.gsStart[c + 1];
+        if (first) {
+            gs0 = m.gsStart[c];
+            gs1 = m.gsStart[c + 1];
+        }
     }
     dep_wait(rec, fadj, cbar, ur, uu, ue, ainr, ainu, aine, a1r, a1u, a1e, a0r, a0u, a0e, sb, objSeed);
-    if (c >= m.nIC) return;
-    // cell adjoint records in 16-byte loads (a record is 80 / 160 bytes, 16-byte aligned)
-    R cb[CBAR];
-    load_vec(cbar + (size_t)c * CBAR, cb, CBAR);
     R pbar[5];
-    for (int k = 0; k < 5; k++) pbar[k] = cb[k];
-    const R* G = cb + 5;
-    {
+    if constexpr (SPLIT) {
+        __shared__ R sh[5 * 32];
+        const int q = at.q0, lane = threadIdx.x & 31;
+        if (c < m.nIC) {
+            const R* r = cbar + (size_t)c * CBAR;
+            R p = r[q], Gn[6][3];
+            const R G[3] = {r[5 + 3 * q], r[6 + 3 * q], r[7 + 3 * q]};
+#pragma unroll
+            for (int s = 0; s < 6; s++)
+                if (nb[s] < m.nIC)
+                    for (int j = 0; j < 3; j++) Gn[s][j] = cbar[(size_t)nb[s] * CBAR + 5 + 3 * q + j];
+            p += G[0] * A[0] + G[1] * A[1] + G[2] * A[2];
+#pragma unroll
+            for (int s = 0; s < 6; s++)
+                if (nb[s] < m.nIC) p += Gn[s][0] * bs[3 * s] + Gn[s][1] * bs[3 * s + 1] + Gn[s][2] * bs[3 * s + 2];
+            sh[q * 32 + lane] = p;
+        }
+        __syncthreads();
+        for (int i = 0; i < 5; i++) pbar[i] = sh[i * 32 + lane];
+    } else {
+        if (c >= m.nIC) return;
+        // cell adjoint records in 16-byte loads (a record is 80 / 160 bytes, 16-byte aligned)
+        R cb[CBAR];
+        load_vec(cbar + (size_t)c * CBAR, cb, CBAR);
+        for (int k = 0; k < 5; k++) pbar[k] = cb[k];
+        const R* G = cb + 5;
         // the cell's own slots at once: sum_s (1 - w'_s) (G . S N'_s) / V = G . gAv
         for (int i = 0; i < 5; i++) pbar[i] += G[3 * i] * A[0] + G[3 * i + 1] * A[1] + G[3 * i + 2] * A[2];
-    }
 #pragma unroll
-    for (int s = 0; s < 6; s++) {
-        if (nb[s] < m.nIC) {
-            // neighbour's gradient: its slot for this face has S N'' = -S N' and weight gwb;
-            // gbs_s = -gwb_s S N'_s / V_nb
-            const R* b = bs + 3 * s;
-            R cn[CBAR];
-            load_vec(cbar + (size_t)nb[s] * CBAR, cn, CBAR);
-            const R* Gn = cn + 5;
-            for (int i = 0; i < 5; i++) pbar[i] += Gn[3 * i] * b[0] + Gn[3 * i + 1] * b[1] + Gn[3 * i + 2] * b[2];
-        }
-    }
-    // ghost cells whose boundary value comes from this cell: transpose of the BC
-    for (int q = gs0; q < gs1; q++) {
-        int g = m.gsList[q];
-        int f = m.nIF + g;
-        int o = m.own[f];
-        int s = m.gslot[g];
-        R gp[5];
-        const R* r = fadj + (size_t)f * FADJ;
-        for (int k = 0; k < 5; k++) gp[k] = r[20 + k];
-        R sn[3] = {m.gsn[(3 * s) * n + o], m.gsn[(3 * s + 1) * n + o], m.gsn[(3 * s + 2) * n + o]};
-        R w = m.gw[s * n + o];
-        R pb[5];
-        phi_bar<R>(cbar + (size_t)o * CBAR + 5, sn, m.rvol[o], pb);
-        for (int k = 0; k < 5; k++) gp[k] += w * pb[k];
-        if (STAGE == 1 && objective == AFVM_OBJ_DRAG && f >= objStart && f < objStart + objN) {
-            // drag = sum (p0 nx - mu(T0) (U0 - U0i)/delta) A, ghost values p0, T0, U0
-            const R* rg = rec + (size_t)(m.nIC + g) * REC;
-            const R* ro = rec + (size_t)o * REC;
-            double T0 = rec_T<R>(P, rg[R_T]), U0 = rg[0], U0i = ro[0];
-            double A = m.area[f], dl = m.dlt[f], nx = m.nrm[f];
-            double mu = viscosity<double>(P, T0);
-            double dmu = (P.muModel == AFVM_MU_SUTHERLAND) ? mu * (1.5 / T0 - 1.0 / (T0 + P.muTs)) : 0.0;
-            gp[R_P] += (R)(obja * nx * A);
-            gp[R_T] += (R)(-obja * dmu * (U0 - U0i) / dl * A);
-            gp[0] += (R)(-obja * mu / dl * A);
-        }
-        if (STAGE == 1 && objSeed)
-            for (int k = 0; k < 5; k++) gp[k] += (R)(obja * objSeed[(size_t)(m.nIC + g) * 5 + k]);
-        int kind = m.gkind[g];
-        int kU = kind & 7, kT = (kind >> 3) & 7, kp = (kind >> 6) & 7;
-        if (kU == GK_TOTALPT) {
-            // transpose of Ub = (U.d) d, Tb = Tt - (U.d)^2/(2 Cp), pb = pt (T/Tt)^kappa
-            const R* rs = rec + (size_t)c * REC;      // this cell is the ghost's source (owner)
-            R d[3] = {m.gval[g], m.gval[(size_t)m.nG + g], m.gval[2 * (size_t)m.nG + g]};
-            R Tt = m.gval[3 * (size_t)m.nG + g], pt = m.gval[4 * (size_t)m.nG + g];
-            R Un = rs[0] * d[0] + rs[1] * d[1] + rs[2] * d[2];
-            R kap = consts<R>(P).ggm1;
-            R Unb = dot3(gp, d) - gp[R_T] * Un / consts<R>(P).Cp;
-            for (int k = 0; k < 3; k++) pbar[k] += Unb * d[k];
-            pbar[R_T] += gp[R_P] * pt * kap * pow(rec_abs_T<R>(P, rs[R_T]) / Tt, kap - R(1)) / Tt;
-            continue;
-        }
-        if (kU == GK_COPY) {
-            for (int k = 0; k < 3; k++) pbar[k] += gp[k];
-        } else if (kU == GK_SYM) {
-            R nr[3] = {m.nrm[f], m.nrm[nF + f], m.nrm[2 * nF + f]};
-            R un = dot3(gp, nr);
-            for (int k = 0; k < 3; k++) pbar[k] += gp[k] - un * nr[k];
-        }
-        if (kT != GK_FIXED) pbar[R_T] += gp[R_T];
-        if (kp != GK_FIXED) pbar[R_P] += gp[R_P];
-    }
-    // an objective evaluated by the caller: its gradient with respect to this cell's primitives
-    if (STAGE == 1 && objSeed)
-        for (int k = 0; k < 5; k++) pbar[k] += (R)(obja * objSeed[(size_t)c * 5 + k]);
-    // objective on the stage-1 primitives
-    if (STAGE == 1 && objective != AFVM_OBJ_NONE) {
-        const R* rc = rec + (size_t)c * REC;
-        if (objective == AFVM_OBJ_KINETIC_ENERGY) {
-            double U[3] = {rc[0], rc[1], rc[2]}, T = rec_T<R>(P, rc[R_T]), p = rec_p<R>(P, rc[R_P]), V = m.vol[c];
-            double d = (P.Cv * T) * P.gm1;
-            double rd = rcp(d);           // (Newton reciprocals: no IEEE divisions on the FP64 pipe)
-            double rho = p * rd;
-            double q = U[0] * U[0] + U[1] * U[1] + U[2] * U[2];
-            for (int k = 0; k < 3; k++) pbar[k] += (R)(obja * rho * U[k] * V);
-            pbar[R_P] += (R)(obja * 0.5 * q * V * rd);
-            pbar[R_T] += (R)(-obja * 0.5 * q * V * rho * rcp(T));
-        } else if (objective == AFVM_OBJ_SUM_T) {
-            pbar[R_T] += (R)obja;
-        } else if (objective == AFVM_OBJ_VANE) {
-            int q = vane.cellPlane[c];
-            if (q >= 0) {
-                double g5[5] = {0, 0, 0, 0, 0};
-                double U[3] = {rc[0], rc[1], rc[2]};
-                vane_cell_grad(P, vane, U, rec_T<R>(P, rc[R_T]), rec_p<R>(P, rc[R_P]), vane.planeArea[q], vane.sums[0],
-                               vane.sums[1], obja, g5);
-                for (int k = 0; k < 5; k++) pbar[k] += (R)g5[k];
+        for (int s = 0; s < 6; s++) {
+            if (nb[s] < m.nIC) {
+                // neighbour's gradient: its slot for this face has S N'' = -S N' and weight gwb;
+                // gbs_s = -gwb_s S N'_s / V_nb
+                const R* b = bs + 3 * s;
+                R cn[CBAR];
+                load_vec(cbar + (size_t)nb[s] * CBAR, cn, CBAR);
+                const R* Gn = cn + 5;
+                for (int i = 0; i < 5; i++) pbar[i] += Gn[3 * i] * b[0] + Gn[3 * i + 1] * b[1] + Gn[3 * i + 2] * b[2];
             }
-            if (vane.b != 0.0) {
+        }
+    }
+    S J[5];
+    auto whole_cell = [&]() {
+        // ghost cells whose boundary value comes from this cell: transpose of the BC
+        for (int q = gs0; q < gs1; q++) {
+            int g = m.gsList[q];
+            int f = m.nIF + g;
+            int o = m.own[f];
+            int s = m.gslot[g];
+            R gp[5];
+            const R* r = fadj + (size_t)f * FADJ;
+            for (int k = 0; k < 5; k++) gp[k] = r[20 + k];
+            R sn[3] = {m.gsn[(3 * s) * n + o], m.gsn[(3 * s + 1) * n + o], m.gsn[(3 * s + 2) * n + o]};
+            R w = m.gw[s * n + o];
+            R pb[5];
+            phi_bar<R>(cbar + (size_t)o * CBAR + 5, sn, m.rvol[o], pb);
+            for (int k = 0; k < 5; k++) gp[k] += w * pb[k];
+            if (STAGE == 1 && objective == AFVM_OBJ_DRAG && f >= objStart && f < objStart + objN) {
+                // drag = sum (p0 nx - mu(T0) (U0 - U0i)/delta) A, ghost values p0, T0, U0
+                const R* rg = rec + (size_t)(m.nIC + g) * REC;
+                const R* ro = rec + (size_t)o * REC;
+                double T0 = rec_T<R>(P, rg[R_T]), U0 = rg[0], U0i = ro[0];
+                double A = m.area[f], dl = m.dlt[f], nx = m.nrm[f];
+                double mu = viscosity<double>(P, T0);
+                double dmu = (P.muModel == AFVM_MU_SUTHERLAND) ? mu * (1.5 / T0 - 1.0 / (T0 + P.muTs)) : 0.0;
+                gp[R_P] += (R)(obja * nx * A);
+                gp[R_T] += (R)(-obja * dmu * (U0 - U0i) / dl * A);
+                gp[0] += (R)(-obja * mu / dl * A);
+            }
+            if (STAGE == 1 && objSeed)
+                for (int k = 0; k < 5; k++) gp[k] += (R)(obja * objSeed[(size_t)(m.nIC + g) * 5 + k]);
+            int kind = m.gkind[g];
+            int kU = kind & 7, kT = (kind >> 3) & 7, kp = (kind >> 6) & 7;
+            if (kU == GK_TOTALPT) {
+                // transpose of Ub = (U.d) d, Tb = Tt - (U.d)^2/(2 Cp), pb = pt (T/Tt)^kappa
+                const R* rs = rec + (size_t)c * REC;      // this cell is the ghost's source (owner)
+                R d[3] = {m.gval[g], m.gval[(size_t)m.nG + g], m.gval[2 * (size_t)m.nG + g]};
+                R Tt = m.gval[3 * (size_t)m.nG + g], pt = m.gval[4 * (size_t)m.nG + g];
+                R Un = rs[0] * d[0] + rs[1] * d[1] + rs[2] * d[2];
+                R kap = consts<R>(P).ggm1;
+                R Unb = dot3(gp, d) - gp[R_T] * Un / consts<R>(P).Cp;
+                for (int k = 0; k < 3; k++) pbar[k] += Unb * d[k];
+                pbar[R_T] += gp[R_P] * pt * kap * pow(rec_abs_T<R>(P, rs[R_T]) / Tt, kap - R(1)) / Tt;
+                continue;
+            }
+            if (kU == GK_COPY) {
+                for (int k = 0; k < 3; k++) pbar[k] += gp[k];
+            } else if (kU == GK_SYM) {
+                R nr[3] = {m.nrm[f], m.nrm[nF + f], m.nrm[2 * nF + f]};
+                R un = dot3(gp, nr);
+                for (int k = 0; k < 3; k++) pbar[k] += gp[k] - un * nr[k];
+            }
+            if (kT != GK_FIXED) pbar[R_T] += gp[R_T];
+            if (kp != GK_FIXED) pbar[R_P] += gp[R_P];
+        }
+        // an objective evaluated by the caller: its gradient with respect to this cell's primitives
+        if (STAGE == 1 && objSeed)
+            for (int k = 0; k < 5; k++) pbar[k] += (R)(obja * objSeed[(size_t)c * 5 + k]);
+        // objective on the stage-1 primitives
+        if (STAGE == 1 && objective != AFVM_OBJ_NONE) {
+            const R* rc = rec + (size_t)c * REC;
+            if (objective == AFVM_OBJ_KINETIC_ENERGY) {
+                double U[3] = {rc[0], rc[1], rc[2]}, T = rec_T<R>(P, rc[R_T]), p = rec_p<R>(P, rc[R_P]), V = m.vol[c];
+                double d = (P.Cv * T) * P.gm1;
+                double rd = rcp(d);           // (Newton reciprocals: no IEEE divisions on the FP64 pipe)
+                double rho = p * rd;
+                double q = U[0] * U[0] + U[1] * U[1] + U[2] * U[2];
+                for (int k = 0; k < 3; k++) pbar[k] += (R)(obja * rho * U[k] * V);
+                pbar[R_P] += (R)(obja * 0.5 * q * V * rd);
+                pbar[R_T] += (R)(-obja * 0.5 * q * V * rho * rcp(T));
+            } else if (objective == AFVM_OBJ_SUM_T) {
+                pbar[R_T] += (R)obja;
+            } else if (objective == AFVM_OBJ_VANE) {
+                int q = vane.cellPlane[c];
+                if (q >= 0) {
+                    double g5[5] = {0, 0, 0, 0, 0};
+                    double U[3] = {rc[0], rc[1], rc[2]};
+                    vane_cell_grad(P, vane, U, rec_T<R>(P, rc[R_T]), rec_p<R>(P, rc[R_P]), vane.planeArea[q], vane.sums[0],
+                                   vane.sums[1], obja, g5);
+                    for (int k = 0; k < 5; k++) pbar[k] += (R)g5[k];
+                }
+                if (vane.b != 0.0) {
+                    for (int s = 0; s < 6; s++) {
+                        int e = m.accf[s * n + c];
+                        if (e < m.nIF) continue;          // owner-side boundary faces only
+                        double k = vane.bHeatCoef[e - m.nIF];
+                        if (k != 0.0) pbar[R_T] += (R)(-obja * vane.b * vane.rw2 * k);
+                    }
+                }
+            } else if (objective == AFVM_OBJ_DRAG) {
                 for (int s = 0; s < 6; s++) {
                     int e = m.accf[s * n + c];
-                    if (e < m.nIF) continue;          // owner-side boundary faces only
-                    double k = vane.bHeatCoef[e - m.nIF];
-                    if (k != 0.0) pbar[R_T] += (R)(-obja * vane.b * vane.rw2 * k);
+                    if (e < objStart || e >= objStart + objN) continue;   // owner-side faces of the patch
+                    const R* rg = rec + (size_t)m.nbr[e] * REC;
+                    double T0 = rec_T<R>(P, rg[R_T]);
+                    double mu = viscosity<double>(P, T0);
+                    pbar[0] += (R)(obja * mu / (double)m.dlt[e] * (double)m.area[e]);
                 }
             }
-        } else if (objective == AFVM_OBJ_DRAG) {
-            for (int s = 0; s < 6; s++) {
-                int e = m.accf[s * n + c];
-                if (e < objStart || e >= objStart + objN) continue;   // owner-side faces of the patch
-                const R* rg = rec + (size_t)m.nbr[e] * REC;
-                double T0 = rec_T<R>(P, rg[R_T]);
-                double mu = viscosity<double>(P, T0);
-                pbar[0] += (R)(obja * mu / (double)m.dlt[e] * (double)m.area[e]);
-            }
         }
-    }
-    // primitive VJP (density.py:162-171)
-    S J[5];
-    if constexpr (sizeof(S) == 4) {
-        // float state: the density row without the low-Mach cancellation of the form below
-        // (rhob and eb E/rho both hold pbar_p (g-1) E): with q = |U|^2/2 and e = E - q,
-        //   J_rho = pbar_p (g-1) q - (pbar_U . U)/rho + (pbar_T/Cv) (q - e)/rho,
-        // which float evaluates to its own rounding, so the FP32 context needs no FP64 here
-        const PhysR<float>& Q = consts<float>(P);
-        float rho = ur[c], rr = rcp(rho);
-        float U[3] = {uu[3 * c] * rr, uu[3 * c + 1] * rr, uu[3 * c + 2] * rr};
-        float E = ue[c] * rr;
-        float q = 0.5f * (U[0] * U[0] + U[1] * U[1] + U[2] * U[2]);
-        float e = E - q;
-        float pT = pbar[R_T] * Q.rCv, pp = pbar[R_P] * Q.gm1;
-        float eb = pT + pp * rho;
-        for (int k = 0; k < 3; k++) J[1 + k] = (pbar[k] - eb * U[k]) * rr;
-        J[4] = eb * rr;
-        J[0] = pp * q - (pbar[0] * U[0] + pbar[1] * U[1] + pbar[2] * U[2]) * rr + pT * (q - e) * rr;
+        // primitive VJP (density.py:162-171)
+        if constexpr (sizeof(S) == 4) {
+            // float state: the density row without the low-Mach cancellation of the form below
+            // (rhob and eb E/rho both hold pbar_p (g-1) E): with q = |U|^2/2 and e = E - q,
+            //   J_rho = pbar_p (g-1) q - (pbar_U . U)/rho + (pbar_T/Cv) (q - e)/rho,
+            // which float evaluates to its own rounding, so the FP32 context needs no FP64 here
+            const PhysR<float>& Q = consts<float>(P);
+            float rho = ur[c], rr = rcp(rho);
+            float U[3] = {uu[3 * c] * rr, uu[3 * c + 1] * rr, uu[3 * c + 2] * rr};
+            float E = ue[c] * rr;
+            float q = 0.5f * (U[0] * U[0] + U[1] * U[1] + U[2] * U[2]);
+            float e = E - q;
+            float pT = pbar[R_T] * Q.rCv, pp = pbar[R_P] * Q.gm1;
+            float eb = pT + pp * rho;
+            for (int k = 0; k < 3; k++) J[1 + k] = (pbar[k] - eb * U[k]) * rr;
+            J[4] = eb * rr;
+            J[0] = pp * q - (pbar[0] * U[0] + pbar[1] * U[1] + pbar[2] * U[2]) * rr + pT * (q - e) * rr;
+        } else {
+            double rho = ur[c], rU[3] = {uu[3 * c], uu[3 * c + 1], uu[3 * c + 2]}, rE = ue[c];
+            double rr = rcp(rho);
+            double U[3] = {rU[0] * rr, rU[1] * rr, rU[2] * rr};
+            double E = rE * rr;
+            double e = E - 0.5 * (U[0] * U[0] + U[1] * U[1] + U[2] * U[2]);
+            double eb = (double)pbar[R_T] * P.rCv + (double)pbar[R_P] * P.gm1 * rho;
+            double rhob = (double)pbar[R_P] * P.gm1 * e;
+            double Ubt[3];
+            for (int k = 0; k < 3; k++) Ubt[k] = (double)pbar[k] - eb * U[k];
+            for (int k = 0; k < 3; k++) J[1 + k] = Ubt[k] * rr;
+            J[4] = eb * rr;
+            J[0] = rhob - (Ubt[0] * U[0] + Ubt[1] * U[1] + Ubt[2] * U[2]) * rr - eb * E * rr;
+        }
+    };
+    if constexpr (SPLIT) {
+        __shared__ S shJ[5 * 32];
+        const int lane = threadIdx.x & 31;
+        if (first && c < m.nIC) {
+            whole_cell();
+            for (int q = 0; q < 5; q++) shJ[q * 32 + lane] = J[q];
+        }
+        __syncthreads();
+        if (c >= m.nIC) return;
+        J[0] = shJ[at.q0 * 32 + lane];
     } else {
-        double rho = ur[c], rU[3] = {uu[3 * c], uu[3 * c + 1], uu[3 * c + 2]}, rE = ue[c];
-        double rr = rcp(rho);
-        double U[3] = {rU[0] * rr, rU[1] * rr, rU[2] * rr};
-        double E = rE * rr;
-        double e = E - 0.5 * (U[0] * U[0] + U[1] * U[1] + U[2] * U[2]);
-        double eb = (double)pbar[R_T] * P.rCv + (double)pbar[R_P] * P.gm1 * rho;
-        double rhob = (double)pbar[R_P] * P.gm1 * e;
-        double Ubt[3];
-        for (int k = 0; k < 3; k++) Ubt[k] = (double)pbar[k] - eb * U[k];
-        for (int k = 0; k < 3; k++) J[1 + k] = Ubt[k] * rr;
-        J[4] = eb * rr;
-        J[0] = rhob - (Ubt[0] * U[0] + Ubt[1] * U[1] + Ubt[2] * U[2]) * rr - eb * E * rr;
+        whole_cell();
     }
-    // SSP-RK reverse (timestep.py:35-45 transposed), in the state's type S
-    S ain[5] = {ainr[c], ainu[3 * c], ainu[3 * c + 1], ainu[3 * c + 2], aine[c]};
-    S out[5];
-    if (STAGE == 2) {
-        for (int k = 0; k < 5; k++) out[k] = S(2. / 3) * ain[k] + (S)J[k];
-        S z[5];
-        for (int k = 0; k < 5; k++) { z[k] = S(1. / 3) * ain[k]; sb[k * n + c] = S(2. / 3) * S(dt) * ain[k]; }
-        a0r[c] = z[0]; a0u[3 * c] = z[1]; a0u[3 * c + 1] = z[2]; a0u[3 * c + 2] = z[3]; a0e[c] = z[4];
-        a1r[c] = out[0]; a1u[3 * c] = out[1]; a1u[3 * c + 1] = out[2]; a1u[3 * c + 2] = out[3]; a1e[c] = out[4];
-    } else if (STAGE == 1) {
-        for (int k = 0; k < 5; k++) out[k] = S(1. / 4) * ain[k] + (S)J[k];
-        S z[5] = {a0r[c], a0u[3 * c], a0u[3 * c + 1], a0u[3 * c + 2], a0e[c]};
-        for (int k = 0; k < 5; k++) { z[k] += S(3. / 4) * ain[k]; sb[k * n + c] += S(1. / 4) * S(dt) * ain[k]; }
-        a0r[c] = z[0]; a0u[3 * c] = z[1]; a0u[3 * c + 1] = z[2]; a0u[3 * c + 2] = z[3]; a0e[c] = z[4];
-        a1r[c] = out[0]; a1u[3 * c] = out[1]; a1u[3 * c + 1] = out[2]; a1u[3 * c + 2] = out[3]; a1e[c] = out[4];
-    } else {
-        S z[5] = {a0r[c], a0u[3 * c], a0u[3 * c + 1], a0u[3 * c + 2], a0e[c]};
-        for (int k = 0; k < 5; k++) z[k] += ain[k] + (S)J[k];
-        // the source adjoint, complete with this stage, in the reference's layout (any part may be
-        // absent; the stages before keep it in rows by component, as the outputs may alias inputs)
-        if (sr) sr[c] = sb[c] + S(dt) * ain[0];
-        if (su)
-            for (int k = 1; k < 4; k++) su[3 * c + k - 1] = sb[k * n + c] + S(dt) * ain[k];
-        if (se) se[c] = sb[4 * n + c] + S(dt) * ain[4];
-        a0r[c] = z[0]; a0u[3 * c] = z[1]; a0u[3 * c + 1] = z[2]; a0u[3 * c + 2] = z[3]; a0e[c] = z[4];
+    // SSP-RK reverse (timestep.py:35-45 transposed), in the state's type S. The source adjoint is
+    // complete with stage 0, which writes it in the reference's layout (any part may be absent); the
+    // stages before keep it in rows by component, as the outputs may alias inputs
+#pragma unroll
+    for (int i = 0; i < (SPLIT ? 1 : 5); i++) {
+        const int q = SPLIT ? at.q0 : i;
+        const S ain = state_at(ainr, ainu, aine, c, q);
+        S& a0 = state_at(a0r, a0u, a0e, c, q);
+        if (STAGE == 2) {
+            sb[q * n + c] = S(2. / 3) * S(dt) * ain;
+            a0 = S(1. / 3) * ain;
+            state_at(a1r, a1u, a1e, c, q) = S(2. / 3) * ain + (S)J[i];
+        } else if (STAGE == 1) {
+            sb[q * n + c] += S(1. / 4) * S(dt) * ain;
+            a0 += S(3. / 4) * ain;
+            state_at(a1r, a1u, a1e, c, q) = S(1. / 4) * ain + (S)J[i];
+        } else {
+            const S src = sb[q * n + c] + S(dt) * ain;
+            a0 += ain + (S)J[i];
+            if (q == 0 ? sr != nullptr : (q == 4 ? se != nullptr : su != nullptr)) state_at(sr, su, se, c, q) = src;
+        }
     }
 }
 
@@ -521,6 +589,7 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
     R* cbar = (R*)c->cbar;
     S* sb = (S*)c->sbar;
     const Shape gF = shape_for(m.nF, FLUX_BLOCK), gC = shape_for(m.nIC, BLOCK);
+    const bool split = split_cells(m.nIC);
     const double beta[3] = {1.0, 1. / 4, 2. / 3};
     // a tape holds the stage's cell records the primal step built (no primitive or gradient
     // launches here) and, in FP64, its face tape
@@ -569,8 +638,11 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
         }
         {
             ProfScope ps(c, KID_ADJ_GATHER, s);
-            launch_after(gC.threads == 32 ? k_adj_cell1<R, 32> : k_adj_cell1<R, BLOCK>, gC.blocks, gC.threads, 0, s, m,
-                         (const R*)fadj, cbar);
+            if (split)
+                launch_after(k_adj_cell1_split<R>, (m.nIC + 31) / 32, 160, 0, s, m, (const R*)fadj, cbar);
+            else
+                launch_after(gC.threads == 32 ? k_adj_cell1<R, 32> : k_adj_cell1<R, BLOCK>, gC.blocks, gC.threads, 0, s,
+                             m, (const R*)fadj, cbar);
         }
         // the stage's share of the mesh / boundary-input gradients (before the cell kernel: the
         // adjoint outputs it writes may alias this stage's input adjoints)
@@ -578,10 +650,17 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
             if (params) launch_param_grads<R, S>(c, *params, rec, coef, ain[0], ain[1], ain[2], st == 1, obja, s);
         ProfScope ps(c, KID_ADJ_GRAD, s);
         S* const* a1 = st == 2 ? A2 : A1;      // (not written by the last stage)
-        launch_after(st == 2 ? k_adj_cell2<R, S, 2> : (st == 1 ? k_adj_cell2<R, S, 1> : k_adj_cell2<R, S, 0>), gC.blocks,
-                     gC.threads, 0, s, m, P, rec, (const R*)fadj, (const R*)cbar, u[0], u[1], u[2], ain[0], ain[1],
-                     ain[2], a1[0], a1[1], a1[2], rhoa, rhoUa, rhoEa, sb, Srhoa, SrhoUa, SrhoEa, dt, c->objective,
-                     c->objStart, c->objN, obja, c->vane, c->objSeed);
+        auto cells = [&](auto stage) {
+            constexpr int ST = decltype(stage)::value;
+            launch_after(split ? k_adj_cell2<R, S, ST, true> : k_adj_cell2<R, S, ST, false>,
+                         split ? (m.nIC + 31) / 32 : gC.blocks, split ? 160 : gC.threads, 0, s, m, P, rec,
+                         (const R*)fadj, (const R*)cbar, u[0], u[1], u[2], ain[0], ain[1], ain[2], a1[0], a1[1], a1[2],
+                         rhoa, rhoUa, rhoEa, sb, Srhoa, SrhoUa, SrhoEa, dt, c->objective, c->objStart, c->objN, obja,
+                         c->vane, c->objSeed);
+        };
+        if (st == 2) cells(std::integral_constant<int, 2>{});
+        else if (st == 1) cells(std::integral_constant<int, 1>{});
+        else cells(std::integral_constant<int, 0>{});
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "adjoint step launch");

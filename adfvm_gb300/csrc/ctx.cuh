@@ -30,6 +30,11 @@ constexpr int FLUX_BLOCK = 128;
 // the limit nothing changes.
 constexpr int SMALL_WARPS = 8 * 4 * 152;
 static inline bool small_grid(long long n) { return n <= 32LL * SMALL_WARPS; }
+// The cell kernels' split form (CellAt, below) up to one warp a sub-partition, where the chain of a
+// cell's instructions is the time: a step and its adjoint (one graph) of box 16^3 195 -> 148 us in
+// FP64, 74 -> 66 in FP32, of box 24^3 318 -> 291 and 84 -> 77; 28^3 (past the line) 445 and 450, 96
+// and 90, 32^3 609 -> 634, 115 -> 118 (the components' repeated table reads).
+static inline bool split_cells(long long n) { return n <= 32LL * 4 * 152; }
 
 // Programmatic dependent launches. The step's kernels follow one another in a stream, each on the
 // results of the one before. Launched this way a kernel's blocks become resident as soon as the
@@ -62,6 +67,32 @@ inline void launch_after(void (*kernel)(P...), int blocks, int threads, size_t s
     cfg.attrs = at;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// Split cell kernels. On a small mesh most SM sub-partitions hold one warp or none and an FP64
+// instruction takes 64 cycles of it, so the chain of one cell's instructions is the kernel's time.
+// With SPLIT the five components of 32 cells are five warps of a block (component q, cell c);
+// where the components meet (primitives, boundary conditions, the primitives' VJP) the first warp
+// goes on alone.
+template <bool SPLIT>
+struct CellAt {
+    int c, q0, q1;     // the cell, and the components this thread works on
+    __device__ __forceinline__ CellAt() {
+        if constexpr (SPLIT) {
+            c = blockIdx.x * 32 + (threadIdx.x & 31);
+            q0 = threadIdx.x >> 5;
+            q1 = q0 + 1;
+        } else {
+            c = blockIdx.x * blockDim.x + threadIdx.x;
+            q0 = 0;
+            q1 = 5;
+        }
+    }
+};
+// component q of cell c of a state (rho (n), rhoU (n x 3), rhoE (n))
+template <typename S>
+__device__ __forceinline__ S& state_at(S* r, S* u, S* e, int c, int q) {
+    return q == 0 ? r[c] : (q == 4 ? e[c] : u[3 * (size_t)c + q - 1]);
 }
 
 // Block-staged record stores. A thread that stores its own W-value record at a W-value stride

@@ -18,9 +18,6 @@
 
 namespace afvm {
 
-// max(a, b) that keeps a NaN operand (fmax drops it)
-__device__ __forceinline__ double nan_max(double a, double b) { return (b > a || b != b) ? b : a; }
-
 // RCF.primitive (adFVM/density.py:162-171) in double. One out-of-line body, so that a ghost
 // cell and its source cell get bit-identical values.
 __device__ __noinline__ void primitive_d(const Phys& P, double rho, double r0, double r1, double r2, double rhoE,
@@ -244,12 +241,46 @@ __global__ void __launch_bounds__(NT) k_grad(MeshDev<R> m, Phys P, R* __restrict
     if (c0 < m.nIC) store_staged<R, REC, NT>(rec, c0, min(NT, m.nIC - c0), stage);
 }
 
+// the split form (CellAt): warp q of a block does component q of 32 cells
+template <typename R>
+__global__ void __launch_bounds__(160) k_grad_split(MeshDev<R> m, Phys P, R* __restrict__ rec) {
+    __shared__ __align__(16) R stage[32 * REC];
+    const CellAt<true> at;
+    const int c = at.c, q = at.q0, c0 = blockIdx.x * 32;
+    GradSlots<R> t;
+    if (c < m.nIC) load_slots<R>(m, c, t);
+    dep_wait(rec);
+    if (c < m.nIC) {
+        const R phi = rec[(size_t)c * REC + q];
+        R g[3], nb[6];
+#pragma unroll
+        for (int s = 0; s < 6; s++) nb[s] = rec[(size_t)t.nb[s] * REC + q];
+        for (int j = 0; j < 3; j++) g[j] = phi * t.a[j];
+#pragma unroll
+        for (int s = 0; s < 6; s++)
+            for (int j = 0; j < 3; j++) g[j] = g[j] + nb[s] * t.ws[3 * s + j];
+        if constexpr (kGauge<R>) {
+            const R offset = q == R_T ? consts<R>(P).gT : consts<R>(P).gP;
+            if (q >= R_T)
+                for (int j = 0; j < 3; j++) g[j] = g[j] + offset * t.cl[j];
+        }
+        R* row = stage + (threadIdx.x & 31) * REC;
+        row[q] = phi;
+        for (int j = 0; j < 3; j++) row[R_GU + 3 * q + j] = g[j];
+    }
+    __syncthreads();
+    if (c0 < m.nIC) store_staged<R, REC, 160>(rec, c0, min(32, m.nIC - c0), stage);
+}
+
 template <typename R>
 static void launch_grad(Ctx* c, R* rec, cudaStream_t s) {
     const MeshDev<R>& m = meshOf<R>(c);
     ProfScope ps(c, KID_GRAD, s);
     const Shape g = shape_for(m.nIC, BLOCK);
-    launch_after(g.threads == 32 ? k_grad<R, 32> : k_grad<R, BLOCK>, g.blocks, g.threads, 0, s, m, c->phys, rec);
+    if (split_cells(m.nIC))
+        launch_after(k_grad_split<R>, (m.nIC + 31) / 32, 160, 0, s, m, c->phys, rec);
+    else
+        launch_after(g.threads == 32 ? k_grad<R, 32> : k_grad<R, BLOCK>, g.blocks, g.threads, 0, s, m, c->phys, rec);
 }
 
 
@@ -332,6 +363,17 @@ __device__ __forceinline__ void load_flux_record(const double* __restrict__ p, d
     }
 }
 
+// reduce_max of the CFL sums (density.py:405-410): a warp's maximum, then an atomic one. Sums of
+// magnitudes order like their bits, compared as integers (an FP64 comparison takes the FP64 pipe). A
+// NaN wins every comparison, as in the reference's max (a NaN's bits are above every finite
+// double's), so a state gone non-finite gives a non-finite CFL sum and the step reports it.
+__device__ __forceinline__ void cfl_max(double d, unsigned long long* dtcBits) {
+    unsigned long long b = (unsigned long long)__double_as_longlong(d);
+    const unsigned hi = (unsigned)(b >> 32), top = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned lo = __reduce_max_sync(0xffffffffu, hi == top ? (unsigned)b : 0u);
+    if ((threadIdx.x & 31) == 0) atomicMax(dtcBits, ((unsigned long long)top << 32) | lo);
+}
+
 // StepEnd's work, by one block
 __device__ __forceinline__ void step_end(const StepEnd& e) {
     __shared__ double sh[BLOCK / 32];
@@ -352,24 +394,23 @@ __device__ __forceinline__ void step_end(const StepEnd& e) {
 }
 
 // Gather of the face fluxes (op.div / op.absDiv, op.py:12-29, collated in the order of
-// density.py:390-402) and the SSP-RK3 stage update (timestep.py:35-45).
-template <typename R, typename S, int STAGE>
-__global__ void __launch_bounds__(BLOCK) k_update(MeshDev<R> m, const R* __restrict__ fflux, double dtv,
-                                                  const double* dtp,
-                                                  const S* u0r, const S* u0u, const S* u0e,
-                                                  const S* u1r, const S* u1u, const S* u1e,
-                                                  const S* u2r, const S* u2u, const S* u2e,
-                                                  const S* __restrict__ Sr, const S* __restrict__ Su,
-                                                  const S* __restrict__ Se,
-                                                  S* outr, S* outu, S* oute,
-                                                  unsigned long long* dtcBits, Phys P, R* __restrict__ recNext,
-                                                  int objKind, double* __restrict__ objPartials, StepEnd end) {
+// density.py:390-402) and the SSP-RK3 stage update (timestep.py:35-45). SPLIT: the form of CellAt
+// with a sixth warp for the CFL sum.
+template <typename R, typename S, int STAGE, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 192 : BLOCK)
+    k_update(MeshDev<R> m, const R* __restrict__ fflux, double dtv, const double* dtp, const S* u0r, const S* u0u,
+             const S* u0e, const S* u1r, const S* u1u, const S* u1e, const S* u2r, const S* u2u, const S* u2e,
+             const S* __restrict__ Sr, const S* __restrict__ Su, const S* __restrict__ Se, S* outr, S* outu, S* oute,
+             unsigned long long* dtcBits, Phys P, R* __restrict__ recNext, int objKind,
+             double* __restrict__ objPartials, StepEnd end) {
     // the gather (and the CFL sum) in the flux type R, the stage update in the state's type S:
     // under FP32 fluxes with an FP64 state the six fluxes are summed in FP32 (each carries FP32
     // rounding already; summing them in FP64 cost six FP64 conversions, products and sums a
     // cell and component) and the state is updated in FP64
     const size_t n = m.nIC;
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const CellAt<SPLIT> at;
+    const int c = at.c;
+    const bool first = !SPLIT || at.q0 == 0;        // the thread that goes on with the whole cell
     int e[6], gs0 = 0, gs1 = 0;
     R w[6];
     if (c < m.nIC) {
@@ -378,8 +419,10 @@ __global__ void __launch_bounds__(BLOCK) k_update(MeshDev<R> m, const R* __restr
             e[k] = m.accf[k * n + c];
             w[k] = m.accw[k * n + c];
         }
-        gs0 = m.gsStart[c];
-        gs1 = m.gsStart[c + 1];
+        if (first) {
+            gs0 = m.gsStart[c];
+            gs1 = m.gsStart[c + 1];
+        }
     }
     dep_wait(fflux, dtp, u0r, u0u, u0e, u1r, u1u, u1e, u2r, u2u, u2e, Sr, Su, Se, recNext);
     if (STAGE == 2 && end.dtcBits && blockIdx.x == gridDim.x - 1) {
@@ -387,7 +430,7 @@ __global__ void __launch_bounds__(BLOCK) k_update(MeshDev<R> m, const R* __restr
         return;
     }
     R dtc = R(0);
-    double objv = 0.0;     // this cell's term of a cell-sum objective (stage 0, objPartials)
+    S o[5];
     if (c < m.nIC) {
         // the sums start at -0, which the compiler drops from the first term's add (-0 + x is x,
         // while +0 + x is one more add; the values differ at most in the sign of a zero)
@@ -396,86 +439,99 @@ __global__ void __launch_bounds__(BLOCK) k_update(MeshDev<R> m, const R* __restr
         for (int k = 0; k < 6; k++) {
             bool ownerSide = e[k] >= 0;
             int f = ownerSide ? e[k] : ~e[k];
-            R F[FREC];
-            load_flux_record(fflux + (size_t)f * FREC, F);
             // the side's sign on the weight (one select a face, not one a term); each product
             // rounded before it is added, as the reference's collate sum does, so that equal
             // and opposite terms cancel exactly
             R ws = ownerSide ? w[k] : -w[k];
-            for (int q = 0; q < 5; q++) res[q] = res[q] + mul_rn(F[q], ws);
-            dtc = dtc + F[5] * w[k];
-        }
-        S rs[5];
-        for (int q = 0; q < 5; q++) rs[q] = S(res[q]);
-        // gauge-form fluxes (FP32): the energy residual is the gathered one plus gaugeH times
-        // the mass residual, the momentum residual the gathered one plus gaugeP times the
-        // cell's sum of A/V N (the gaugeP N the face fluxes leave out; zero when the cell's
-        // face area vectors close), both added in the state's type
-        if constexpr (kGauge<R>) {
-            rs[4] = rs[4] + S(P.gaugeH) * rs[0];
-            // (a float state reads the float copy of the closure sums: half the bytes)
-            for (int k = 0; k < 3; k++)
-                rs[1 + k] = rs[1 + k] + S(P.gaugeP) * (sizeof(S) == 4 ? S(m.gcl[k * n + c]) : S(m.gclD[k * n + c]));
-        }
-        S Sv[5] = {Sr[c], Su[3 * c], Su[3 * c + 1], Su[3 * c + 2], Se[c]};
-        S a[5] = {u0r[c], u0u[3 * c], u0u[3 * c + 1], u0u[3 * c + 2], u0e[c]};
-        S o[5];
-        const S rdt = S(dtp ? *dtp : dtv);
-        // u = sum_j alpha_j u_j - beta dt (R - S) with -beta dt formed once a cell
-        if (STAGE == 0) {
-            const S k = -rdt;
-            for (int q = 0; q < 5; q++) o[q] = a[q] + k * (rs[q] - Sv[q]);
-        } else if (STAGE == 1) {
-            S b[5] = {u1r[c], u1u[3 * c], u1u[3 * c + 1], u1u[3 * c + 2], u1e[c]};
-            const S k = S(-(1. / 4)) * rdt;
-            for (int q = 0; q < 5; q++) o[q] = (S(3. / 4) * a[q] + S(1. / 4) * b[q]) + k * (rs[q] - Sv[q]);
-        } else {
-            S b[5] = {u2r[c], u2u[3 * c], u2u[3 * c + 1], u2u[3 * c + 2], u2e[c]};
-            const S k = S(-(2. / 3)) * rdt;
-            for (int q = 0; q < 5; q++) o[q] = (S(1. / 3) * a[q] + S(2. / 3) * b[q]) + k * (rs[q] - Sv[q]);
-        }
-        outr[c] = o[0];
-        outu[3 * c] = o[1]; outu[3 * c + 1] = o[2]; outu[3 * c + 2] = o[3];
-        oute[c] = o[4];
-        if (recNext) {
-            // the next stage's k_prim, fused: this cell's primitives and those of the ghost
-            // cells whose source it is, from the values just stored (the same bits k_prim
-            // would read back)
-            R v[5];
-            prim_values(P, o[0], o[1], o[2], o[3], o[4], v);
-            store_prims(recNext + (size_t)c * REC, v);
-            if (STAGE == 0 && objPartials) objv = cell_objective<R>(P, objKind, v, m.vol[c]);
-            for (int q = gs0; q < gs1; q++) {
-                int g = m.gsList[q];
-                R gv[5] = {v[0], v[1], v[2], v[3], v[4]};
-                ghost_prims<R>(m, P, g, gv);
-                store_prims(recNext + (size_t)(m.nIC + g) * REC, gv);
+            if constexpr (SPLIT) {
+                const R F = fflux[(size_t)f * FREC + at.q0];
+                if (at.q0 == 5) dtc = dtc + F * w[k];
+                else res[1] = res[1] + mul_rn(F, ws);
+                // (the energy residual's gauge term takes the mass residual)
+                if (kGauge<R> && at.q0 == 4) res[0] = res[0] + mul_rn(fflux[(size_t)f * FREC], ws);
+            } else {
+                R F[FREC];
+                load_flux_record(fflux + (size_t)f * FREC, F);
+                for (int q = 0; q < 5; q++) res[q] = res[q] + mul_rn(F[q], ws);
+                dtc = dtc + F[5] * w[k];
             }
+        }
+        const S rdt = S(dtp ? *dtp : dtv);
+#pragma unroll
+        for (int i = 0; i < (SPLIT ? 1 : 5); i++) {
+            const int q = SPLIT ? at.q0 : i;
+            if (SPLIT && q == 5) break;
+            S rs = S(res[SPLIT ? 1 : i]);
+            // gauge-form fluxes (FP32): the energy residual is the gathered one plus gaugeH times
+            // the mass residual, the momentum residual the gathered one plus gaugeP times the
+            // cell's sum of A/V N (the gaugeP N the face fluxes leave out; zero when the cell's
+            // face area vectors close), both added in the state's type
+            if constexpr (kGauge<R>) {
+                if (q == 4) rs = rs + S(P.gaugeH) * S(res[0]);
+                // (a float state reads the float copy of the closure sums: half the bytes)
+                if (q >= 1 && q <= 3)
+                    rs = rs + S(P.gaugeP) * (sizeof(S) == 4 ? S(m.gcl[(q - 1) * n + c]) : S(m.gclD[(q - 1) * n + c]));
+            }
+            const S Sv = state_at(Sr, Su, Se, c, q), a = state_at(u0r, u0u, u0e, c, q);
+            // u = sum_j alpha_j u_j - beta dt (R - S) with -beta dt formed once a cell
+            S v;
+            if (STAGE == 0) {
+                const S k = -rdt;
+                v = a + k * (rs - Sv);
+            } else if (STAGE == 1) {
+                const S b = state_at(u1r, u1u, u1e, c, q);
+                const S k = S(-(1. / 4)) * rdt;
+                v = (S(3. / 4) * a + S(1. / 4) * b) + k * (rs - Sv);
+            } else {
+                const S b = state_at(u2r, u2u, u2e, c, q);
+                const S k = S(-(2. / 3)) * rdt;
+                v = (S(1. / 3) * a + S(2. / 3) * b) + k * (rs - Sv);
+            }
+            o[i] = v;
+            state_at(outr, outu, oute, c, q) = v;
+        }
+    }
+    if constexpr (SPLIT) {
+        __shared__ S sh[5 * 32];
+        const int lane = threadIdx.x & 31;
+        if (at.q0 < 5) sh[at.q0 * 32 + lane] = o[0];
+        __syncthreads();
+        if (STAGE == 1 && at.q0 == 5) {
+            cfl_max(c < m.nIC ? (double)dtc : 0.0, dtcBits);
+            return;
+        }
+        if (!first || !recNext) return;
+        for (int q = 0; q < 5; q++) o[q] = sh[q * 32 + lane];
+    }
+    double objv = 0.0;     // this cell's term of a cell-sum objective (stage 0, objPartials)
+    if (c < m.nIC && recNext) {
+        // the next stage's k_prim, fused: this cell's primitives and those of the ghost
+        // cells whose source it is, from the values just stored (the same bits k_prim
+        // would read back)
+        R v[5];
+        prim_values(P, o[0], o[1], o[2], o[3], o[4], v);
+        store_prims(recNext + (size_t)c * REC, v);
+        if (STAGE == 0 && objPartials) objv = cell_objective<R>(P, objKind, v, m.vol[c]);
+        for (int q = gs0; q < gs1; q++) {
+            int g = m.gsList[q];
+            R gv[5] = {v[0], v[1], v[2], v[3], v[4]};
+            ghost_prims<R>(m, P, g, gv);
+            store_prims(recNext + (size_t)(m.nIC + g) * REC, gv);
         }
     }
     if (STAGE == 0 && objPartials) {
         // the objective stage's primitives are the ones this stage-0 update writes: the
         // objective's block partial sums (the same terms and order as k_objective)
-        __shared__ double osh[BLOCK / 32];
-        double sum = block_sum(objv, osh);
-        if (threadIdx.x == 0) objPartials[blockIdx.x] = sum;
-    }
-    if (STAGE == 1) {
-        // reduce_max of the CFL sums (density.py:405-410): warp shuffle, block, then an atomic
-        // max on the bit pattern (non-negative doubles order like their bits). A NaN wins every
-        // comparison, as in the reference's max (a NaN's bits are above every finite double's),
-        // so a state gone non-finite gives a non-finite CFL sum and the step reports it
-        double d = (double)dtc;
-        for (int off = 16; off > 0; off >>= 1) d = nan_max(d, __shfl_down_sync(0xffffffffu, d, off));
-        __shared__ double wmax[BLOCK / 32];
-        if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = d;
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            d = (threadIdx.x < blockDim.x / 32) ? wmax[threadIdx.x] : 0.0;
-            for (int off = 16; off > 0; off >>= 1) d = nan_max(d, __shfl_down_sync(0xffffffffu, d, off));
-            if (threadIdx.x == 0) atomicMax(dtcBits, (unsigned long long)__double_as_longlong(d));
+        if constexpr (SPLIT) {
+            for (int off = 16; off > 0; off >>= 1) objv += __shfl_down_sync(0xffffffffu, objv, off);
+            if (threadIdx.x == 0) objPartials[blockIdx.x] = objv;
+        } else {
+            __shared__ double osh[BLOCK / 32];
+            double sum = block_sum(objv, osh);
+            if (threadIdx.x == 0) objPartials[blockIdx.x] = sum;
         }
     }
+    if (!SPLIT && STAGE == 1) cfl_max((double)dtc, dtcBits);
 }
 
 // rows of U (3), T, p with absolute T and p from records of stride `stride` (FP32 records hold
@@ -636,19 +692,18 @@ void launch_flux_update(Ctx* c, int st, double dt, const double* dtDev, const S*
     R* recNext = nextPrims ? (recOut ? recOut : rec) : nullptr;
     ProfScope ps(c, KID_UPDATE, s);
     const S* none = nullptr;
-    const StepEnd noEnd = {};
-    if (st == 0)
-        launch_after(k_update<R, S, 0>, g.blocks, g.threads, 0, s, m, ff, dt, dtDev, u0[0], u0[1], u0[2], none, none,
-                     none, none, none, none, Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P, recNext, c->objective,
-                     recNext ? objPartials : nullptr, noEnd);
-    else if (st == 1)
-        launch_after(k_update<R, S, 1>, g.blocks, g.threads, 0, s, m, ff, dt, dtDev, u0[0], u0[1], u0[2], u1[0], u1[1],
-                     u1[2], none, none, none, Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P, recNext, c->objective,
-                     (double*)nullptr, noEnd);
-    else
-        launch_after(k_update<R, S, 2>, g.blocks + (end ? 1 : 0), g.threads, 0, s, m, ff, dt, dtDev, u0[0], u0[1], u0[2],
-                     none, none, none, u2[0], u2[1], u2[2], Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P, recNext,
-                     c->objective, (double*)nullptr, end ? *end : noEnd);
+    const bool split = split_cells(m.nIC);
+    const S *const *b = st == 1 ? u1 : u2, *b0 = st ? b[0] : none, *b1 = st ? b[1] : none, *b2 = st ? b[2] : none;
+    auto update = [&](auto stage) {
+        constexpr int ST = decltype(stage)::value;
+        launch_after(split ? k_update<R, S, ST, true> : k_update<R, S, ST, false>, (split ? (m.nIC + 31) / 32 : g.blocks) +
+                     (ST == 2 && end ? 1 : 0), split ? 192 : g.threads, 0, s, m, ff, dt, dtDev, u0[0], u0[1], u0[2], b0,
+                     b1, b2, b0, b1, b2, Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P, recNext, c->objective,
+                     ST == 0 && recNext ? objPartials : nullptr, ST == 2 && end ? *end : StepEnd{});
+    };
+    if (st == 0) update(std::integral_constant<int, 0>{});
+    else if (st == 1) update(std::integral_constant<int, 1>{});
+    else update(std::integral_constant<int, 2>{});
 }
 
 template <typename S>
@@ -705,7 +760,7 @@ int primal_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double d
             int start = 0, n = m.nIC;
             if (c->objective == AFVM_OBJ_DRAG) { start = c->objStart; n = c->objN; }
             const Shape g = shape_for(n, BLOCK);
-            nObjBlocks = g.blocks;
+            nObjBlocks = cell_sum_objective(c->objective) && split_cells(n) ? (n + 31) / 32 : g.blocks;
             if (nObjBlocks > c->nPartials) return fail(c, AFVM_ERR_BAD_ARG, "objective partials overflow");
             // a cell-sum objective's partials were written by the stage-0 update
             if (n > 0 && !cell_sum_objective(c->objective)) {

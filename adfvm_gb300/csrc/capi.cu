@@ -440,6 +440,15 @@ int alloc_work(Ctx* c) {
     if ((st = dalloc(c, (void**)&c->scal, sizeof(double) * 8))) return st;
     cudaMemset(c->scal, 0, sizeof(double) * 8);
     if ((st = dalloc(c, (void**)&c->dtcBits, sizeof(unsigned long long)))) return st;
+    void* host = nullptr;
+    if (cudaHostAlloc(&host, 4 * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(c, AFVM_ERR_OOM, "host memory of the step's results");
+    }
+    c->hostOut = (volatile double*)host;
+    for (int k = 0; k < 4; k++) c->hostOut[k] = 0.0;
+    cudaError_t e = cudaHostGetDevicePointer((void**)&c->hostOutDev, host, 0);
+    if (e != cudaSuccess) return cuda_fail(c, e, "host memory of the step's results");
     return AFVM_OK;
 }
 
@@ -475,6 +484,8 @@ void release(Ctx* c) {
     c->allocs.clear();
     if (c->sensScratch) cudaFree(c->sensScratch);
     c->sensScratch = nullptr;
+    if (c->hostOut) cudaFreeHost((void*)c->hostOut);
+    c->hostOut = nullptr;
     if (prev >= 0) cudaSetDevice(prev);
 }
 
@@ -505,10 +516,10 @@ inline size_t record_size(const Ctx* c) { return c->precision == AFVM_FP64 ? siz
 
 int get_results(Ctx* c, double* dtc_out, double* obj_out, cudaStream_t s) {
     if (!dtc_out && !obj_out) return AFVM_OK;
-    double tmp[2];
-    cudaError_t e = cudaMemcpyAsync(tmp, c->scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    // the step's last kernel left both in mapped host memory
+    cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(c, e, "step results");
+    const double tmp[2] = {c->hostOut[0], c->hostOut[1]};
     if (dtc_out) *dtc_out = tmp[0];
     if (obj_out) *obj_out = tmp[1];
     if (!std::isfinite(tmp[0]) || !std::isfinite(tmp[1]))

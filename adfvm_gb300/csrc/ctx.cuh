@@ -234,8 +234,12 @@ struct Ctx {
     void* zeroS = nullptr;    // nIC x 5 zeros (absent sources)
     double* partials = nullptr;   // reduction scratch (block partial sums)
     int nPartials = 0;
-    double* scal = nullptr;   // device scalars: [0] dtc (stage 1 max), [1] obj, [2] dt, [3] sensitivity
+    double* scal = nullptr;   // device scalars: [0] dtc (stage 1 max), [1] obj, [2] dt, [3] the next step's dt
     unsigned long long* dtcBits = nullptr;
+    // mapped host memory the kernels leave results in: [0] dtc, [1] obj of a step, [2] sensitivity,
+    // [3] energy; read after the stream has been waited for (a copy back took 6 us more a step)
+    volatile double* hostOut = nullptr;
+    double* hostOutDev = nullptr;
     // ghost BC values on the host for updates
     std::vector<int> ghostPatchOffset;   // first ghost index of each patch (sorted order)
     std::vector<int> bcKinds;            // per patch: U,T,p kinds
@@ -300,6 +304,7 @@ struct StepEnd {
     int nPartials;               // 0: no objective
     unsigned long long* dtcBits; // read and cleared for the next step
     double *dtcOut, *objOut;
+    double* host;                // also [0] dtc and [1] obj (NULL: not)
     const double* dt;
     double *dtNext, *dtHist;
     double CFL, stepFactor;
@@ -370,7 +375,7 @@ inline void stage_views(P* stages, int n, P** u1, P** u2) {
 // turbine-vane objective partial sums of the stage-1 record now in c->rec into c->vaneSums
 // rec: the cell records to read/write (NULL: the context's)
 template <typename R>
-void launch_vane_sums(Ctx* c, cudaStream_t s, double* objOut, const R* rec = nullptr);
+void launch_vane_sums(Ctx* c, cudaStream_t s, double* objOut, const R* rec = nullptr, double* objHost = nullptr);
 template <typename R, typename S = R>
 void launch_prim(Ctx* c, const S* r, const S* ru, const S* re, cudaStream_t s, R* rec = nullptr);
 template <typename R, typename S = R>

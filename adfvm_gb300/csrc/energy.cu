@@ -66,11 +66,12 @@ int energy_dev(Ctx* c, const void* ra, const void* rua, const void* rea, const v
         ProfScope ps(c, KID_ADJ_MISC, s);
         k_energy<R, S><<<nb, BLOCK, 0, s>>>(m, c->phys.gamma, (const S*)ra, (const S*)rua, (const S*)rea,
                                             (const S*)r, (const S*)ru, (const S*)re, c->partials);
-        k_energy_finish<<<1, BLOCK, 0, s>>>(c->partials, nb, c->scal + 4);
+        k_energy_finish<<<1, BLOCK, 0, s>>>(c->partials, nb, c->hostOutDev + 3);
     }
-    cudaError_t e = cudaMemcpyAsync(out, c->scal + 4, sizeof(double), cudaMemcpyDeviceToHost, s);
+    cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(c, e, "afvm_adjoint_energy");
+    *out = c->hostOut[3];
     return AFVM_OK;
 }
 

@@ -386,6 +386,10 @@ __device__ __forceinline__ void step_end(const StepEnd& e) {
     *e.dtcBits = 0;
     if (e.objOut) *e.objOut = s;
     if (e.dtcOut) *e.dtcOut = dtc;
+    if (e.host) {
+        e.host[0] = dtc;
+        if (e.objOut) e.host[1] = s;
+    }
     if (e.dtNext) {
         const double d = *e.dt;
         if (e.dtHist) *e.dtHist = d;
@@ -611,7 +615,7 @@ __global__ void __launch_bounds__(BLOCK) k_obj_vane(MeshDev<R> m, Phys P, const 
 // fixed-order sums of the vane partials into sums[0..2]; with objOut, also the objective
 // a L/W + b H/sum(A w)
 __global__ void __launch_bounds__(BLOCK) k_vane_finish(const double* partials, int nBlocks, VaneDev v, double* sums,
-                                                       double* objOut) {
+                                                       double* objOut, double* objHost) {
     __shared__ double sh0[BLOCK / 32], sh1[BLOCK / 32], sh2[BLOCK / 32];
     dep_wait(partials);
     double a = 0.0, b = 0.0, c = 0.0;
@@ -625,12 +629,14 @@ __global__ void __launch_bounds__(BLOCK) k_vane_finish(const double* partials, i
         sums[0] = L;
         sums[1] = W;
         sums[2] = H;
-        if (objOut) *objOut = v.a * (L / W) + v.b * (H * v.rw2);
+        const double J = v.a * (L / W) + v.b * (H * v.rw2);
+        if (objOut) *objOut = J;
+        if (objHost) *objHost = J;
     }
 }
 
 template <typename R>
-void launch_vane_sums(Ctx* c, cudaStream_t s, double* objOut, const R* rec) {
+void launch_vane_sums(Ctx* c, cudaStream_t s, double* objOut, const R* rec, double* objHost) {
     const MeshDev<R>& m = meshOf<R>(c);
     {
         ProfScope ps(c, KID_OBJECTIVE, s);
@@ -638,7 +644,8 @@ void launch_vane_sums(Ctx* c, cudaStream_t s, double* objOut, const R* rec) {
                      c->nVaneBlocks, c->vanePartials);
     }
     ProfScope ps(c, KID_FINISH, s);
-    launch_after(k_vane_finish, 1, BLOCK, 0, s, c->vanePartials, c->nVaneBlocks, c->vane, c->vaneSums, objOut);
+    launch_after(k_vane_finish, 1, BLOCK, 0, s, c->vanePartials, c->nVaneBlocks, c->vane, c->vaneSums, objOut,
+                 objHost);
 }
 
 template <typename R, typename S>
@@ -755,7 +762,7 @@ int primal_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double d
                                   cudaMemcpyDeviceToDevice, s);
         }
         if (st == 1 && c->objective == AFVM_OBJ_VANE) {
-            launch_vane_sums<R>(c, s, objDev, (const R*)recs[1]);
+            launch_vane_sums<R>(c, s, objDev, (const R*)recs[1], rule ? nullptr : c->hostOutDev + 1);
         } else if (st == 1 && c->objective != AFVM_OBJ_NONE) {
             int start = 0, n = m.nIC;
             if (c->objective == AFVM_OBJ_DRAG) { start = c->objStart; n = c->objN; }
@@ -782,6 +789,7 @@ int primal_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double d
             end.nPartials = nObjBlocks;
             end.dtcBits = c->dtcBits;
             end.dtcOut = dtcDev;
+            end.host = rule ? nullptr : c->hostOutDev;
             end.objOut = c->objective == AFVM_OBJ_VANE ? nullptr : objDev;    // (k_vane_finish's)
         }
         launch_flux_update<R, S>(c, st, dt, dtDev, u0c, u1c, u2c, Srho, SrhoU, SrhoE, out, s, st < 2 || nextStep,
@@ -835,7 +843,7 @@ AFVM_PRIMAL_INST(float, float)
 AFVM_PRIMAL_INST(float, double)
 template void default_sources<double>(Ctx*, const double*&, const double*&, const double*&);
 template void default_sources<float>(Ctx*, const float*&, const float*&, const float*&);
-template void launch_vane_sums<double>(Ctx*, cudaStream_t, double*, const double*);
-template void launch_vane_sums<float>(Ctx*, cudaStream_t, double*, const float*);
+template void launch_vane_sums<double>(Ctx*, cudaStream_t, double*, const double*, double*);
+template void launch_vane_sums<float>(Ctx*, cudaStream_t, double*, const float*, double*);
 
 }  // namespace afvm

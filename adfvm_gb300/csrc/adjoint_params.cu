@@ -53,8 +53,13 @@ __device__ __forceinline__ void ghost_bar(const MeshDev<R>& m, const Phys& P, co
     }
 }
 
+// The FP64 pipe binds (about 750 FP64 instructions a face): the face flux is evaluated once, into a
+// tape in registers and local memory that its VJP reads, where both needed an evaluation of their
+// own before; two blocks a SM hold more of it in registers than the compiler's choice: 768 -> 605 us a
+// launch of 317,955 faces. (Products on the integer pipes, soft64.cuh, gave 601 at three blocks: its
+// serial chains are too long for so few warps.)
 template <typename R, typename S>
-__global__ void __launch_bounds__(FLUX_BLOCK) k_param_face(MeshDev<R> m, Phys P, const R* __restrict__ rec, R coef,
+__global__ void __launch_bounds__(FLUX_BLOCK, 2) k_param_face(MeshDev<R> m, Phys P, const R* __restrict__ rec, R coef,
                                                            const S* __restrict__ ar, const S* __restrict__ au,
                                                            const S* __restrict__ ae, const R* __restrict__ fadj,
                                                            const R* __restrict__ cbar, int inviscid, int dragStage,
@@ -80,18 +85,24 @@ __global__ void __launch_bounds__(FLUX_BLOCK) k_param_face(MeshDev<R> m, Phys P,
     FaceIn<R> in;
     load_face<R>(m, rec, f, in);
     R F[5], maxaF;
-    face_flux<R>(P, kind, inviscid != 0, in, F, maxaF);
-    FaceBar<R> b;
+    FaceBar<R> b;      // (the cells' share comes from fadj: dead here)
     zero_bar(b);
     GeoBar<R> geo;
     zero_geo(geo);
-    face_vjp<R>(P, kind, inviscid != 0, in, Fb, b, &geo);
+    if (kind == FACE_BOUNDARY) {
+        face_flux<R>(P, kind, inviscid != 0, in, F, maxaF);
+        face_vjp<R>(P, kind, inviscid != 0, in, Fb, b, &geo);
+    } else {
+        TapeLocal<R, true> t;
+        face_flux<R>(P, kind, inviscid != 0, in, F, maxaF, t);
+        face_vjp_t<R>(P, kind, inviscid != 0, in, t, Fb, b, &geo);
+    }
     const R A = m.area[f];
     // op.div: + F A/V_L into the owner, - F A/V_R into the internal neighbour (1/V_L, 1/V_R from
     // the weights A/V_L, A/V_R of the volumesL / volumesR inputs)
     R sP = R(0), sN = R(0);
     for (int k = 0; k < 5; k++) { sP += rbP[k] * F[k]; sN += rbN[k] * F[k]; }
-    R rA = R(1) / A;
+    R rA = rcp(A);
     R areasb = sP * (wp * rA);
     R volLb = -sP * (wp * wp * rA);
     R volRb = R(0);

@@ -76,31 +76,25 @@ struct AdjFaceMesh {
     R wp, wn;          // A/V_L and, of an internal face, A/V_R
 };
 template <typename R, typename Q>
-__device__ __forceinline__ void load_adj_face_mesh(const MeshDev<R>& m, int f, AdjFaceMesh<R, Q>& a) {
-    a.at = load_face_mesh<R, Q>(m, f, a.in);
+__device__ __forceinline__ void load_adj_face_at(const MeshDev<R>& m, int f, AdjFaceMesh<R, Q>& a) {
+    a.at = face_at<R>(m, f);
     a.wp = m.wpf[f];
     a.wn = f < m.nIF ? m.wnf[f] : R(0);
 }
+template <typename R, typename Q>
+__device__ __forceinline__ void load_adj_face_mesh(const MeshDev<R>& m, int f, AdjFaceMesh<R, Q>& a) {
+    load_adj_face_at<R, Q>(m, f, a);
+    load_face_geometry<R, Q>(m, f, a.in);
+}
 
-// one face's record of k_adj_flux into st; TAPED: the forward values of a non-boundary face come
-// from its tape column instead of a re-evaluation of the face flux
-template <typename R, typename S, bool TAPED, typename Q, typename Stage>
-__device__ __forceinline__ void adj_face(const MeshDev<R>& m, const Phys& P, AdjFaceMesh<R, Q>& a,
-                                         const R* __restrict__ rec, R coef, const S* __restrict__ ar,
-                                         const S* __restrict__ au, const S* __restrict__ ae, int inviscid, int f,
-                                         const Stage& st, const R* __restrict__ tape, unsigned* most = nullptr) {
-    constexpr bool COLUMN = std::is_same<Stage, ColumnStage<R>>::value;
-    // (mixed contexts keep the order their FP64 adjoints have always rounded in)
-    constexpr bool VFIRST = sizeof(R) == 4 && sizeof(S) == 8;
-    const int kind = a.at.kind;
-    const bool fromTape = TAPED && kind != FACE_BOUNDARY;
-    if constexpr (TAPED && COLUMN)
-        if (fromTape) st.fetch(tape + f, (size_t)m.nF);
-    // Fbar = coef (abar_P A/V_L - abar_N A/V_R), coef folded into the two weights
+// the face flux's adjoint Fbar = coef (abar_P A/V_L - abar_N A/V_R), coef folded into the two weights
+template <typename R, typename S, typename Q>
+__device__ __forceinline__ void adj_seeds(const MeshDev<R>& m, const AdjFaceMesh<R, Q>& a, R coef,
+                                          const S* __restrict__ ar, const S* __restrict__ au,
+                                          const S* __restrict__ ae, int f, Q* Fb, unsigned* most = nullptr) {
     const int iP = a.at.own;
     Q wp = Q(coef) * Q(a.wp);
     R aP[5] = {R(ar[iP]), R(au[3 * iP]), R(au[3 * iP + 1]), R(au[3 * iP + 2]), R(ae[iP])};
-    Q Fb[5];
     for (int k = 0; k < 5; k++) {
         if constexpr (!std::is_same<R, Q>::value) soft_seen(*most, aP[k]);
         Fb[k] = Q(aP[k]) * wp;
@@ -114,36 +108,46 @@ __device__ __forceinline__ void adj_face(const MeshDev<R>& m, const Phys& P, Adj
             Fb[k] = Fb[k] - Q(aN[k]) * wn;
         }
     }
+}
+
+// one face's record of k_adj_flux into st; TAPED: the forward values of a non-boundary face come
+// from its tape column instead of a re-evaluation of the face flux
+template <typename R, typename S, bool TAPED, typename Q, typename Stage>
+__device__ __forceinline__ void adj_face(const MeshDev<R>& m, const Phys& P, AdjFaceMesh<R, Q>& a,
+                                         const R* __restrict__ rec, R coef, const S* __restrict__ ar,
+                                         const S* __restrict__ au, const S* __restrict__ ae, int inviscid, int f,
+                                         const Stage& st, const R* __restrict__ tape, unsigned* most = nullptr) {
+    constexpr bool COLUMN = std::is_same<Stage, ColumnStage<R>>::value;
+    const int kind = a.at.kind;
+    const bool fromTape = TAPED && kind != FACE_BOUNDARY;
+    if constexpr (TAPED && COLUMN)
+        if (fromTape) st.fetch(tape + f, (size_t)m.nF);
+    Q Fb[5];
+    adj_seeds<R, S, Q>(m, a, coef, ar, au, ae, f, Fb, most);
     FaceIn<Q>& in = a.in;
     FaceBar<Q> b;
     zero_bar(b);
     if (fromTape) {
         if constexpr (COLUMN) {
             st.fetched();
-            face_vjp_t<Q, VFIRST>(P, kind, inviscid != 0, in, TapeColumn<R, Q>{st.col, most}, Fb, b);
+            face_vjp_t<Q>(P, kind, inviscid != 0, in, TapeColumn<R, Q>{st.col, most}, Fb, b);
         } else {
-            face_vjp_t<Q, VFIRST>(P, kind, inviscid != 0, in, TapeLoad<R, Q>{tape + f, (size_t)m.nF, most}, Fb, b);
+            face_vjp_t<Q>(P, kind, inviscid != 0, in, TapeLoad<R, Q>{tape + f, (size_t)m.nF, most}, Fb, b);
         }
     } else {
         load_face_cells<R, Q>(rec, a.at, in, most);
-        if constexpr (kGauge<R>) {
-            // the VJP differentiates the absolute-form flux (the same function of the state as
-            // the gauge form the forward evaluates)
-            in.TP = rec_abs_T<R>(P, in.TP); in.TN = rec_abs_T<R>(P, in.TN);
-            in.pP = rec_abs_p<R>(P, in.pP); in.pN = rec_abs_p<R>(P, in.pN);
-        }
         if constexpr (COLUMN && !TAPED) {
             if (kind != FACE_BOUNDARY) {
                 // the forward's values through the column
                 const TapeColumn<R, Q> t{st.col, most};
                 Q F[5], maxaF;
                 face_flux<Q>(P, kind, inviscid != 0, in, F, maxaF, t);
-                face_vjp_t<Q, VFIRST>(P, kind, inviscid != 0, in, t, Fb, b);
+                face_vjp_t<Q>(P, kind, inviscid != 0, in, t, Fb, b);
             } else {
-                face_vjp<Q, VFIRST>(P, kind, inviscid != 0, in, Fb, b);
+                face_vjp<Q>(P, kind, inviscid != 0, in, Fb, b);
             }
         } else {
-            face_vjp<Q, VFIRST>(P, kind, inviscid != 0, in, Fb, b);
+            face_vjp<Q>(P, kind, inviscid != 0, in, Fb, b);
         }
     }
     const Q* src = &b.UP[0];
@@ -164,7 +168,7 @@ __device__ __noinline__ void adj_face_again(const MeshDev<R>& m, const Phys& P, 
 }
 
 template <typename R, typename S, bool TAPED, int NT>
-__global__ void __launch_bounds__(NT, (sizeof(R) == 8 ? 3 : 5) * FLUX_BLOCK / NT)
+__global__ void __launch_bounds__(NT, 3 * FLUX_BLOCK / NT)
     k_adj_flux(MeshDev<R> m, Phys P, const R* __restrict__ rec, R coef, const S* __restrict__ ar,
                const S* __restrict__ au, const S* __restrict__ ae, R* __restrict__ fadj, int inviscid,
                const R* __restrict__ tape) {
@@ -182,6 +186,78 @@ __global__ void __launch_bounds__(NT, (sizeof(R) == 8 ? 3 : 5) * FLUX_BLOCK / NT
                                  tape);
     __syncthreads();
     store_staged<R, FADJ, NT>(fadj, f0, min(NT, m.nF - f0), stage);
+}
+
+// the forward values of a warp's faces in shared memory, value k of lane's face at p[32 k]. FULL: all
+// of them, else those of a lean tape (TapeLocal)
+template <bool FULL>
+struct TapeWarp {
+    static constexpr bool kFull = FULL;
+    float* p;
+    __device__ __forceinline__ void put(int k, float x) const { p[32 * k] = x; }
+    __device__ __forceinline__ float get(int k) const { return p[32 * k]; }
+};
+
+// FP32. The kernel waits for its loads (and issues 44 % of the time), so the warps a SM holds count:
+// the forward values of a face go through shared memory instead of registers, which lets six
+// blocks a SM in at 80 registers without spills, and each warp copies its 32 records out of the
+// same memory by itself, in one bulk copy: no barrier of the block, no loads and stores for it.
+// At 128^3 412 -> 368 us a launch (five blocks 392, seven 472; the same with block-wide
+// staging 379, with the cell records fetched by the warp together 397). Mixed contexts: 5 blocks a SM,
+// 80^3 step and adjoint 1.131 ms (six 1.159, four 1.166).
+template <typename S, int NT>
+__global__ void __launch_bounds__(NT, NT == 32 ? 12 : sizeof(S) == 8 ? 5 : 6)
+    k_adj_flux_f32(MeshDev<float> m, Phys P, const float* __restrict__ rec, float coef, const S* __restrict__ ar,
+                   const S* __restrict__ au, const S* __restrict__ ae, float* __restrict__ fadj, int inviscid) {
+    static_assert(FADJ <= TAPE, "a warp's forward values, then its results");
+    __shared__ __align__(16) float shared[NT / 32][32 * TAPE];
+    const int lane = threadIdx.x & 31;
+    const int f = blockIdx.x * NT + threadIdx.x;
+    float* sh = shared[threadIdx.x >> 5];
+    AdjFaceMesh<float, float> a;
+    if (f < m.nF) load_adj_face_at<float, float>(m, f, a);
+    dep_wait(rec, ar, au, ae, fadj);
+    float v[FADJ];
+    if (f < m.nF) {
+        float Fb[5];
+        adj_seeds<float, S, float>(m, a, coef, ar, au, ae, f, Fb);
+        FaceIn<float>& in = a.in;
+        FaceBar<float> b;
+        zero_bar(b);
+        load_face_geometry<float, float>(m, f, in);
+        load_face_cells<float, float>(rec, a.at, in);
+        // the VJP differentiates the absolute-form flux (the same function of the state as the
+        // gauge form the forward evaluates)
+        in.TP = rec_abs_T<float>(P, in.TP); in.TN = rec_abs_T<float>(P, in.TN);
+        in.pP = rec_abs_p<float>(P, in.pP); in.pN = rec_abs_p<float>(P, in.pN);
+        // (mixed contexts keep the operations and the order their FP64 adjoints have always
+        // rounded in)
+        constexpr bool VFIRST = sizeof(S) == 8;
+        if (a.at.kind != FACE_BOUNDARY) {
+            const TapeWarp<!VFIRST> t{sh + lane};
+            float F[5], maxaF;
+            face_flux<float>(P, a.at.kind, inviscid != 0, in, F, maxaF, t);
+            face_vjp_t<float, VFIRST>(P, a.at.kind, inviscid != 0, in, t, Fb, b);
+        } else {
+            face_vjp<float, VFIRST>(P, a.at.kind, inviscid != 0, in, Fb, b);
+        }
+        const float* src = &b.UP[0];
+        for (int k = 0; k < 5; k++) { v[k] = src[k]; v[20 + k] = src[5 + k]; }
+        for (int k = 0; k < 15; k++) { v[5 + k] = src[10 + k]; v[25 + k] = src[25 + k]; }
+    }
+    __syncwarp();
+    if (f < m.nF) stage_row<float, FADJ>(sh + lane * FADJ, v);
+    // the warp's records, contiguous in fadj, in one bulk copy
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0 && f < m.nF) {
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(fadj + (size_t)f * FADJ),
+                     "r"((unsigned)__cvta_generic_to_shared(sh)),
+                     "r"((unsigned)(min(32, m.nF - f) * FADJ * sizeof(float)))
+                     : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    }
 }
 
 // The same with products, reciprocals and square roots on the integer pipes (soft64.cuh), FP64.
@@ -233,87 +309,45 @@ int prepare_adjoint(Ctx* c) {
     return e == cudaSuccess ? AFVM_OK : cuda_fail(c, e, "adjoint set-up");
 }
 
-// one cell's sum of its faces' adjoint records (and of the ghosts whose gradient is its own):
-// e the cell's faces in collate order, ghosts gs0..gs1 of the list
+// One cell's sum of its faces' adjoint records (and of the ghosts whose gradient is its own) in
+// collate order. Bound by the records' bytes; a thread sums one 16-byte piece of its cell's record,
+// so that the lanes side by side read a record's pieces side by side: with a thread a cell each
+// load asked for 32 different lines. At 128^3 in FP32 246 -> 189 us (1.23 GB of records, indexes and
+// results: 6.5 TB/s), at 64^3 in FP64 92 -> 62 us (320 and 640 threads a block: 63, 65).
+constexpr int CELL1_BLOCK = 160;
 template <typename R>
-__device__ __forceinline__ void adj_cell_gather(const MeshDev<R>& m, const R* __restrict__ fadj, const int* e, int gs0,
-                                                int gs1, R* row) {
-    // the first slot initialises the sums: adding it to zeros would cost 20 more adds (FP64
-    // pipe issues in double) and changes nothing but the sign of a zero
-    R acc[CBAR];
+__global__ void __launch_bounds__(CELL1_BLOCK) k_adj_cell1(MeshDev<R> m, const R* __restrict__ fadj, R* __restrict__ cbar) {
+    constexpr int PER = 16 / sizeof(R), PIECES = CBAR / PER;
+    const long long t = blockIdx.x * (long long)CELL1_BLOCK + threadIdx.x;
+    const int c = (int)(t / PIECES), k0 = PER * (int)(t % PIECES);
+    int e[6], gs0 = 0, gs1 = 0;
+    if (c < m.nIC) {
+#pragma unroll
+        for (int s = 0; s < 6; s++) e[s] = m.accf[s * (size_t)m.nIC + c];
+        gs0 = m.gsStart[c];
+        gs1 = m.gsStart[c + 1];
+    }
+    dep_wait(fadj, cbar);
+    if (c >= m.nIC) return;
+    R v[6][PER], acc[PER];
 #pragma unroll
     for (int s = 0; s < 6; s++) {
-        bool ownerSide = e[s] >= 0;
-        int f = ownerSide ? e[s] : ~e[s];
-        R v[CBAR];
-        load_vec(fadj + (size_t)f * FADJ + (ownerSide ? 0 : CBAR), v, CBAR);
-        if (s == 0)
-            for (int k = 0; k < CBAR; k++) acc[k] = v[k];
-        else
-            for (int k = 0; k < CBAR; k++) acc[k] += v[k];
+        const bool ownerSide = e[s] >= 0;
+        load_vec(fadj + (size_t)(ownerSide ? e[s] : ~e[s]) * FADJ + (ownerSide ? 0 : CBAR) + k0, v[s], PER);
     }
+    // the first slot initialises the sums (adding it to zeros changes nothing but the sign of a
+    // zero)
+    for (int k = 0; k < PER; k++) acc[k] = v[0][k];
+#pragma unroll
+    for (int s = 1; s < 6; s++)
+        for (int k = 0; k < PER; k++) acc[k] += v[s][k];
     // gradient adjoints of the ghosts whose gradient is a copy of this cell's
     for (int q = gs0; q < gs1; q++) {
-        int g = m.gsList[q];
-        const R* r = fadj + (size_t)(m.nIF + g) * FADJ;
-        for (int k = 0; k < 15; k++) acc[5 + k] += r[25 + k];
+        const R* r = fadj + (size_t)(m.nIF + m.gsList[q]) * FADJ + CBAR + k0;
+        for (int k = 0; k < PER; k++)
+            if (k0 + k >= 5) acc[k] += r[k];
     }
-    stage_row<R, CBAR>(row, acc);
-}
-
-template <typename R, int NT>
-__global__ void __launch_bounds__(NT) k_adj_cell1(MeshDev<R> m, const R* __restrict__ fadj, R* __restrict__ cbar) {
-    __shared__ __align__(16) R stage[NT * CBAR];
-    const int c0 = blockIdx.x * NT;
-    const int c = c0 + threadIdx.x;
-    int e[6], gs0 = 0, gs1 = 0;
-    if (c < m.nIC) {
-#pragma unroll
-        for (int s = 0; s < 6; s++) e[s] = m.accf[s * (size_t)m.nIC + c];
-        gs0 = m.gsStart[c];
-        gs1 = m.gsStart[c + 1];
-    }
-    dep_wait(fadj, cbar);
-    if (c < m.nIC) adj_cell_gather<R>(m, fadj, e, gs0, gs1, stage + threadIdx.x * CBAR);
-    __syncthreads();
-    if (c0 < m.nIC) store_staged<R, CBAR, NT>(cbar, c0, min(NT, m.nIC - c0), stage);
-}
-
-
-// the split form (CellAt): warp q of a block sums values 4q..4q+3 of 32 cells
-template <typename R>
-__global__ void __launch_bounds__(160) k_adj_cell1_split(MeshDev<R> m, const R* __restrict__ fadj, R* __restrict__ cbar) {
-    __shared__ __align__(16) R stage[32 * CBAR];
-    const CellAt<true> at;
-    const int c = at.c, k0 = 4 * at.q0, c0 = blockIdx.x * 32;
-    int e[6], gs0 = 0, gs1 = 0;
-    if (c < m.nIC) {
-#pragma unroll
-        for (int s = 0; s < 6; s++) e[s] = m.accf[s * (size_t)m.nIC + c];
-        gs0 = m.gsStart[c];
-        gs1 = m.gsStart[c + 1];
-    }
-    dep_wait(fadj, cbar);
-    if (c < m.nIC) {
-        R v[6][4], acc[4];
-#pragma unroll
-        for (int s = 0; s < 6; s++) {
-            const bool ownerSide = e[s] >= 0;
-            load_vec(fadj + (size_t)(ownerSide ? e[s] : ~e[s]) * FADJ + (ownerSide ? 0 : CBAR) + k0, v[s], 4);
-        }
-        for (int k = 0; k < 4; k++) acc[k] = v[0][k];
-#pragma unroll
-        for (int s = 1; s < 6; s++)
-            for (int k = 0; k < 4; k++) acc[k] += v[s][k];
-        for (int q = gs0; q < gs1; q++) {
-            const R* r = fadj + (size_t)(m.nIF + m.gsList[q]) * FADJ + CBAR + k0;
-            for (int k = 0; k < 4; k++)
-                if (k0 + k >= 5) acc[k] += r[k];
-        }
-        for (int k = 0; k < 4; k++) stage[(threadIdx.x & 31) * CBAR + k0 + k] = acc[k];
-    }
-    __syncthreads();
-    if (c0 < m.nIC) store_staged<R, CBAR, 160>(cbar, c0, min(32, m.nIC - c0), stage);
+    stage_row<R, PER>(cbar + (size_t)c * CBAR + k0, acc);
 }
 
 // phiFbar_i = rv * sum_j G[i][j] sn_j  (transpose of grad += phiF (x) S N', scaled by 1/V)
@@ -610,39 +644,30 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
         {
             ProfScope ps(c, KID_ADJ_FLUX, s);
             const R* ft = faceTape ? faceTape + (size_t)st * TAPE * m.nF : nullptr;
-            using Small = std::integral_constant<int, 32>;
-            using Big = std::integral_constant<int, FLUX_BLOCK>;
             const bool small = gF.threads == 32;
-            auto flux = [&](auto taped, auto nt) {
-                launch_after(k_adj_flux<R, S, decltype(taped)::value, decltype(nt)::value>, gF.blocks, gF.threads, 0, s,
-                             m, P, rec, coef, ain[0], ain[1], ain[2], fadj, inviscid, ft);
-            };
-            bool done = false;
-            if constexpr (std::is_same<R, double>::value) {
-                if (use_soft(c, m.nF) && std::fabs(coef) < 0x1p64) {
-                    auto soft = [&](auto kernel) {
-                        launch_after(kernel, (m.nF + FLUX_BLOCK - 1) / FLUX_BLOCK, FLUX_BLOCK, COLUMN_BYTES, s, m, P,
-                                     rec, coef, ain[0], ain[1], ain[2], fadj, inviscid, ft);
-                    };
-                    if (ft) soft(k_adj_flux_soft<true>);
-                    else soft(k_adj_flux_soft<false>);
-                    done = true;
-                }
+            if constexpr (std::is_same<R, float>::value) {
+                launch_after(small ? k_adj_flux_f32<S, 32> : k_adj_flux_f32<S, FLUX_BLOCK>, gF.blocks, gF.threads, 0, s,
+                             m, P, rec, coef, ain[0], ain[1], ain[2], fadj, inviscid);
+            } else if (use_soft(c, m.nF) && std::fabs(coef) < 0x1p64) {
+                launch_after(ft ? k_adj_flux_soft<true> : k_adj_flux_soft<false>, (m.nF + FLUX_BLOCK - 1) / FLUX_BLOCK,
+                             FLUX_BLOCK, COLUMN_BYTES, s, m, P, rec, coef, ain[0], ain[1], ain[2], fadj, inviscid, ft);
+            } else {
+                auto flux = [&](auto taped, auto nt) {
+                    launch_after(k_adj_flux<R, S, decltype(taped)::value, decltype(nt)::value>, gF.blocks, gF.threads,
+                                 0, s, m, P, rec, coef, ain[0], ain[1], ain[2], fadj, inviscid, ft);
+                };
+                using Small = std::integral_constant<int, 32>;
+                using Big = std::integral_constant<int, FLUX_BLOCK>;
+                if (ft && small) flux(std::true_type{}, Small{});
+                else if (ft) flux(std::true_type{}, Big{});
+                else if (small) flux(std::false_type{}, Small{});
+                else flux(std::false_type{}, Big{});
             }
-            if (done) {
-                // (launched)
-            } else if (ft && small) flux(std::true_type{}, Small{});
-            else if (ft) flux(std::true_type{}, Big{});
-            else if (small) flux(std::false_type{}, Small{});
-            else flux(std::false_type{}, Big{});
         }
         {
             ProfScope ps(c, KID_ADJ_GATHER, s);
-            if (split)
-                launch_after(k_adj_cell1_split<R>, (m.nIC + 31) / 32, 160, 0, s, m, (const R*)fadj, cbar);
-            else
-                launch_after(gC.threads == 32 ? k_adj_cell1<R, 32> : k_adj_cell1<R, BLOCK>, gC.blocks, gC.threads, 0, s,
-                             m, (const R*)fadj, cbar);
+            const long long n = m.nIC * (CBAR * sizeof(R) / 16);
+            launch_after(k_adj_cell1<R>, (int)((n + CELL1_BLOCK - 1) / CELL1_BLOCK), CELL1_BLOCK, 0, s, m, (const R*)fadj, cbar);
         }
         // the stage's share of the mesh / boundary-input gradients (before the cell kernel: the
         // adjoint outputs it writes may alias this stage's input adjoints)

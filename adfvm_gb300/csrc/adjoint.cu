@@ -17,6 +17,7 @@
 #include <cmath>
 #include <type_traits>
 #include "facedev.cuh"
+#include "ff32.cuh"
 #include "vane.cuh"
 
 namespace afvm {
@@ -362,7 +363,7 @@ __global__ void __launch_bounds__(SPLIT ? 160 : BLOCK)
                 const R* __restrict__ cbar, const S* __restrict__ ur, const S* __restrict__ uu,
                 const S* __restrict__ ue, const S* ainr, const S* ainu, const S* aine, S* a1r, S* a1u, S* a1e, S* a0r,
                 S* a0u, S* a0e, S* sb, S* sr, S* su, S* se, double dt, int objective, int objStart, int objN,
-                double obja, VaneDev vane, const double* __restrict__ objSeed) {
+                double obja, ff objaPair, VaneDev vane, const double* __restrict__ objSeed) {
     const CellAt<SPLIT> at;
     const int c = at.c;
     const bool first = !SPLIT || at.q0 == 0;        // the thread that goes on with the whole cell
@@ -484,7 +485,12 @@ __global__ void __launch_bounds__(SPLIT ? 160 : BLOCK)
         // objective on the stage-1 primitives
         if (STAGE == 1 && objective != AFVM_OBJ_NONE) {
             const R* rc = rec + (size_t)c * REC;
-            if (objective == AFVM_OBJ_KINETIC_ENERGY) {
+            bool done = false;
+            if constexpr (sizeof(S) == 4)
+                done = objective == AFVM_OBJ_KINETIC_ENERGY && kinetic_grad_ff(P.pair, objaPair, rc, m.vol[c], pbar);
+            if (done) {
+                // (added in pairs of floats)
+            } else if (objective == AFVM_OBJ_KINETIC_ENERGY) {
                 double U[3] = {rc[0], rc[1], rc[2]}, T = rec_T<R>(P, rc[R_T]), p = rec_p<R>(P, rc[R_P]), V = m.vol[c];
                 double d = (P.Cv * T) * P.gm1;
                 double rd = rcp(d);           // (Newton reciprocals: no IEEE divisions on the FP64 pipe)
@@ -681,7 +687,7 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
                          split ? (m.nIC + 31) / 32 : gC.blocks, split ? 160 : gC.threads, 0, s, m, P, rec,
                          (const R*)fadj, (const R*)cbar, u[0], u[1], u[2], ain[0], ain[1], ain[2], a1[0], a1[1], a1[2],
                          rhoa, rhoUa, rhoEa, sb, Srhoa, SrhoUa, SrhoEa, dt, c->objective, c->objStart, c->objN, obja,
-                         c->vane, c->objSeed);
+                         ff_of(obja), c->vane, c->objSeed);
         };
         if (st == 2) cells(std::integral_constant<int, 2>{});
         else if (st == 1) cells(std::integral_constant<int, 1>{});

@@ -93,6 +93,19 @@ struct PhysR {
     R gP, gT, gH, gK;
 };
 
+// pairs of floats h + l (ff32.cuh), and the constants that meet them in FP32 contexts
+struct ff {
+    float h, l;
+};
+inline ff ff_of(double x) {
+    const float h = (float)x;
+    return {h, (float)(x - (double)h)};
+}
+struct PhysFF {
+    ff gm1, rCv, Rg;
+    float gP, gT;
+};
+
 // FP32 cell records hold the pressure and temperature as offsets from a gauge state,
 // p - gaugeP and T - gaugeT, and the FP32 face fluxes carry the momentum flux without
 // gaugeP N and the energy flux less gaugeH times the mass flux. The update adds gaugeH times
@@ -109,6 +122,7 @@ struct Phys {
     double gaugeP = 0.0, gaugeT = 0.0, gaugeH = 0.0;
     PhysR<double> d;
     PhysR<float> f;
+    PhysFF pair;
 };
 
 // the record types that hold gauge offsets
@@ -142,6 +156,7 @@ inline void fill_consts(const Phys& P, PhysR<R>& q) {
 inline void finish_phys(Phys& P) {
     fill_consts(P, P.d);
     fill_consts(P, P.f);
+    P.pair = {ff_of(P.gm1), ff_of(P.rCv), ff_of(P.Cv * P.gm1), (float)P.gaugeP, (float)P.gaugeT};
 }
 
 // the precision of a working type's constants (a double evaluated otherwise, soft64.cuh, has

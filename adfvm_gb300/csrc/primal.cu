@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 #include "ctx.cuh"
 #include "facedev.cuh"
+#include "ff32.cuh"
 #include "vane.cuh"
 
 namespace afvm {
@@ -31,12 +32,14 @@ __device__ __noinline__ void primitive_d(const Phys& P, double rho, double r0, d
     out[3] = e * P.rCv;
 }
 
-// FP32 state: velocity and temperature in float; the internal energy rho*e = rhoE - |rhoU|^2/(2 rho)
-// (the low-Mach cancellation) and the pressure recovered in double from the float state.
-__device__ __noinline__ void primitive_f(const Phys& P, float rho, float r0, float r1, float r2, float rhoE,
-                                         float* out) {
+// FP32 state: velocity in float; the internal energy rho*e = rhoE - |rhoU|^2/(2 rho) (the low-Mach
+// cancellation), the pressure and the temperature from the float state in pairs of floats, or in
+// double where a value is out of their range
+__device__ __noinline__ void primitive_f(const Phys& P, float rho, float r0, float r1, float r2,
+                                         float rhoE, float* out) {
     float rr = rcp(rho);
     out[0] = r0 * rr; out[1] = r1 * rr; out[2] = r2 * rr;
+    if (__builtin_expect(prim_ff(P.pair, rho, r0, r1, r2, rhoE, rr, out + R_P, out + R_T), 1)) return;
     double q = (double)r0 * r0 + (double)r1 * r1 + (double)r2 * r2;
     double rhoe = (double)rhoE - 0.5 * q * (double)rr;
     out[4] = (float)(P.gm1 * rhoe - P.gaugeP);

@@ -183,6 +183,14 @@ def check(status, ctx=None, what=''):
         raise AfvmError(status, msg)
 
 
+def stream_of(t):
+    """The handle of the current stream of the CUDA tensor t's device."""
+    import torch
+    if not t.is_cuda:
+        torch.cuda.current_stream(t.device)      # (raises)
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
+
+
 def to_device(a, t):
     """Host array `a` (numpy, float64 or float32, any host memory) into the CUDA tensor `t`
     (same number of values, float64 or float32), converted when the types differ; ordered on
@@ -190,13 +198,11 @@ def to_device(a, t):
     import numpy as np
     import torch
     a = np.ascontiguousarray(a)
-    if (a.dtype not in (np.float64, np.float32) or t.dtype not in (torch.float64, torch.float32)
-            or a.size != t.numel() or not t.is_contiguous() or t.device.type != 'cuda'):
+    if (a.dtype.char not in 'df' or not a.dtype.isnative or t.dtype not in (torch.float64, torch.float32)
+            or a.size != t.numel() or not t.is_contiguous() or not t.is_cuda):
         raise ValueError('to_device: %s array of %d values into a %s tensor of %d' % (a.dtype, a.size, t.dtype, t.numel()))
-    stream = torch.cuda.current_stream(t.device).cuda_stream
-    check(lib().afvm_copy_to_device(t.device.index, C.c_void_p(t.data_ptr()), t.element_size(),
-                                    C.c_void_p(a.ctypes.data), a.itemsize, a.size, C.c_void_p(stream)),
-          None, 'afvm_copy_to_device')
+    check(lib().afvm_copy_to_device(t.get_device(), t.data_ptr(), t.element_size(), a.ctypes.data, a.itemsize,
+                                    a.size, stream_of(t)), None, 'afvm_copy_to_device')
     return t
 
 
@@ -204,16 +210,13 @@ def to_host(t, out):
     """The CUDA tensor `t` (float64 or float32) into the numpy array `out` (float64 or float32,
     C-contiguous, same number of values), converted when the types differ; returns once `out`
     holds the values (afvm_copy_to_host)."""
-    import numpy as np
     import torch
     t = t.contiguous()
-    if (out.dtype not in (np.float64, np.float32) or t.dtype not in (torch.float64, torch.float32)
-            or out.size != t.numel() or not out.flags['C_CONTIGUOUS'] or t.device.type != 'cuda'):
+    if (out.dtype.char not in 'df' or not out.dtype.isnative or t.dtype not in (torch.float64, torch.float32)
+            or out.size != t.numel() or not out.flags.c_contiguous or not t.is_cuda):
         raise ValueError('to_host: %s tensor of %d values into a %s array of %d' % (t.dtype, t.numel(), out.dtype, out.size))
-    stream = torch.cuda.current_stream(t.device).cuda_stream
-    check(lib().afvm_copy_to_host(t.device.index, C.c_void_p(out.ctypes.data), out.itemsize,
-                                  C.c_void_p(t.data_ptr()), t.element_size(), out.size, C.c_void_p(stream)),
-          None, 'afvm_copy_to_host')
+    check(lib().afvm_copy_to_host(t.get_device(), out.ctypes.data, out.itemsize, t.data_ptr(), t.element_size(),
+                                  out.size, stream_of(t)), None, 'afvm_copy_to_host')
     return out
 
 

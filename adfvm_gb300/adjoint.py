@@ -64,12 +64,12 @@ class Adjoint(object):
         m = self.mesh
         nT, nS = len(Mesh.gradFields) + len(Mesh.intFields), len(m.getScalar())
         base = 4 + nT + nS
-        nBC = len(p.getBoundaryTensor(1)) + len(p.extraArgs())
+        nB = len(p.getBoundaryTensor(1))
+        nBC = nB + len(p.extraArgs())
         primal_in = inputs[:base + 3 + nBC]
         rest = inputs[base + 3 + nBC:]
         if len(rest) != 6:
             raise ValueError('adjoint map: expected 3 adjoint fields, dtca, obja and scaling after the primal inputs')
-        nB = len(p.getBoundaryTensor(1))
         p._apply_bc_tensors(list(primal_in[base + 3:base + 3 + nB]))
         p._apply_extra(list(primal_in[base + 3 + nB:]))
         x = p.upload(primal_in[:3])
@@ -142,12 +142,10 @@ class Adjoint(object):
         checkpoints = []
         x = x0
         objs = []
-        for k in range(nSteps):
-            if k % writeInterval == 0:
-                checkpoints.append([t.clone() for t in x])
-            r = p.step(x[0], x[1], x[2], dts[k], S=S)
-            objs.append(r[4])
-            x = list(r[:3])
+        for k in range(0, nSteps, writeInterval):
+            checkpoints.append(x)
+            x = [t.clone() for t in x]
+            objs += p.run_fixed(x, dts[k:k + writeInterval], S)
         perts = [[torch.as_tensor(np.ascontiguousarray(np.asarray(a, np.float64).reshape(-1)), device=dev)
                   for a in pert] for pert in perturbations]
         result = [0.0] * len(perts)

@@ -63,9 +63,17 @@ int stager_wait(Stager& st, int k) {
     return AFVM_OK;
 }
 
+// the host threads for `bytes` of copying or page touching: one for every 256 KB, so that a small array
+// wakes none (a parallel region of 16 threads that have gone to sleep costs more than 37 KB take;
+// the map's 24 copies of 1,536 cells' arrays)
+int threads_for(size_t bytes) {
+    const size_t most = (size_t)omp_get_max_threads(), want = bytes / (size_t(256) << 10);
+    return (int)(want < 1 ? 1 : (want < most ? want : most));
+}
+
 // n values from src (element size ss) to dst (element size ds), split over the host threads
 void host_convert(void* dst, int ds, const void* src, int ss, size_t n) {
-    const int nt = omp_get_max_threads();
+    const int nt = threads_for(n * (size_t)(ss > ds ? ss : ds));
     const size_t per = (n + (size_t)nt - 1) / (size_t)nt;
 #pragma omp parallel num_threads(nt)
     {
@@ -131,7 +139,7 @@ void touch_pages(void* p, size_t bytes) {
     if (!bytes) return;
     unsigned char* b = (unsigned char*)p;
     const long long pages = (long long)((bytes + 4095) / 4096);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) num_threads(threads_for(bytes))
     for (long long i = 0; i < pages; i++) b[(size_t)i * 4096] = 0;
     b[bytes - 1] = 0;
 }

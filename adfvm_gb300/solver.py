@@ -28,6 +28,7 @@ The GPU library is mandatory: there is no CPU path.
 """
 import collections
 import ctypes as C
+import functools
 import os
 import sys
 
@@ -74,6 +75,12 @@ class ObjectiveSolver(object):
         if self._rcf.mu is None:
             return SUTHERLAND[0] * T ** 1.5 / (T + SUTHERLAND[1])
         return T * 0 + float(self._rcf.mu)
+
+
+@functools.lru_cache(maxsize=64)
+def _sample(n):
+    """The indexes at which a fingerprint reads an array of n values."""
+    return np.linspace(0, n - 1, num=min(n, 97)).astype(np.int64)
 
 
 class RCF(object):
@@ -176,6 +183,7 @@ class RCF(object):
         st = L.lib().afvm_ctx_create(C.byref(mt), bcs, C.byref(phys), self.precision, self.device, C.byref(ctx))
         L.check(st, None, 'afvm_ctx_create')
         self._ctx = ctx
+        self._bufferTypes = None
         self._bcvals = self.getBoundaryTensor(1)
         if self.vane is not None:
             self._set_vane(self.vane)
@@ -397,8 +405,7 @@ class RCF(object):
                 parts.append(b'-')
                 continue
             v = np.asarray(a).reshape(-1)
-            idx = np.linspace(0, len(v) - 1, num=min(len(v), 97)).astype(np.int64)
-            parts.append(np.ascontiguousarray(v[idx]).tobytes())
+            parts.append(v[_sample(len(v))].tobytes())
             parts.append(str(v.shape).encode())
         return b'|'.join(parts)
 
@@ -493,13 +500,21 @@ class RCF(object):
         td = torch.float64 if self.record_dtype == np.float64 else torch.float32
         return torch.empty(int(L.lib().afvm_tape_elements(self._ctx)), dtype=td, device='cuda:%d' % self.device)
 
+    def _buffer_types(self):
+        """The torch types of the states and of the records, and a tape's number of values."""
+        t = self._bufferTypes
+        if t is None:
+            torch = _torch()
+            t = self._bufferTypes = (torch.float64 if self.dtype == np.float64 else torch.float32,
+                                     torch.float64 if self.record_dtype == np.float64 else torch.float32,
+                                     int(L.lib().afvm_tape_elements(self._ctx)))
+        return t
+
     def _check_tape(self, tape, stages):
-        torch = _torch()
-        td = torch.float64 if self.record_dtype == np.float64 else torch.float32
+        td, n = self._buffer_types()[1:]
         if stages is None:
             raise ValueError('tape: kept together with stages')
-        if tape.dtype != td or tape.numel() < int(L.lib().afvm_tape_elements(self._ctx)) or \
-                not tape.is_contiguous() or not tape.is_cuda:
+        if tape.dtype != td or tape.numel() < n or not tape.is_contiguous() or not tape.is_cuda:
             raise ValueError('tape: a contiguous device buffer of afvm_tape_elements %s values' % td)
         return tape
 
@@ -509,26 +524,23 @@ class RCF(object):
         adjoint_step(..., stages=) on the same state; tape: optional tape_buffer() (with stages)
         that receives the step's face tape, for adjoint_step(..., tape=)."""
         torch = _torch()
-        stream = torch.cuda.current_stream(rho.device).cuda_stream
+        stream = L.stream_of(rho)
         if out is None:
             out = (torch.empty_like(rho), torch.empty_like(rhoU), torch.empty_like(rhoE))
-        Sp = [None, None, None] if S is None else [C.c_void_p(s.data_ptr()) for s in S]
+        Sp = (None, None, None) if S is None else [s.data_ptr() for s in S]
         dtc = C.c_double()
         obj = C.c_double()
-        sp = None if stages is None else C.c_void_p(self._check_stages(stages).data_ptr())
-        tp = None if tape is None else C.c_void_p(self._check_tape(tape, stages).data_ptr())
-        st = L.lib().afvm_primal_step_tape(self._ctx, C.c_void_p(rho.data_ptr()), C.c_void_p(rhoU.data_ptr()),
-                                           C.c_void_p(rhoE.data_ptr()), float(dt), Sp[0], Sp[1], Sp[2],
-                                           C.c_void_p(out[0].data_ptr()), C.c_void_p(out[1].data_ptr()),
-                                           C.c_void_p(out[2].data_ptr()), sp, tp,
-                                           C.byref(dtc) if want_scalars else None,
-                                           C.byref(obj) if want_scalars else None, C.c_void_p(stream))
+        sp = None if stages is None else self._check_stages(stages).data_ptr()
+        tp = None if tape is None else self._check_tape(tape, stages).data_ptr()
+        st = L.lib().afvm_primal_step_tape(self._ctx, rho.data_ptr(), rhoU.data_ptr(), rhoE.data_ptr(), float(dt),
+                                           Sp[0], Sp[1], Sp[2], out[0].data_ptr(), out[1].data_ptr(),
+                                           out[2].data_ptr(), sp, tp, C.byref(dtc) if want_scalars else None,
+                                           C.byref(obj) if want_scalars else None, stream)
         L.check(st, self._ctx, 'afvm_primal_step_tape')
         return out[0], out[1], out[2], dtc.value, self._objective_after(obj.value) if want_scalars else obj.value
 
     def _check_stages(self, stages):
-        torch = _torch()
-        td = torch.float64 if self.dtype == np.float64 else torch.float32
+        td = self._buffer_types()[0]
         if stages.dtype != td or stages.numel() < 10 * self.mesh.nInternalCells or not stages.is_contiguous() \
                 or not stages.is_cuda:
             raise ValueError('stages: a contiguous device buffer of 10 x nInternalCells %s values' % td)
@@ -662,23 +674,22 @@ class RCF(object):
         also the gradients with respect to those parameters (afvm_adjoint_step_params, FP64
         contexts), returned as a fifth item: a list of float64 CUDA tensors of param_shapes()."""
         torch = _torch()
-        stream = torch.cuda.current_stream(rho.device).cuda_stream
+        stream = L.stream_of(rho)
         if out is None:
             out = (torch.empty_like(rho), torch.empty_like(rhoU), torch.empty_like(rhoE))
         Sg = None
         if source_grad:
             Sg = tuple(source_out) if source_out is not None else \
                 (torch.empty_like(rho), torch.empty_like(rhoU), torch.empty_like(rhoE))
-        Sp = [None, None, None] if S is None else [C.c_void_p(s.data_ptr()) for s in S]
-        vp = lambda t: C.c_void_p(t.data_ptr())
-        gp = [None, None, None] if Sg is None else [vp(t) for t in Sg]
-        sp = None if stages is None else vp(self._check_stages(stages))
-        tp = None if tape is None else vp(self._check_tape(tape, stages))
+        Sp = (None, None, None) if S is None else [s.data_ptr() for s in S]
+        gp = (None, None, None) if Sg is None else [t.data_ptr() for t in Sg]
+        sp = None if stages is None else self._check_stages(stages).data_ptr()
+        tp = None if tape is None else self._check_tape(tape, stages).data_ptr()
         if params is None:
-            st = L.lib().afvm_adjoint_step_tape(self._ctx, vp(rho), vp(rhoU), vp(rhoE), float(dt), Sp[0], Sp[1],
-                                                Sp[2], sp, tp, vp(seeds[0]), vp(seeds[1]), vp(seeds[2]), 0.0,
-                                                float(obja), vp(out[0]), vp(out[1]), vp(out[2]), gp[0], gp[1], gp[2],
-                                                C.c_void_p(stream))
+            st = L.lib().afvm_adjoint_step_tape(self._ctx, rho.data_ptr(), rhoU.data_ptr(), rhoE.data_ptr(), float(dt),
+                                                Sp[0], Sp[1], Sp[2], sp, tp, seeds[0].data_ptr(), seeds[1].data_ptr(),
+                                                seeds[2].data_ptr(), 0.0, float(obja), out[0].data_ptr(),
+                                                out[1].data_ptr(), out[2].data_ptr(), gp[0], gp[1], gp[2], stream)
             L.check(st, self._ctx, 'afvm_adjoint_step_tape')
             return out[0], out[1], out[2], Sg
         grads = [torch.empty(sh, dtype=torch.float64, device=rho.device) for sh in self.param_shapes(params)]
@@ -698,10 +709,11 @@ class RCF(object):
             r = self._adjoint_step(rho, rhoU, rhoE, dt, seeds, obja, S, out, source_grad, stages, tape)
             grads[0].zero_()
             return r + (grads,)
-        st = L.lib().afvm_adjoint_step_params(self._ctx, vp(rho), vp(rhoU), vp(rhoE), float(dt), Sp[0], Sp[1], Sp[2],
-                                              sp, tp, vp(seeds[0]), vp(seeds[1]), vp(seeds[2]), 0.0, float(obja),
-                                              vp(out[0]), vp(out[1]), vp(out[2]), gp[0], gp[1], gp[2], C.byref(pg),
-                                              C.c_void_p(stream))
+        st = L.lib().afvm_adjoint_step_params(self._ctx, rho.data_ptr(), rhoU.data_ptr(), rhoE.data_ptr(), float(dt),
+                                              Sp[0], Sp[1], Sp[2], sp, tp, seeds[0].data_ptr(), seeds[1].data_ptr(),
+                                              seeds[2].data_ptr(), 0.0, float(obja), out[0].data_ptr(),
+                                              out[1].data_ptr(), out[2].data_ptr(), gp[0], gp[1], gp[2],
+                                              C.byref(pg), stream)
         L.check(st, self._ctx, 'afvm_adjoint_step_params')
         return out[0], out[1], out[2], Sg, grads
 
@@ -739,12 +751,11 @@ class RCF(object):
         for g, p in zip(gs, ps):
             if g.dtype != torch.float64 or p.dtype != torch.float64 or g.numel() != p.numel():
                 raise ValueError('sensitivity: float64 arrays of equal size required')
-        ga = (L._d * k)(*[C.cast(C.c_void_p(g.data_ptr()), L._d) for g in gs])
-        pa = (L._d * k)(*[C.cast(C.c_void_p(p.data_ptr()), L._d) for p in ps])
+        ga = C.cast((C.c_void_p * k)(*[g.data_ptr() for g in gs]), C.POINTER(L._d))
+        pa = C.cast((C.c_void_p * k)(*[p.data_ptr() for p in ps]), C.POINTER(L._d))
         na = (C.c_int64 * k)(*[g.numel() for g in gs])
         out = C.c_double()
-        stream = torch.cuda.current_stream(gs[0].device).cuda_stream
-        L.check(L.lib().afvm_sensitivity(self._ctx, k, ga, pa, na, C.byref(out), C.c_void_p(stream)), self._ctx)
+        L.check(L.lib().afvm_sensitivity(self._ctx, k, ga, pa, na, C.byref(out), L.stream_of(gs[0])), self._ctx)
         return out.value
 
     def adjoint_energy(self, adj, state):
@@ -775,6 +786,21 @@ class RCF(object):
                                      hp[0], hp[1], hp[2], C.c_void_p(stream))
         L.check(st, self._ctx, 'afvm_primal_run')
         return hist
+
+    def run_fixed(self, x, dts, S=None):
+        """len(dts) steps of these sizes in place on the CUDA tensors x = [rho, rhoU, rhoE]; returns
+        their objectives (floats). Steps of one size run on the device in one go (the same bits as
+        step() gives), the host waiting once instead of after each."""
+        if self.objectiveFn is None and all(d == dts[0] for d in dts):
+            torch = _torch()
+            obj = torch.zeros(len(dts), dtype=torch.float64, device=x[0].device)
+            Sp = (None, None, None) if S is None else [s.data_ptr() for s in S]
+            st = L.lib().afvm_primal_run(self._ctx, x[0].data_ptr(), x[1].data_ptr(), x[2].data_ptr(), len(dts),
+                                         float(dts[0]), float(self.CFL), float(self.stepFactor), 1, Sp[0], Sp[1], Sp[2],
+                                         None, None, C.cast(C.c_void_p(obj.data_ptr()), L._d), L.stream_of(x[0]))
+            L.check(st, self._ctx, 'afvm_primal_run')
+            return obj.tolist()
+        return [self.step(x[0], x[1], x[2], d, S=S, out=x)[4] for d in dts]
 
     # ------------------------------------------------------------------ case files
     @classmethod

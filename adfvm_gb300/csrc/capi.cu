@@ -562,7 +562,8 @@ static bool soft_inputs(const HostTables& h, const Phys& P) {
         if (!(std::fabs(v) < 0x1p64)) return false;
     for (double d : h.dlt)
         if (!(d > 0x1p-64)) return false;              // 1/deltas
-    return below(h.nrm) && below(h.du) && below(h.lw) && below(h.qw) && below(h.wpf) && below(h.wnf);
+    return below(h.nrm) && below(h.du) && below(h.lw) && below(h.qw) && below(h.wpf) && below(h.wnf) &&
+           below(h.accw);
 }
 
 // the default gauge state: the mean fixed boundary pressure and temperature (the totals of

@@ -402,9 +402,13 @@ __device__ __forceinline__ void step_end(const StepEnd& e) {
 
 // Gather of the face fluxes (op.div / op.absDiv, op.py:12-29, collated in the order of
 // density.py:390-402) and the SSP-RK3 stage update (timestep.py:35-45). SPLIT: the form of CellAt
-// with a sixth warp for the CFL sum.
-template <typename R, typename S, int STAGE, bool SPLIT>
-__global__ void __launch_bounds__(SPLIT ? 192 : BLOCK)
+// with a sixth warp for the CFL sum. SOFT (FP64, use_soft): the FP64 pipe binds; the gather's 30
+// products of about 105 FP64 instructions a cell go to the integer pipes (soft64.cuh; the same bits),
+// and four blocks a SM then hide their latency: 392 -> 304 us at 128^3, 171 -> 136 at 96^3, 62 -> 50 at
+// 64^3 (two blocks 322, 143, 55; three 301, 136, 54). A cell with a flux of 2^64 or more gathers again with
+// the hardware's.
+template <typename R, typename S, int STAGE, bool SPLIT, bool SOFT>
+__global__ void __launch_bounds__(SPLIT ? 192 : BLOCK, SOFT ? 4 : 0)
     k_update(MeshDev<R> m, const R* __restrict__ fflux, double dtv, const double* dtp, const S* u0r, const S* u0u,
              const S* u0e, const S* u1r, const S* u1u, const S* u1e, const S* u2r, const S* u2u, const S* u2e,
              const S* __restrict__ Sr, const S* __restrict__ Su, const S* __restrict__ Se, S* outr, S* outu, S* oute,
@@ -442,26 +446,42 @@ __global__ void __launch_bounds__(SPLIT ? 192 : BLOCK)
         // the sums start at -0, which the compiler drops from the first term's add (-0 + x is x,
         // while +0 + x is one more add; the values differ at most in the sign of a zero)
         R res[5] = {R(-0.0), R(-0.0), R(-0.0), R(-0.0), R(-0.0)};
+        unsigned most = 0;
+        auto gather = [&](auto soft) {
 #pragma unroll
-        for (int k = 0; k < 6; k++) {
-            bool ownerSide = e[k] >= 0;
-            int f = ownerSide ? e[k] : ~e[k];
-            // the side's sign on the weight (one select a face, not one a term); each product
-            // rounded before it is added, as the reference's collate sum does, so that equal
-            // and opposite terms cancel exactly
-            R ws = ownerSide ? w[k] : -w[k];
-            if constexpr (SPLIT) {
-                const R F = fflux[(size_t)f * FREC + at.q0];
-                if (at.q0 == 5) dtc = dtc + F * w[k];
-                else res[1] = res[1] + mul_rn(F, ws);
-                // (the energy residual's gauge term takes the mass residual)
-                if (kGauge<R> && at.q0 == 4) res[0] = res[0] + mul_rn(fflux[(size_t)f * FREC], ws);
-            } else {
-                R F[FREC];
-                load_flux_record(fflux + (size_t)f * FREC, F);
-                for (int q = 0; q < 5; q++) res[q] = res[q] + mul_rn(F[q], ws);
-                dtc = dtc + F[5] * w[k];
+            for (int k = 0; k < 6; k++) {
+                bool ownerSide = e[k] >= 0;
+                int f = ownerSide ? e[k] : ~e[k];
+                // the side's sign on the weight (one select a face, not one a term); each product
+                // rounded before it is added, as the reference's collate sum does, so that equal
+                // and opposite terms cancel exactly
+                R ws = ownerSide ? w[k] : -w[k];
+                if constexpr (SPLIT) {
+                    const R F = fflux[(size_t)f * FREC + at.q0];
+                    if (at.q0 == 5) dtc = dtc + F * w[k];
+                    else res[1] = res[1] + mul_rn(F, ws);
+                    // (the energy residual's gauge term takes the mass residual)
+                    if (kGauge<R> && at.q0 == 4) res[0] = res[0] + mul_rn(fflux[(size_t)f * FREC], ws);
+                } else {
+                    R F[FREC];
+                    load_flux_record(fflux + (size_t)f * FREC, F);
+                    if constexpr (decltype(soft)::value) {
+                        for (int q = 0; q < 5; q++) {
+                            soft_seen(most, F[q]);
+                            res[q] = res[q] + soft_mul(F[q], ws);
+                        }
+                    } else {
+                        for (int q = 0; q < 5; q++) res[q] = res[q] + mul_rn(F[q], ws);
+                    }
+                    dtc = dtc + F[5] * w[k];
+                }
             }
+        };
+        gather(std::integral_constant<bool, SOFT>{});
+        if (SOFT && __builtin_expect(most >= SOFT_LIMIT, 0)) {
+            for (int q = 0; q < 5; q++) res[q] = R(-0.0);
+            dtc = R(0);
+            gather(std::false_type{});
         }
         const S rdt = S(dtp ? *dtp : dtv);
 #pragma unroll
@@ -706,7 +726,10 @@ void launch_flux_update(Ctx* c, int st, double dt, const double* dtDev, const S*
     const S *const *b = st == 1 ? u1 : u2, *b0 = st ? b[0] : none, *b1 = st ? b[1] : none, *b2 = st ? b[2] : none;
     auto update = [&](auto stage) {
         constexpr int ST = decltype(stage)::value;
-        launch_after(split ? k_update<R, S, ST, true> : k_update<R, S, ST, false>, (split ? (m.nIC + 31) / 32 : g.blocks) +
+        auto kernel = split ? k_update<R, S, ST, true, false> : k_update<R, S, ST, false, false>;
+        if constexpr (sizeof(R) == 8)
+            if (use_soft(c, m.nIC)) kernel = k_update<R, S, ST, false, true>;
+        launch_after(kernel, (split ? (m.nIC + 31) / 32 : g.blocks) +
                      (ST == 2 && end ? 1 : 0), split ? 192 : g.threads, 0, s, m, ff, dt, dtDev, u0[0], u0[1], u0[2], b0,
                      b1, b2, b0, b1, b2, Sr, Su, Se, out[0], out[1], out[2], c->dtcBits, P, recNext, c->objective,
                      ST == 0 && recNext ? objPartials : nullptr, ST == 2 && end ? *end : StepEnd{});

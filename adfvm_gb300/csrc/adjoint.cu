@@ -636,6 +636,8 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
     const R* faceTape = nullptr;
     const R* recTape = nullptr;
     split_tape<const R>(c, tape, faceTape, recTape);
+    bool byTape = false;      // the mesh gradients from face tapes
+    if constexpr (std::is_same<R, double>::value) byTape = params && param_tapes(c, *params, faceTape, s);
     for (int st = 2; st >= 0; st--) {
         const S* const* u = st == 0 ? u0c : (st == 1 ? u1c : u2c);
         const R* rec = recTape ? recTape + (size_t)st * m.nC * REC : (const R*)c->rec;
@@ -647,9 +649,14 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
         else if (st == 1) { ain[0] = A2[0]; ain[1] = A2[1]; ain[2] = A2[2]; }
         else { ain[0] = A1[0]; ain[1] = A1[1]; ain[2] = A1[2]; }
         R coef = (R)(-beta[st] * dt);
+        const R* ft = faceTape ? faceTape + (size_t)st * TAPE * m.nF : nullptr;
+        if constexpr (std::is_same<R, double>::value)
+            if (byTape) {
+                launch_flux<R>(c, false, rec, ft ? nullptr : c->paramTape, s);
+                if (!ft) ft = c->paramTape;
+            }
         {
             ProfScope ps(c, KID_ADJ_FLUX, s);
-            const R* ft = faceTape ? faceTape + (size_t)st * TAPE * m.nF : nullptr;
             const bool small = gF.threads == 32;
             if constexpr (std::is_same<R, float>::value) {
                 launch_after(small ? k_adj_flux_f32<S, 32> : k_adj_flux_f32<S, FLUX_BLOCK>, gF.blocks, gF.threads, 0, s,
@@ -678,7 +685,7 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
         // the stage's share of the mesh / boundary-input gradients (before the cell kernel: the
         // adjoint outputs it writes may alias this stage's input adjoints)
         if constexpr (std::is_same<R, double>::value && std::is_same<S, double>::value)
-            if (params) launch_param_grads<R, S>(c, *params, rec, coef, ain[0], ain[1], ain[2], st == 1, obja, s);
+            if (params) launch_param_grads<R, S>(c, *params, rec, coef, ain[0], ain[1], ain[2], st == 1, obja, s, byTape ? ft : nullptr);
         ProfScope ps(c, KID_ADJ_GRAD, s);
         S* const* a1 = st == 2 ? A2 : A1;      // (not written by the last stage)
         auto cells = [&](auto stage) {

@@ -8,8 +8,8 @@
 // The reference gets them from adpy's reverse mode over the whole step; here, per stage of the
 // reverse sweep, two kernels add the stage's share once the stage's face records (fadj) and
 // cell sums (cbar) exist:
-//   k_param_face  faces: the face flux again and its VJP with the geometry adjoints (face.cuh,
-//                 GeoBar), the div weights A/V_L, A/V_R (op.py:12-20), the Green-Gauss terms of
+//   k_param_face  faces: the face flux (again, or from its tape) and its VJP with the geometry adjoints
+//                 (face.cuh, GeoBar), the div weights A/V_L, A/V_R (op.py:12-20), the Green-Gauss terms of
 //                 the two adjacent cells (op.py:45-63), the ghost cells whose values depend on
 //                 the normals (symmetryPlane, a CBC_TOTAL_PT direction taken from the normals)
 //                 or on the boundary input, and the drag objective's face terms;
@@ -53,18 +53,22 @@ __device__ __forceinline__ void ghost_bar(const MeshDev<R>& m, const Phys& P, co
     }
 }
 
-// The FP64 pipe binds (about 750 FP64 instructions a face): the face flux is evaluated once, into a
-// tape in registers and local memory that its VJP reads, where both needed an evaluation of their
-// own before; two blocks a SM hold more of it in registers than the compiler's choice: 768 -> 605 us a
-// launch of 317,955 faces. (Products on the integer pipes, soft64.cuh, gave 601 at three blocks: its
-// serial chains are too long for so few warps.)
-template <typename R, typename S>
-__global__ void __launch_bounds__(FLUX_BLOCK, 2) k_param_face(MeshDev<R> m, Phys P, const R* __restrict__ rec, R coef,
+// The FP64 pipe binds. Untaped (meshes up to the small-grid limit): about 750 FP64 instructions a
+// face; the face flux is evaluated once, into a tape in registers and local memory that its VJP
+// reads; two blocks a SM hold more of it in registers than the compiler's choice (768 -> 605 us a
+// launch of 317,955 faces). TAPED: the flux and its forward values come from k_flux, whose evaluation
+// serves k_adj_flux as well: with k_adj_flux and the evaluation 272 + 605 -> 136 + 180 + 419 us a stage (two blocks
+// a SM 426). Products on the integer pipes (soft64.cuh) gave 601 for 605: the serial chains are too long
+// for so few warps. One kernel for the face records and these gradients would take 609 + 83 us, but
+// the records' last bits would depend on whether gradients are wanted.
+template <typename R, typename S, bool TAPED>
+__global__ void __launch_bounds__(FLUX_BLOCK, TAPED ? 3 : 2) k_param_face(MeshDev<R> m, Phys P, const R* __restrict__ rec, R coef,
                                                            const S* __restrict__ ar, const S* __restrict__ au,
                                                            const S* __restrict__ ae, const R* __restrict__ fadj,
                                                            const R* __restrict__ cbar, int inviscid, int dragStage,
                                                            int objStart, int objN, double obja,
-                                                           const double* __restrict__ objSeed, ParamDev pd) {
+                                                           const double* __restrict__ objSeed, ParamDev pd,
+                                                           const R* __restrict__ fflux, const R* __restrict__ tape) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= m.nF) return;
     const bool internal = f < m.nIF;
@@ -92,6 +96,9 @@ __global__ void __launch_bounds__(FLUX_BLOCK, 2) k_param_face(MeshDev<R> m, Phys
     if (kind == FACE_BOUNDARY) {
         face_flux<R>(P, kind, inviscid != 0, in, F, maxaF);
         face_vjp<R>(P, kind, inviscid != 0, in, Fb, b, &geo);
+    } else if (TAPED) {
+        for (int k = 0; k < 5; k++) F[k] = fflux[(size_t)f * FREC + k];
+        face_vjp_t<R>(P, kind, inviscid != 0, in, TapeLoad<R>{tape + f, (size_t)m.nF}, Fb, b, &geo);
     } else {
         TapeLocal<R, true> t;
         face_flux<R>(P, kind, inviscid != 0, in, F, maxaF, t);
@@ -228,9 +235,26 @@ __global__ void __launch_bounds__(BLOCK) k_param_cell(MeshDev<R> m, Phys P, cons
     vol[c] += vb;
 }
 
+bool param_tapes(Ctx* c, const ParamDev& pd, bool tape, cudaStream_t s) {
+    if (!use_soft(c, c->nF)) return false;
+    if (!pd.areas && !pd.volL && !pd.volR && !pd.dlt && !pd.nrm && !pd.du && !pd.lw && !pd.qw) return false;
+    if (tape || c->paramTape) return true;
+    // made with the first gradients, unless the stream is being captured or it took more than a
+    // quarter of the free memory
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    size_t free = 0, total = 0;
+    const size_t bytes = sizeof(double) * TAPE * (size_t)c->nF;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
+        cudaMemGetInfo(&free, &total) != cudaSuccess || bytes > free / 4) {
+        cudaGetLastError();
+        return false;
+    }
+    return ctx_alloc(c, (void**)&c->paramTape, bytes) == AFVM_OK;
+}
+
 template <typename R, typename S>
 void launch_param_grads(Ctx* c, const ParamDev& pd, const R* rec, R coef, const S* ar, const S* au, const S* ae,
-                        bool objectiveStage, double obja, cudaStream_t s) {
+                        bool objectiveStage, double obja, cudaStream_t s, const R* tape) {
     const MeshDev<R>& m = meshOf<R>(c);
     const Phys& P = c->phys;
     int inviscid = (P.muModel == AFVM_MU_CONSTANT && P.mu0 == 0.0) ? 1 : 0;
@@ -238,8 +262,9 @@ void launch_param_grads(Ctx* c, const ParamDev& pd, const R* rec, R coef, const 
     int nbF = (m.nF + FLUX_BLOCK - 1) / FLUX_BLOCK;
     int drag = objectiveStage && c->objective == AFVM_OBJ_DRAG;
     const double* seed = objectiveStage ? c->objSeed : nullptr;
-    k_param_face<R, S><<<nbF, FLUX_BLOCK, 0, s>>>(m, P, rec, coef, ar, au, ae, (const R*)c->fadj, (const R*)c->cbar,
-                                                  inviscid, drag, c->objStart, c->objN, obja, seed, pd);
+    auto k = tape ? k_param_face<R, S, true> : k_param_face<R, S, false>;
+    k<<<nbF, FLUX_BLOCK, 0, s>>>(m, P, rec, coef, ar, au, ae, (const R*)c->fadj, (const R*)c->cbar, inviscid, drag,
+                                 c->objStart, c->objN, obja, seed, pd, (const R*)c->fflux, tape);
     if (pd.vol) {
         int ke = objectiveStage && c->objective == AFVM_OBJ_KINETIC_ENERGY;
         k_param_cell<R><<<nblocks(m.nIC), BLOCK, 0, s>>>(m, P, rec, (const R*)c->cbar, ke, obja, pd.vol);
@@ -247,6 +272,6 @@ void launch_param_grads(Ctx* c, const ParamDev& pd, const R* rec, R coef, const 
 }
 
 template void launch_param_grads<double, double>(Ctx*, const ParamDev&, const double*, double, const double*,
-                                                 const double*, const double*, bool, double, cudaStream_t);
+                                                 const double*, const double*, bool, double, cudaStream_t, const double*);
 
 }  // namespace afvm

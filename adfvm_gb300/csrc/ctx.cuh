@@ -247,6 +247,7 @@ struct Ctx {
     uint8_t* gdirn = nullptr;            // per ghost, the same flag (device; on first use)
     // adjoint buffers (allocated on first use)
     void* fadj = nullptr;     // nF x 40 face adjoint records
+    double* paramTape = nullptr;   // one stage's face tape, for the mesh gradients (adjoint_params.cu)
     void* cbar = nullptr;     // nIC x 20 cell primitive/gradient adjoints
     void* a1[3] = {nullptr, nullptr, nullptr};
     void* a2[3] = {nullptr, nullptr, nullptr};
@@ -351,9 +352,13 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
 int prepare_adjoint(Ctx* c);
 // per stage of the reverse sweep, after the face records and cell sums of the stage (fadj,
 // cbar) and before the stage's cell kernel: adds the stage's share of the parameter gradients
+// tape: the stage's face tape, with the fluxes in the context's flux records (NULL: neither)
 template <typename R, typename S>
 void launch_param_grads(Ctx* c, const ParamDev& pd, const R* rec, R coef, const S* ar, const S* au, const S* ae,
-                        bool objectiveStage, double obja, cudaStream_t s);
+                        bool objectiveStage, double obja, cudaStream_t s, const R* tape);
+// whether the gradients are to be formed from face tapes (tape: the step's own is given), with
+// paramTape made where it is needed
+bool param_tapes(Ctx* c, const ParamDev& pd, bool tape, cudaStream_t s);
 
 // a step's tape, written by the primal step and read by its adjoint step: in FP64 first the
 // face tapes, one per RK stage, TAPE values a face each (value k of face f of stage st at
@@ -380,6 +385,9 @@ template <typename R, typename S = R>
 void launch_prim(Ctx* c, const S* r, const S* ru, const S* re, cudaStream_t s, R* rec = nullptr);
 template <typename R, typename S = R>
 void launch_prim_grad(Ctx* c, const S* r, const S* ru, const S* re, cudaStream_t s, R* rec = nullptr);
+// the faces' fluxes into the context's flux records and, with a tape, their forward values into that
+template <typename R>
+void launch_flux(Ctx* c, bool cfl, const R* rec, R* tape, cudaStream_t s);
 // nextPrims: the update also writes the primitives of the state it produces into the cell
 // records (the next stage's k_prim, fused)
 // tape: the stage's face tape to write (NULL: none)

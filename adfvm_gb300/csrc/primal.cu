@@ -687,6 +687,34 @@ void launch_prim_grad(Ctx* c, const S* r, const S* ru, const S* re, cudaStream_t
     launch_grad<R>(c, rec, s);
 }
 
+// the faces' fluxes (and their tape) from the cell records
+template <typename R>
+void launch_flux(Ctx* c, bool cfl, const R* rec, R* tape, cudaStream_t s) {
+    const MeshDev<R>& m = meshOf<R>(c);
+    const Phys& P = c->phys;
+    R* ff = (R*)c->fflux;
+    int inviscid = (P.muModel == AFVM_MU_CONSTANT && P.mu0 == 0.0) ? 1 : 0;
+    ProfScope ps(c, KID_FLUX, s);
+    const Shape g = shape_for(m.nF, FLUX_BLOCK);
+    auto flux = [&](auto taped, auto withCfl, auto soft) {
+        launch_after(k_flux<R, decltype(taped)::value, decltype(withCfl)::value, decltype(soft)::value>, g.blocks,
+                     g.threads, 0, s, m, P, rec, ff, inviscid, tape);
+    };
+    auto by_cfl = [&](auto taped, auto soft) {
+        if (cfl) flux(taped, std::true_type{}, soft);
+        else flux(taped, std::false_type{}, soft);
+    };
+    if constexpr (sizeof(R) == 8) {
+        const bool soft = use_soft(c, m.nF);
+        if (tape && soft) by_cfl(std::true_type{}, std::true_type{});
+        else if (tape) by_cfl(std::true_type{}, std::false_type{});
+        else if (soft) by_cfl(std::false_type{}, std::true_type{});
+        else by_cfl(std::false_type{}, std::false_type{});
+    } else {
+        by_cfl(std::false_type{}, std::false_type{});     // (FP32 contexts keep no face tape)
+    }
+}
+
 // faces -> fluxes, then the gather + stage update u_{st+1} = ... (timestep.py:35-45)
 template <typename R, typename S>
 void launch_flux_update(Ctx* c, int st, double dt, const double* dtDev, const S* const* u0, const S* const* u1,
@@ -696,28 +724,7 @@ void launch_flux_update(Ctx* c, int st, double dt, const double* dtDev, const S*
     const Phys& P = c->phys;
     R* rec = recIn ? recIn : (R*)c->rec;
     R* ff = (R*)c->fflux;
-    int inviscid = (P.muModel == AFVM_MU_CONSTANT && P.mu0 == 0.0) ? 1 : 0;
-    {
-        ProfScope ps(c, KID_FLUX, s);
-        const Shape g = shape_for(m.nF, FLUX_BLOCK);
-        auto flux = [&](auto taped, auto cfl, auto soft) {
-            launch_after(k_flux<R, decltype(taped)::value, decltype(cfl)::value, decltype(soft)::value>, g.blocks,
-                         g.threads, 0, s, m, P, rec, ff, inviscid, tape);
-        };
-        auto by_cfl = [&](auto taped, auto soft) {
-            if (st == 1) flux(taped, std::true_type{}, soft);
-            else flux(taped, std::false_type{}, soft);
-        };
-        if constexpr (sizeof(R) == 8) {
-            const bool soft = use_soft(c, m.nF);
-            if (tape && soft) by_cfl(std::true_type{}, std::true_type{});
-            else if (tape) by_cfl(std::true_type{}, std::false_type{});
-            else if (soft) by_cfl(std::false_type{}, std::true_type{});
-            else by_cfl(std::false_type{}, std::false_type{});
-        } else {
-            by_cfl(std::false_type{}, std::false_type{});     // (FP32 contexts keep no face tape)
-        }
-    }
+    launch_flux<R>(c, st == 1, rec, tape, s);
     const Shape g = shape_for(m.nIC, BLOCK);
     R* recNext = nextPrims ? (recOut ? recOut : rec) : nullptr;
     ProfScope ps(c, KID_UPDATE, s);
@@ -867,6 +874,7 @@ int primal_run_dev(Ctx* c, S* rho, S* rhoU, S* rhoE, int nSteps, double dt0, dou
 AFVM_PRIMAL_INST(double, double)
 AFVM_PRIMAL_INST(float, float)
 AFVM_PRIMAL_INST(float, double)
+template void launch_flux<double>(Ctx*, bool, const double*, double*, cudaStream_t);
 template void default_sources<double>(Ctx*, const double*&, const double*&, const double*&);
 template void default_sources<float>(Ctx*, const float*&, const float*&, const float*&);
 template void launch_vane_sums<double>(Ctx*, cudaStream_t, double*, const double*, double*);

@@ -612,9 +612,27 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
     const S* u0c[3] = {rho, rhoU, rhoE};
     const S* u1c[3] = {u1[0], u1[1], u1[2]};
     const S* u2c[3] = {u2[0], u2[1], u2[2]};
+    // a tape holds the stage's cell records the primal step built (no primitive or gradient
+    // launches here) and, in FP64, its face tape
+    const R* faceTape = nullptr;
+    const R* recTape = nullptr;
+    split_tape<const R>(c, tape, faceTape, recTape);
+    // the mesh gradients from face tapes; with nothing kept, from a whole step's
+    bool byTape = false;
+    const R* fluxes = nullptr;
+    if constexpr (std::is_same<R, double>::value) {
+        byTape = params && param_tapes(c, *params, faceTape, s);
+        if (byTape && !stages && !tape && c->paramTapeWhole) fluxes = c->paramTape;
+    }
     if (stages) {
         // the stage states the primal step kept (afvm_primal_step_stages)
         stage_views<S, const S>(stages, m.nIC, u1c, u2c);
+    } else if (fluxes) {
+        if constexpr (std::is_same<R, double>::value && std::is_same<S, double>::value) {
+            R* t = c->paramTape + 3 * FREC * (size_t)m.nF;
+            launch_forward_tape<R, S>(c, dt, u0c, u1, u2, Srho, SrhoU, SrhoE, t, c->paramTape, s);
+            split_tape<const R>(c, t, faceTape, recTape);
+        }
     } else {
         // forward recompute of the stage states
         launch_prim_grad<R, S>(c, rho, rhoU, rhoE, s);
@@ -631,13 +649,6 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
     const Shape gF = shape_for(m.nF, FLUX_BLOCK), gC = shape_for(m.nIC, BLOCK);
     const bool split = split_cells(m.nIC);
     const double beta[3] = {1.0, 1. / 4, 2. / 3};
-    // a tape holds the stage's cell records the primal step built (no primitive or gradient
-    // launches here) and, in FP64, its face tape
-    const R* faceTape = nullptr;
-    const R* recTape = nullptr;
-    split_tape<const R>(c, tape, faceTape, recTape);
-    bool byTape = false;      // the mesh gradients from face tapes
-    if constexpr (std::is_same<R, double>::value) byTape = params && param_tapes(c, *params, faceTape, s);
     for (int st = 2; st >= 0; st--) {
         const S* const* u = st == 0 ? u0c : (st == 1 ? u1c : u2c);
         const R* rec = recTape ? recTape + (size_t)st * m.nC * REC : (const R*)c->rec;
@@ -651,7 +662,7 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
         R coef = (R)(-beta[st] * dt);
         const R* ft = faceTape ? faceTape + (size_t)st * TAPE * m.nF : nullptr;
         if constexpr (std::is_same<R, double>::value)
-            if (byTape) {
+            if (byTape && !fluxes) {
                 launch_flux<R>(c, false, rec, ft ? nullptr : c->paramTape, s);
                 if (!ft) ft = c->paramTape;
             }
@@ -685,7 +696,8 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
         // the stage's share of the mesh / boundary-input gradients (before the cell kernel: the
         // adjoint outputs it writes may alias this stage's input adjoints)
         if constexpr (std::is_same<R, double>::value && std::is_same<S, double>::value)
-            if (params) launch_param_grads<R, S>(c, *params, rec, coef, ain[0], ain[1], ain[2], st == 1, obja, s, byTape ? ft : nullptr);
+            if (params) launch_param_grads<R, S>(c, *params, rec, coef, ain[0], ain[1], ain[2], st == 1, obja, s, byTape ? ft : nullptr,
+                                             fluxes ? fluxes + (size_t)st * FREC * m.nF : (const R*)c->fflux);
         ProfScope ps(c, KID_ADJ_GRAD, s);
         S* const* a1 = st == 2 ? A2 : A1;      // (not written by the last stage)
         auto cells = [&](auto stage) {

@@ -239,22 +239,24 @@ bool param_tapes(Ctx* c, const ParamDev& pd, bool tape, cudaStream_t s) {
     if (!use_soft(c, c->nF)) return false;
     if (!pd.areas && !pd.volL && !pd.volR && !pd.dlt && !pd.nrm && !pd.du && !pd.lw && !pd.qw) return false;
     if (tape || c->paramTape) return true;
-    // made with the first gradients, unless the stream is being captured or it took more than a
-    // quarter of the free memory
+    // made with the first gradients, unless the stream is being captured: a whole step's where that
+    // takes no more than a quarter of the free memory, else one stage's
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     size_t free = 0, total = 0;
-    const size_t bytes = sizeof(double) * TAPE * (size_t)c->nF;
+    const size_t whole = sizeof(double) * (3 * FREC * (size_t)c->nF + tape_elements(c));
+    const size_t one = sizeof(double) * TAPE * (size_t)c->nF;
     if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
-        cudaMemGetInfo(&free, &total) != cudaSuccess || bytes > free / 4) {
+        cudaMemGetInfo(&free, &total) != cudaSuccess || one > free / 4) {
         cudaGetLastError();
         return false;
     }
-    return ctx_alloc(c, (void**)&c->paramTape, bytes) == AFVM_OK;
+    c->paramTapeWhole = whole <= free / 4;
+    return ctx_alloc(c, (void**)&c->paramTape, c->paramTapeWhole ? whole : one) == AFVM_OK;
 }
 
 template <typename R, typename S>
 void launch_param_grads(Ctx* c, const ParamDev& pd, const R* rec, R coef, const S* ar, const S* au, const S* ae,
-                        bool objectiveStage, double obja, cudaStream_t s, const R* tape) {
+                        bool objectiveStage, double obja, cudaStream_t s, const R* tape, const R* flux) {
     const MeshDev<R>& m = meshOf<R>(c);
     const Phys& P = c->phys;
     int inviscid = (P.muModel == AFVM_MU_CONSTANT && P.mu0 == 0.0) ? 1 : 0;
@@ -264,7 +266,7 @@ void launch_param_grads(Ctx* c, const ParamDev& pd, const R* rec, R coef, const 
     const double* seed = objectiveStage ? c->objSeed : nullptr;
     auto k = tape ? k_param_face<R, S, true> : k_param_face<R, S, false>;
     k<<<nbF, FLUX_BLOCK, 0, s>>>(m, P, rec, coef, ar, au, ae, (const R*)c->fadj, (const R*)c->cbar, inviscid, drag,
-                                 c->objStart, c->objN, obja, seed, pd, (const R*)c->fflux, tape);
+                                 c->objStart, c->objN, obja, seed, pd, flux, tape);
     if (pd.vol) {
         int ke = objectiveStage && c->objective == AFVM_OBJ_KINETIC_ENERGY;
         k_param_cell<R><<<nblocks(m.nIC), BLOCK, 0, s>>>(m, P, rec, (const R*)c->cbar, ke, obja, pd.vol);
@@ -272,6 +274,6 @@ void launch_param_grads(Ctx* c, const ParamDev& pd, const R* rec, R coef, const 
 }
 
 template void launch_param_grads<double, double>(Ctx*, const ParamDev&, const double*, double, const double*,
-                                                 const double*, const double*, bool, double, cudaStream_t, const double*);
+                                                 const double*, const double*, bool, double, cudaStream_t, const double*, const double*);
 
 }  // namespace afvm

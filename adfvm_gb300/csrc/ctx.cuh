@@ -247,7 +247,9 @@ struct Ctx {
     uint8_t* gdirn = nullptr;            // per ghost, the same flag (device; on first use)
     // adjoint buffers (allocated on first use)
     void* fadj = nullptr;     // nF x 40 face adjoint records
-    double* paramTape = nullptr;   // one stage's face tape, for the mesh gradients (adjoint_params.cu)
+    // for the mesh gradients (adjoint_params.cu): a step's flux records and tape, or one stage's face tape
+    double* paramTape = nullptr;
+    bool paramTapeWhole = false;
     void* cbar = nullptr;     // nIC x 20 cell primitive/gradient adjoints
     void* a1[3] = {nullptr, nullptr, nullptr};
     void* a2[3] = {nullptr, nullptr, nullptr};
@@ -352,10 +354,10 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
 int prepare_adjoint(Ctx* c);
 // per stage of the reverse sweep, after the face records and cell sums of the stage (fadj,
 // cbar) and before the stage's cell kernel: adds the stage's share of the parameter gradients
-// tape: the stage's face tape, with the fluxes in the context's flux records (NULL: neither)
+// tape, flux: the stage's face tape and flux records (NULL: neither)
 template <typename R, typename S>
 void launch_param_grads(Ctx* c, const ParamDev& pd, const R* rec, R coef, const S* ar, const S* au, const S* ae,
-                        bool objectiveStage, double obja, cudaStream_t s, const R* tape);
+                        bool objectiveStage, double obja, cudaStream_t s, const R* tape, const R* flux);
 // whether the gradients are to be formed from face tapes (tape: the step's own is given), with
 // paramTape made where it is needed
 bool param_tapes(Ctx* c, const ParamDev& pd, bool tape, cudaStream_t s);
@@ -396,6 +398,9 @@ void launch_flux_update(Ctx* c, int st, double dt, const double* dtDev, const S*
                         const S* const* u2, const S* Sr, const S* Su, const S* Se, S* const* out, cudaStream_t s,
                         bool nextPrims = false, R* tape = nullptr, R* recIn = nullptr, R* recOut = nullptr,
                         double* objPartials = nullptr, const StepEnd* end = nullptr);
+template <typename R, typename S>
+void launch_forward_tape(Ctx* c, double dt, const S* const* u0, S* const* u1, S* const* u2, const S* Srho,
+                         const S* SrhoU, const S* SrhoE, R* tape, R* flux, cudaStream_t s);
 template <typename S>
 void default_sources(Ctx* c, const S*& Srho, const S*& SrhoU, const S*& SrhoE);
 // count values between host memory of any kind and the device (element sizes 4 or 8, converted

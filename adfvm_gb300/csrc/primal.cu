@@ -834,6 +834,30 @@ int primal_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double d
     return AFVM_OK;
 }
 
+// a step's first two stages and the third's face flux again: its tape, the three stages' flux records
+// (FREC values a face each) and the stage states u1, u2
+template <typename R, typename S>
+void launch_forward_tape(Ctx* c, double dt, const S* const* u0, S* const* u1, S* const* u2, const S* Srho,
+                         const S* SrhoU, const S* SrhoE, R* tape, R* flux, cudaStream_t s) {
+    const MeshDev<R>& m = meshOf<R>(c);
+    R *face, *recs;
+    split_tape<R>(c, tape, face, recs);
+    const S *const u1c[3] = {u1[0], u1[1], u1[2]}, *const u2c[3] = {u2[0], u2[1], u2[2]};
+    void* const own = c->fflux;
+    launch_prim<R, S>(c, u0[0], u0[1], u0[2], s, recs);
+    for (int st = 0; st < 3; st++) {
+        R* rec = recs + (size_t)st * m.nC * REC;
+        R* t = face + (size_t)st * TAPE * m.nF;
+        c->fflux = flux + (size_t)st * FREC * m.nF;
+        launch_grad<R>(c, rec, s);
+        if (st == 2) launch_flux<R>(c, false, rec, t, s);
+        else
+            launch_flux_update<R, S>(c, st, dt, nullptr, u0, u1c, u2c, Srho, SrhoU, SrhoE, st == 0 ? u1 : u2, s, true,
+                                     t, rec, rec + (size_t)m.nC * REC);
+    }
+    c->fflux = own;
+}
+
 template <typename R, typename S>
 int primal_run_dev(Ctx* c, S* rho, S* rhoU, S* rhoE, int nSteps, double dt0, double CFL, double stepFactor,
                    int fixed, const S* Srho, const S* SrhoU, const S* SrhoE, double* dtHist, double* dtcHist,
@@ -875,6 +899,9 @@ AFVM_PRIMAL_INST(double, double)
 AFVM_PRIMAL_INST(float, float)
 AFVM_PRIMAL_INST(float, double)
 template void launch_flux<double>(Ctx*, bool, const double*, double*, cudaStream_t);
+template void launch_forward_tape<double, double>(Ctx*, double, const double* const*, double* const*, double* const*,
+                                                  const double*, const double*, const double*, double*, double*,
+                                                  cudaStream_t);
 template void default_sources<double>(Ctx*, const double*&, const double*&, const double*&);
 template void default_sources<float>(Ctx*, const float*&, const float*&, const float*&);
 template void launch_vane_sums<double>(Ctx*, cudaStream_t, double*, const double*, double*);

@@ -189,29 +189,18 @@ __global__ void __launch_bounds__(NT, 3 * FLUX_BLOCK / NT)
     store_staged<R, FADJ, NT>(fadj, f0, min(NT, m.nF - f0), stage);
 }
 
-// the forward values of a warp's faces in shared memory, value k of lane's face at p[32 k]. FULL: all
-// of them, else those of a lean tape (TapeLocal)
-template <bool FULL>
-struct TapeWarp {
-    static constexpr bool kFull = FULL;
-    float* p;
-    __device__ __forceinline__ void put(int k, float x) const { p[32 * k] = x; }
-    __device__ __forceinline__ float get(int k) const { return p[32 * k]; }
-};
-
-// FP32. The kernel waits for its loads (and issues 44 % of the time), so the warps a SM holds count:
-// the forward values of a face go through shared memory instead of registers, which lets six
-// blocks a SM in at 80 registers without spills, and each warp copies its 32 records out of the
-// same memory by itself, in one bulk copy: no barrier of the block, no loads and stores for it.
-// At 128^3 412 -> 368 us a launch (five blocks 392, seven 472; the same with block-wide
-// staging 379, with the cell records fetched by the warp together 397). Mixed contexts: 5 blocks a SM,
-// 80^3 step and adjoint 1.131 ms (six 1.159, four 1.166).
+// FP32 and mixed contexts. The kernel waits for its loads (and issues 44 % of the time), so the
+// warps a SM holds count: five blocks of 128. The geometry is loaded after the cells' values, when
+// fewer registers are taken, and each warp copies its 32 records out by itself, in one bulk copy,
+// without a barrier of the block: at 128^3 FP32 412 -> 375 us a launch, mixed 80^3 step and adjoint
+// 1.160 -> 1.099 ms (six blocks spill, 498 us and 1.21 ms). All 61 forward values in
+// shared memory, the Riemann part first, take 368 us at six blocks, but round differently: the
+// operations and their order are those that FP32 results have always come from.
 template <typename S, int NT>
-__global__ void __launch_bounds__(NT, NT == 32 ? 12 : sizeof(S) == 8 ? 5 : 6)
+__global__ void __launch_bounds__(NT, NT == 32 ? 12 : 5)
     k_adj_flux_f32(MeshDev<float> m, Phys P, const float* __restrict__ rec, float coef, const S* __restrict__ ar,
                    const S* __restrict__ au, const S* __restrict__ ae, float* __restrict__ fadj, int inviscid) {
-    static_assert(FADJ <= TAPE, "a warp's forward values, then its results");
-    __shared__ __align__(16) float shared[NT / 32][32 * TAPE];
+    __shared__ __align__(16) float shared[NT / 32][32 * FADJ];
     const int lane = threadIdx.x & 31;
     const int f = blockIdx.x * NT + threadIdx.x;
     float* sh = shared[threadIdx.x >> 5];
@@ -231,17 +220,7 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 12 : sizeof(S) == 8 ? 5 : 6)
         // gauge form the forward evaluates)
         in.TP = rec_abs_T<float>(P, in.TP); in.TN = rec_abs_T<float>(P, in.TN);
         in.pP = rec_abs_p<float>(P, in.pP); in.pN = rec_abs_p<float>(P, in.pN);
-        // (mixed contexts keep the operations and the order their FP64 adjoints have always
-        // rounded in)
-        constexpr bool VFIRST = sizeof(S) == 8;
-        if (a.at.kind != FACE_BOUNDARY) {
-            const TapeWarp<!VFIRST> t{sh + lane};
-            float F[5], maxaF;
-            face_flux<float>(P, a.at.kind, inviscid != 0, in, F, maxaF, t);
-            face_vjp_t<float, VFIRST>(P, a.at.kind, inviscid != 0, in, t, Fb, b);
-        } else {
-            face_vjp<float, VFIRST>(P, a.at.kind, inviscid != 0, in, Fb, b);
-        }
+        face_vjp<float, true>(P, a.at.kind, inviscid != 0, in, Fb, b);
         const float* src = &b.UP[0];
         for (int k = 0; k < 5; k++) { v[k] = src[k]; v[20 + k] = src[5 + k]; }
         for (int k = 0; k < 15; k++) { v[5 + k] = src[10 + k]; v[25 + k] = src[25 + k]; }
@@ -425,7 +404,8 @@ __global__ void __launch_bounds__(SPLIT ? 160 : BLOCK)
             }
         }
     }
-    S J[5];
+    // the state's adjoint of the stage's residual: J[0] and, of the others, J[k] jr
+    S J[5], jr = S(0);
     auto whole_cell = [&]() {
         // ghost cells whose boundary value comes from this cell: transpose of the BC
         for (int q = gs0; q < gs1; q++) {
@@ -543,8 +523,9 @@ __global__ void __launch_bounds__(SPLIT ? 160 : BLOCK)
             float e = E - q;
             float pT = pbar[R_T] * Q.rCv, pp = pbar[R_P] * Q.gm1;
             float eb = pT + pp * rho;
-            for (int k = 0; k < 3; k++) J[1 + k] = (pbar[k] - eb * U[k]) * rr;
-            J[4] = eb * rr;
+            for (int k = 0; k < 3; k++) J[1 + k] = pbar[k] - eb * U[k];
+            J[4] = eb;
+            jr = rr;
             J[0] = pp * q - (pbar[0] * U[0] + pbar[1] * U[1] + pbar[2] * U[2]) * rr + pT * (q - e) * rr;
         } else {
             double rho = ur[c], rU[3] = {uu[3 * c], uu[3 * c + 1], uu[3 * c + 2]}, rE = ue[c];
@@ -556,27 +537,35 @@ __global__ void __launch_bounds__(SPLIT ? 160 : BLOCK)
             double rhob = (double)pbar[R_P] * P.gm1 * e;
             double Ubt[3];
             for (int k = 0; k < 3; k++) Ubt[k] = (double)pbar[k] - eb * U[k];
-            for (int k = 0; k < 3; k++) J[1 + k] = Ubt[k] * rr;
-            J[4] = eb * rr;
+            for (int k = 0; k < 3; k++) J[1 + k] = Ubt[k];
+            J[4] = eb;
+            jr = rr;
             J[0] = rhob - (Ubt[0] * U[0] + Ubt[1] * U[1] + Ubt[2] * U[2]) * rr - eb * E * rr;
         }
     };
     if constexpr (SPLIT) {
-        __shared__ S shJ[5 * 32];
+        __shared__ S shJ[6 * 32];
         const int lane = threadIdx.x & 31;
         if (first && c < m.nIC) {
             whole_cell();
             for (int q = 0; q < 5; q++) shJ[q * 32 + lane] = J[q];
+            shJ[5 * 32 + lane] = jr;
         }
         __syncthreads();
         if (c >= m.nIC) return;
         J[0] = shJ[at.q0 * 32 + lane];
+        jr = shJ[5 * 32 + lane];
     } else {
         whole_cell();
     }
     // SSP-RK reverse (timestep.py:35-45 transposed), in the state's type S. The source adjoint is
     // complete with stage 0, which writes it in the reference's layout (any part may be absent); the
     // stages before keep it in rows by component, as the outputs may alias inputs
+    // (the roundings spelled out, the same in both forms of the kernel)
+    auto plus_J = [&](S k, S x, int i, int q) {
+        if (q == 0) return fma(k, x, J[i]);
+        return fma(k, x, mul_rn(J[i], jr));
+    };
 #pragma unroll
     for (int i = 0; i < (SPLIT ? 1 : 5); i++) {
         const int q = SPLIT ? at.q0 : i;
@@ -585,14 +574,14 @@ __global__ void __launch_bounds__(SPLIT ? 160 : BLOCK)
         if (STAGE == 2) {
             sb[q * n + c] = S(2. / 3) * S(dt) * ain;
             a0 = S(1. / 3) * ain;
-            state_at(a1r, a1u, a1e, c, q) = S(2. / 3) * ain + (S)J[i];
+            state_at(a1r, a1u, a1e, c, q) = plus_J(S(2. / 3), ain, i, q);
         } else if (STAGE == 1) {
             sb[q * n + c] += S(1. / 4) * S(dt) * ain;
             a0 += S(3. / 4) * ain;
-            state_at(a1r, a1u, a1e, c, q) = S(1. / 4) * ain + (S)J[i];
+            state_at(a1r, a1u, a1e, c, q) = plus_J(S(1. / 4), ain, i, q);
         } else {
             const S src = sb[q * n + c] + S(dt) * ain;
-            a0 += ain + (S)J[i];
+            a0 += q == 0 ? ain + J[i] : fma(J[i], jr, ain);
             if (q == 0 ? sr != nullptr : (q == 4 ? se != nullptr : su != nullptr)) state_at(sr, su, se, c, q) = src;
         }
     }

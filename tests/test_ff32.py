@@ -1,8 +1,7 @@
-"""The FP32 contexts' pairs of floats (adfvm_gb300/csrc/ff32.cuh) against extended precision. A pair
-operation errs by at most 2^-44 of its operands; the pressure takes six of them and the temperature
-eight on values up to rhoE, so 2^-41 of (g-1) rhoE (of its temperature) and the rounding of the result;
-the objective's gradient a dozen relative ones, 2^-40, and the rounding. Values out of the pairs'
-range, infinities and NaN are refused with nothing written."""
+"""The FP32 contexts' pairs of floats (adfvm_gb300/csrc/ff32.cuh) against extended precision: what they
+take comes out correctly rounded (they give up, with nothing written, where their error could decide
+a rounding), which is nearly all of a flow's values; values out of their range, infinities and NaN
+are refused with nothing written."""
 import ctypes as C
 import os
 import subprocess
@@ -47,12 +46,12 @@ def test_primitives(lib, mach, gauge):
     s = _states(mach)
     out, ok = np.empty((len(s), 2), np.float32), np.empty(len(s), np.int32)
     lib.ff_prims(_p(np.array(AIR + gauge)), _p(s), len(s), _p(out), _p(ok))
-    assert ok.all()
+    ok = ok.astype(bool)
+    assert ok.mean() > 0.9
     d = s.astype(np.longdouble)
     e = d[:, 4] - (d[:, 1:4] ** 2).sum(1) * d[:, 5] / 2
-    for got, want, size in ((out[:, 0], AIR[0] * e - gauge[0], AIR[0] * d[:, 4]),
-                            (out[:, 1], e * d[:, 5] / np.longdouble(AIR[1]) - gauge[1], d[:, 4] * d[:, 5] / AIR[1])):
-        assert np.all(np.abs(got - want) <= 0.5 * np.spacing(np.abs(got)) + 2.0 ** -41 * size)
+    for got, want in ((out[:, 0], AIR[0] * e - gauge[0]), (out[:, 1], e * d[:, 5] / np.longdouble(AIR[1]) - gauge[1])):
+        assert np.array_equal(got[ok], want.astype(np.float32)[ok])
 
 
 def test_kinetic_gradient(lib):
@@ -64,13 +63,14 @@ def test_kinetic_gradient(lib):
     v[:, 5] = 10.0 ** rng.uniform(-9, 0, n)
     g, ok = np.zeros((n, 5), np.float32), np.empty(n, np.int32)
     lib.ff_kinetic(_p(np.array(AIR + gauge)), C.c_double(obja), _p(v), n, _p(g), _p(ok))
-    assert ok.all()
+    ok = ok.astype(bool)
+    assert ok.mean() > 0.99
     d = v.astype(np.longdouble)
     T, p, V = d[:, 3] + gauge[1], d[:, 4] + gauge[0], d[:, 5]
     Rg = np.longdouble(AIR[1] * AIR[0])
     q = (d[:, :3] ** 2).sum(1) / 2 * obja * V
     want = np.stack([obja * p / (Rg * T) * d[:, k] * V for k in range(3)] + [-q * p / (Rg * T * T), q / (Rg * T)], 1)
-    assert np.all(np.abs(g - want) <= (2.0 ** -24 + 2.0 ** -40) * np.abs(want))
+    assert np.array_equal(g[ok], want.astype(np.float32)[ok]) and not g[~ok].any()
 
 
 @pytest.mark.parametrize('column,value', [(0, 0.0), (0, -1.0), (0, np.inf), (0, np.nan), (0, 1e13), (1, np.inf),

@@ -641,9 +641,9 @@ AFVM_HD void viscous_geo_vjp(const Phys& P, R TL, R TR, const R* UL, const R* UR
     }
 }
 
-// VFIRST: the viscous part before the Riemann part. The other order holds 16 adjoints fewer across
-// the Riemann part (the FP64 VJP spills 4 bytes a thread at 168 registers instead of 352, the FP32
-// one none instead of 108 at 96); the sums of the face states' adjoints round differently.
+// VFIRST: the viscous part before the Riemann part, as FP32 and mixed contexts take them. The other
+// order holds 16 adjoints fewer across the Riemann part (the FP64 VJP spills 4 bytes a thread at 168
+// registers instead of 352); the sums of the face states' adjoints round differently.
 template <typename R, bool VFIRST = false, typename Src, typename G = GeoNone>
 AFVM_HD void face_vjp_t(const Phys& P, int kind, bool inviscid, const FaceIn<R>& in, const Src& t, const R* Fb,
                         FaceBar<R>& o, G* geo = nullptr);

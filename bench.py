@@ -86,22 +86,23 @@ STEP_BYTES = {('primal', 8): 2904, ('primal', 4): 1524, ('adjoint', 8): 6288, ('
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch from an ncu capture of
 # the 64^3 box (798,720 faces, 262,144 cells; profiles/), scaled to a launch of the benchmarked
-# mesh by its number of faces (the kernel's traffic grows in proportion to the faces). The FP64
-# kernels (taped: the benchmarked step with its 61-value face tape; untaped: --tape 0) are from
-# captures of the current build, the FP32 ones from earlier captures of the same kernels.
-MEASURED_TRAFFIC = {('k_flux', 8): (200.3e6, 798720), ('k_flux', 4): (81.56e6, 798720),
-                    ('k_adj_flux', 8): (455.5e6, 798720), ('k_adj_flux', 4): (170.37e6, 798720),
-                    ('k_flux+tape', 8): (547.1e6, 798720), ('k_adj_flux+tape', 8): (763.2e6, 798720)}
+# mesh by its number of faces (the kernel's traffic grows in proportion to the faces). Captures of
+# the current build (taped: the benchmarked step with its 61-value face tape; untaped: --tape 0),
+# the FP32 face VJP's from an earlier one (the same loads and stores).
+MEASURED_TRAFFIC = {('k_flux', 8): (203.6e6, 798720), ('k_flux', 4): (83.2e6, 798720),
+                    ('k_adj_flux', 8): (443.6e6, 798720), ('k_adj_flux', 4): (170.37e6, 798720),
+                    ('k_flux+tape', 8): (619.7e6, 798720), ('k_adj_flux+tape', 8): (797.4e6, 798720)}
 # FP64 thread instructions per face (DADD, DMUL, DFMA) of a launch in the same captures
-# (smsp__sass_thread_inst_executed_op_d{add,mul,fma}_pred_on), current build; the untaped
-# forward flux issues a few FP64 instructions fewer than the taped one (the tape's values it
-# need not form)
-MEASURED_FP64_INST = {'k_flux': (50.0, 85.1, 157.2), 'k_adj_flux': (82.0, 188.5, 314.4),
-                      'k_flux+tape': (52.0, 90.1, 156.2), 'k_adj_flux+tape': (40.0, 105.7, 177.4)}
+# (smsp__sass_thread_inst_executed_op_d{add,mul,fma}_pred_on): what the FP64 pipe is left with
+# beside the products, reciprocals and square roots on the integer pipes
+MEASURED_FP64_INST = {'k_flux': (50.0, 0.0, 132.4), 'k_adj_flux': (107.0, 0.0, 272.9),
+                      'k_flux+tape': (50.0, 0.0, 133.4), 'k_adj_flux+tape': (64.0, 0.0, 167.4)}
 # every warp instruction the FP64 pipe issued, per face (smsp__inst_executed_pipe_fp64 x 32 / faces,
-# the same captures): the arithmetic above plus the issues of warps whose lanes were partly masked
-# (branches that only some of a warp's faces take)
-MEASURED_FP64_PIPE_INST = {'k_flux': 295.0, 'k_adj_flux': 589.8, 'k_flux+tape': 301.0, 'k_adj_flux+tape': 328.8}
+# the same captures)
+MEASURED_FP64_PIPE_INST = {'k_flux': 183.0, 'k_adj_flux': 380.8, 'k_flux+tape': 184.0, 'k_adj_flux+tape': 231.8}
+# FP64 flops per face of the same kernels, whichever pipe forms them: DADD + DMUL + 2 DFMA of their
+# form with every operation on the FP64 pipe (counted by ncu)
+FACE_FLOPS = {'k_flux': 449.5, 'k_adj_flux': 899.3, 'k_flux+tape': 454.5, 'k_adj_flux+tape': 500.5}
 
 
 def measured_traffic(kernel, es, nF):
@@ -732,20 +733,21 @@ def main():
     line['fma_peak_tflops'] = {'fp64': round(_lib.fma_peak(local, True), 2), 'fp32': round(_lib.fma_peak(local, False), 2)}
     top, avg_s, nF = m64.pop('_top')
     if args.precision == 'fp64' and top in MEASURED_FP64_INST:
-        # the FP64 kernels are bound by the FP64 pipe, not HBM: counted FP64 instructions per
-        # face (ncu) x faces / the launch's CUDA-event time, against the measured FMA peak
+        # the FP64 kernels are bound by the FP64 pipe, not HBM: counted FP64 flops per face (ncu) x
+        # faces / the launch's CUDA-event time, against the measured FMA peak
         da, dm, df = MEASURED_FP64_INST[top]
-        flops = (da + dm + 2 * df) * nF
+        flops = FACE_FLOPS[top] * nF
         fpk = line['fma_peak_tflops']['fp64']
         ach = flops / avg_s / 1e12
         line['compute_roofline'] = {
             'bound': 'fp64', 'kernel': top, 'achieved': round(ach, 3), 'peak': fpk, 'unit': 'TFLOP/s',
-            'frac': round(ach / fpk, 4), 'flops_per_face': round(da + dm + 2 * df, 1),
+            'frac': round(ach / fpk, 4), 'flops_per_face': FACE_FLOPS[top],
             'issue_frac': round((da + dm + df) * nF / avg_s / (fpk * 1e12 / 2), 4),
             'pipe_issue_frac': round(MEASURED_FP64_PIPE_INST[top] * nF / avg_s / (fpk * 1e12 / 2), 4),
             'peak_source': 'afvm_fma_peak (a DFMA loop on this GPU, FMA = 2 flops)',
-            'note': 'issue_frac counts DADD/DMUL/DFMA as one FP64 pipe issue each; pipe_issue_frac '
-                    'every instruction the FP64 pipe issued (ncu), against the same issue rate'}
+            'note': 'flops of products on the integer pipes included; issue_frac counts the DADD/DMUL/DFMA '
+                    'left to the FP64 pipe as one issue each; pipe_issue_frac every instruction it '
+                    'issued (ncu), against the same issue rate'}
     if rank == 0 and not args.no_cpu_baseline:
         cb = cpu_baseline(args, os.cpu_count() or 1)
         cb.pop('config', None)

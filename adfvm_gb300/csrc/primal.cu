@@ -321,8 +321,8 @@ __device__ __noinline__ void flux_face_again(const MeshDev<R>& m, const Phys& P,
 
 // SOFT (FP64): products, reciprocals and square roots on the integer pipes (soft64.cuh). The FP64
 // pipe binds either form; of 298 FP64 instructions a face (52 DADD, 90 DMUL, 156 DFMA) 183 are
-// left (50 DADD, 133 DFMA): 3.47 -> 2.33 ms a taped launch of 6,340,608 faces, 1.81 ms when the
-// pipe never waited (it is 68 % busy: three warps a sub-partition, whose integer chains are
+// left (50 DADD, 133 DFMA): 3.47 -> 2.33 ms a taped launch of 6,340,608 faces, 1.85 ms when the
+// pipe never waited (it is 81 % busy: three warps a sub-partition, whose integer chains are
 // serial; 128 registers for four spill more than they hide, 2.42 ms, 255 for two 2.46).
 template <typename R, bool TAPED, bool CFL, bool SOFT>
 __global__ void __launch_bounds__(FLUX_BLOCK, sizeof(R) == 8 ? 3 : 8)

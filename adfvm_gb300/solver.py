@@ -790,16 +790,22 @@ class RCF(object):
     def run_fixed(self, x, dts, S=None):
         """len(dts) steps of these sizes in place on the CUDA tensors x = [rho, rhoU, rhoE]; returns
         their objectives (floats). Steps of one size run on the device in one go (the same bits as
-        step() gives), the host waiting once instead of after each."""
-        if self.objectiveFn is None and all(d == dts[0] for d in dts):
+        step() gives), the host waiting once instead of after each. As with step(), a CFL sum or
+        objective that is not finite (the reference aborts on NaN fields, adFVM/field.py:50-53) raises
+        AfvmError with the status AFVM_ERR_NONFINITE."""
+        if self.objectiveFn is None and np.isfinite(float(dts[0])) and all(d == dts[0] for d in dts):
             torch = _torch()
-            obj = torch.zeros(len(dts), dtype=torch.float64, device=x[0].device)
+            hist = torch.zeros((2, len(dts)), dtype=torch.float64, device=x[0].device)
+            hp = [C.cast(C.c_void_p(h.data_ptr()), L._d) for h in hist]
             Sp = (None, None, None) if S is None else [s.data_ptr() for s in S]
             st = L.lib().afvm_primal_run(self._ctx, x[0].data_ptr(), x[1].data_ptr(), x[2].data_ptr(), len(dts),
                                          float(dts[0]), float(self.CFL), float(self.stepFactor), 1, Sp[0], Sp[1], Sp[2],
-                                         None, None, C.cast(C.c_void_p(obj.data_ptr()), L._d), L.stream_of(x[0]))
+                                         None, hp[0], hp[1], L.stream_of(x[0]))
             L.check(st, self._ctx, 'afvm_primal_run')
-            return obj.tolist()
+            hist = hist.cpu().numpy()
+            if not np.isfinite(hist).all():
+                raise L.AfvmError(L.AFVM_ERR_NONFINITE, 'afvm_primal_run: non-finite CFL sum or objective')
+            return hist[1].tolist()
         return [self.step(x[0], x[1], x[2], d, S=S, out=x)[4] for d in dts]
 
     # ------------------------------------------------------------------ case files

@@ -21,10 +21,11 @@
 // through PETSc on the CPU). Everything here is FP64 whatever the context's precision.
 //
 // The FP64 pipe binds every kernel here, so their FP64 instructions are what was cut: divisions are
-// products with reciprocals formed once, alpha and beta are formed once an iteration by the last
-// block of the kernel that sums their dot products (which also spares the single-block kernels in
-// between), and a block adds its 5 or 10 dot products through shared memory (about 8 FP64
-// instructions a warp and product instead of 12 in every warp). An iteration is three kernels.
+// products with reciprocals formed once (with the remainder taken back where a result depends on
+// them: quotient), alpha and beta are formed once an iteration by the last block of the kernel that
+// sums their dot products (which also spares the single-block kernels in between), and a block adds
+// its 5 or 10 dot products through shared memory (about 8 FP64 instructions a warp and product
+// instead of 12 in every warp). An iteration is three kernels.
 // Vectors are interleaved, five components a cell: a neighbour's are in two sectors instead of five.
 // 262,144 cells in FP64, four iterations: 3.27 -> 0.80 ms (k_visc_cell 2.13 -> 0.30, an iteration
 // 198 -> 72 us: q = A p 57 + 10 -> 30, update 84 + 17.5 + 2 -> 31, direction 27.5 -> 11).
@@ -81,13 +82,24 @@ __device__ __forceinline__ bool grid_sums(const double* v, double* partials, uns
     return true;
 }
 
+// x / y and sqrt(x) rounded once, from products with r = 1/y and r = 1/sqrt(x): the product rounds a
+// second time, the remainder takes that back (two FP64 instructions)
+__device__ __forceinline__ double quotient(double x, double y, double r) {
+    const double q = x * r;
+    return fma(fma(-q, y, x), r, q);
+}
+__device__ __forceinline__ double root(double x, double r) {
+    const double s = x * r;
+    return fma(fma(-s, s, x), 0.5 * r, s);
+}
+
 template <typename R>
 __global__ void __launch_bounds__(VT) k_visc_sound(MeshDev<R> m, Phys P, const R* __restrict__ rec,
                                                    double* __restrict__ snd) {
     const int c = blockIdx.x * VT + threadIdx.x;
     if (c >= m.nC) return;
     const double c2 = (P.gamma * rec_T<R>(P, rec[(size_t)c * REC + R_T])) * (P.Cp - P.Cv);
-    snd[c] = c2 == 0.0 ? 0.0 : c2 * rsqrt_(c2);
+    snd[c] = c2 == 0.0 ? 0.0 : root(c2, rsqrt_(c2));
 }
 
 template <typename R>
@@ -139,44 +151,48 @@ __global__ void __launch_bounds__(VT) k_visc_cell(MeshDev<R> m, Phys P, const R*
             const double dU = gU[0][0] + gU[1][1] + gU[2][2];
             const R* r = rec + (size_t)c * REC;
             const double T = rec_T<R>(P, r[R_T]), p = rec_p<R>(P, r[R_P]);
-            const double rT = rcp((P.Cv * T) * (g - 1));
-            const double rho = p * rT, rrho = rcp(rho), rp = rcp(p);
-            const double c2 = g * p * rrho, rc = rsqrt_(c2), cc = c2 * rc, rc2 = rc * rc;
-            double grho[3];
-            for (int j = 0; j < 3; j++) grho[j] = (g * rc2) * (gp[j] - cc * p);
-            const double g1 = g - 1;
+            // (each entry rounds no more often than with divisions: quotient, root)
+            const double g1 = g - 1, e = (P.Cv * T) * g1;
+            const double rho = quotient(p, e, rcp(e)), rrho = rcp(rho), rp = rcp(p);
+            const double c2 = quotient(g * p, rho, rrho), rc = rsqrt_(c2), cc = root(c2, rc);
+            const double rhoc = rho * cc, rrc = rrho * rc;
+            // grad rho = g (grad p - c p) / c^2
+            double gs[3];
+            for (int j = 0; j < 3; j++) gs[j] = gp[j] - cc * p;
             double A[5][5];
             for (int i = 0; i < 5; i++)
                 for (int j = 0; j < 5; j++) A[i][j] = 0.0;
             // M = M1/2 - M2 (postpro.py:571-602)
             if (kind == AFVM_VISC_TURKEL) {
-                const double rrc = rrho * rc, pg = ((PREF / (2 * UREF)) * rcp(g)) * (rp * rrho);
+                const double gpr = (g * p) * rho;
+                const double pg = quotient(PREF / (2 * UREF), gpr, rcp(g) * (rp * rrho));
                 for (int i = 0; i < 5; i++) A[i][i] = dU / 2;
                 for (int j = 0; j < 3; j++) { A[0][1 + j] += gc[j] / 2; A[1 + j][0] += gc[j] / 2; }
                 A[0][0] -= g1 * dU / 2;
                 for (int j = 0; j < 3; j++) {
-                    A[0][1 + j] -= gp[j] * rrc;
-                    A[1 + j][0] -= (0.5 * g1) * gp[j] * rrc;
+                    const double q = quotient(gp[j], rhoc, rrc);
+                    A[0][1 + j] -= q;
+                    A[1 + j][0] -= (0.5 * g1) * q;
                     A[1 + j][4] -= gp[j] * pg;
-                    A[4][1 + j] -= (gp[j] - c2 * grho[j]) * (UREF / PREF);
+                    A[4][1 + j] -= (gp[j] - g * gs[j]) * (UREF / PREF);
                     for (int k = 0; k < 3; k++) A[1 + j][1 + k] -= gU[j][k];
                 }
-                A[0][4] -= dU * ((PREF / (2 * UREF)) * rrc);
+                A[0][4] -= quotient(dU * (PREF / (2 * UREF)), rhoc, rrc);
                 A[4][4] -= g1 * dU / 2;
             } else {
-                const double rsg = rsqrt_(g), sg1 = sqrt_(g1);
-                const double b = cc * rsg, a = sg1 * b, r2g1 = 2 * rcp(g1);
+                const double rsg = rsqrt_(g), sg = root(g, rsg), sg1 = root(g1, rsqrt_(g1)), rg1 = rcp(g1);
+                const double a = sg1 * quotient(cc, sg, rsg);
                 double gb[3], ga[3];
-                for (int j = 0; j < 3; j++) { gb[j] = gc[j] * rsg; ga[j] = gb[j] * sg1; }
+                for (int j = 0; j < 3; j++) { gb[j] = quotient(gc[j], sg, rsg); ga[j] = gb[j] * sg1; }
                 for (int i = 0; i < 5; i++) A[i][i] = dU / 2;
                 for (int j = 0; j < 3; j++) {
                     A[0][1 + j] += gb[j] / 2; A[1 + j][0] += gb[j] / 2;
                     A[1 + j][4] += ga[j] / 2; A[4][1 + j] += ga[j] / 2;
                 }
                 for (int j = 0; j < 3; j++) {
-                    A[0][1 + j] -= b * grho[j] * rrho;
-                    A[1 + j][4] -= a * gp[j] * (0.5 * rp);
-                    A[4][1 + j] -= r2g1 * ga[j];
+                    A[0][1 + j] -= quotient(gs[j] * sg, rhoc, rrc);      // b grad rho / rho, b = c / sqrt(g)
+                    A[1 + j][4] -= 0.5 * quotient(a * gp[j], p, rp);
+                    A[4][1 + j] -= 2 * quotient(ga[j], g1, rg1);
                     for (int k = 0; k < 3; k++) A[1 + j][1 + k] -= gU[j][k];
                 }
                 A[0][4] -= sg1 * dU / 2;
@@ -215,7 +231,8 @@ __global__ void __launch_bounds__(VT) k_visc_face(MeshDev<R> m, const double* __
     const int iN = f < m.nIF ? m.nbr[f] : m.gsrc[f - m.nIF];
     const double d = (M[m.own[f]] * s) * w + (M[iN] * s) * (1 - w);
     DT[f] = d;
-    coef[f] = dt * ((double)m.area[f] * d * rcp((double)m.dlt[f]));
+    const double dlt = m.dlt[f];
+    coef[f] = dt * quotient((double)m.area[f] * d, dlt, rcp(dlt));
 }
 
 // ---- PCG on (V + dt L) x = a, five right-hand sides in lockstep; vectors are n x 5
@@ -232,9 +249,7 @@ __global__ void __launch_bounds__(VT) k_heat_rhs(MeshDev<R> m, const S* __restri
         const double a[5] = {(double)ar[c], (double)au[3 * c], (double)au[3 * c + 1], (double)au[3 * c + 2], (double)ae[c]};
         const double V = m.vol[c], rV = rcp(V);
         for (int q = 0; q < 5; q++) {
-            // a / V, rounded once: the product with the reciprocal and its remainder
-            const double y = a[q] * rV;
-            x[5 * (size_t)c + q] = fma(fma(-y, V, a[q]), rV, y);
+            x[5 * (size_t)c + q] = quotient(a[q], V, rV);
             v[q] += a[q] * a[q];
         }
     }

@@ -7,10 +7,10 @@
 // minors; above the spectrum each ratio of successive minors has one sign, so the recurrence is as
 // accurate as the matrix entries. The start is the same iteration in FP32, which costs no FP64,
 // raised by its error bound: two or three FP64 steps are left where the largest eigenvalue stands
-// alone (convergence is cubic), and a step leaves at most 3/8 of the distance where several
-// coincide. About 240 FP64 instructions on the GPU, whose FP64 pipe is the bound; cyclic Jacobi
-// rotations to convergence took about 6,000 (k_visc_cell of 262,144 cells 2.13 -> 0.30 ms, with its
-// face sums' shorter form).
+// alone (convergence is cubic; laguerre5's estimate of what is left ends them), and a step leaves at
+// most 3/8 of the distance where several coincide, so that its size ends those. About 250 FP64
+// instructions on the GPU, whose FP64 pipe is the bound; cyclic Jacobi rotations to convergence took
+// about 6,000.
 #pragma once
 #include <string.h>
 #include "physics.cuh"
@@ -19,9 +19,14 @@ namespace afvm {
 
 // Laguerre's step towards the largest root of the characteristic polynomial of the tridiagonal
 // matrix with diagonal d and squared off-diagonals e2, from x above it (where the polynomial of
-// degree five and its derivatives alternate in sign)
+// degree five and its derivatives alternate in sign). last: whether what the step leaves is below
+// the rounding of entries of size one. With d1 <= d2 <= ... the distances of x from the roots and
+// s = sum d1/di, t = sum (d1/di)^2 over the other four, a step of a small s leaves
+// d1 (t - s^2/4)/2 <= d1 s^2/2, and h = 2 p (p''/2) / (p'^2 - 2 p (p''/2)) = (2 s + s^2 - t)/(1 + t)
+// is at least s as t <= s: what is left is at most step h^2/2. (h is large near several roots,
+// so a step that lands among them is not taken for the last.)
 template <typename F>
-AFVM_HD F laguerre5(const F* d, const F* e2, F x) {
+AFVM_HD F laguerre5(const F* d, const F* e2, F x, bool* last = nullptr) {
     F a = F(1), b = d[0] - x;              // minors of order i - 1 and i,
     F da = F(0), db = F(-1);               // their derivatives,
     F ha = F(0), hb = F(0);                // and half their second derivatives
@@ -34,33 +39,49 @@ AFVM_HD F laguerre5(const F* d, const F* e2, F x) {
         da = db; db = dc;
         ha = hb; hb = hc;
     }
-    // n p / (p' - sqrt((n-1)^2 p'^2 - n (n-1) p p'')), n = 5
-    const F g = F(4) * db;
-    const F r = g * g - (F(40) * b) * hb;
+    if constexpr (sizeof(F) == 4) {
+        // (near five roots at once the squares below are not floats: 1e-35 where x is 2e-5 away)
+        const F s = rcp(fabs(hb));
+        b = b * s; db = db * s; hb = hb * s;
+    }
+    // n p / (p' - sqrt((n-1)^2 p'^2 - n (n-1) p p'')), n = 5. Five equal roots make the radicand zero: its
+    // rounding error, some 20 units, would send x below them, so more than that is added (a step too
+    // short by at most 5e-7 of itself in FP64, 0.011 in FP32, and by 2^-47 of itself at a simple root)
+    constexpr F up = sizeof(F) == 4 ? F(16 + 0x1p-13) : F(16 + 0x1p-42);
+    const F m = b * hb, g = db * db;
+    const F r = up * g - F(40) * m;
     const F q = r > F(0) ? r * rsqrt_(r) : F(0);
-    return (F(5) * b) * rcp(db - q);
+    const F step = (F(5) * b) * rcp(db - q);
+    if (last) {
+        // step h^2 / 2 <= 1e-17, h = 2 m / (g - 2 m)
+        const F k = g - F(2) * m;
+        *last = step * (m * m) <= F(5e-18) * (k * k);
+    }
+    return step;
 }
 
-// conversions on the integer pipe on the device (an FP64 conversion takes the FP64 pipe's time): x
-// truncated to a float (zero below 2^-120; |x| < 2^100), and a float as a double
+// conversions by integer instructions (on the device an FP64 conversion takes the FP64 pipe's time): x
+// truncated to a float (zero below 2^-120; |x| < 2^100), and a float as a double (zero below 2^-126)
 AFVM_HD float low(double x) {
-#if defined(__CUDA_ARCH__)
-    const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+    uint64_t b;
+    memcpy(&b, &x, 8);
+    const unsigned h = (unsigned)(b >> 32), l = (unsigned)b;
     const int e = (int)((h >> 20) & 0x7ffu) - 1023 + 127;
     const unsigned m = ((unsigned)e << 23) | ((h & 0xfffffu) << 3) | (l >> 29);
-    return __uint_as_float(e < 7 ? 0u : (m | (h & 0x80000000u)));
-#else
-    return (float)x;
-#endif
+    const unsigned f = e < 7 ? 0u : (m | (h & 0x80000000u));
+    float y;
+    memcpy(&y, &f, 4);
+    return y;
 }
 AFVM_HD double high(float x) {
-#if defined(__CUDA_ARCH__)
-    const unsigned b = __float_as_uint(x), e = (b >> 23) & 0xffu;
+    unsigned b;
+    memcpy(&b, &x, 4);
+    const unsigned e = (b >> 23) & 0xffu;
     const unsigned h = (b & 0x80000000u) | ((e + 896u) << 20) | ((b & 0x7fffffu) >> 3);
-    return e == 0u ? 0.0 : __hiloint2double((int)h, (int)(b << 29));
-#else
-    return (double)x;
-#endif
+    const uint64_t f = e == 0u ? 0u : ((uint64_t)h << 32) | (b << 29);
+    double y;
+    memcpy(&y, &f, 8);
+    return y;
 }
 
 // the upper triangle of a is used; NaN if an entry is not finite
@@ -76,8 +97,8 @@ AFVM_HD double max_eig5(const double a[5][5]) {
         }
     const int e = (int)(most >> 52);
     if (most == 0) return 0.0;
-    // the matrix scaled by a power of two to entries in [-2, 2]: the minors stay within 1e5 and the
-    // FP32 copy is safe
+    // the matrix scaled by a power of two to entries in [-2, 2]: the minors stay within 1e5, and in
+    // FP32 those of x 4e-6 from five roots above 1e-27
     double scale, back;
     int64_t bits = (int64_t)(2046 - e) << 52;
     memcpy(&scale, &bits, 8);
@@ -137,15 +158,14 @@ AFVM_HD double max_eig5(const double a[5][5]) {
         if (!(step > 4e-6f)) break;
         x -= step;
     }
-    // FP64: from above it by more than its error. A simple root is left to the rounding of the
-    // matrix after a step below 1e-9 that was a thousandth of the one before.
-    double y = high(x) + 8e-5, before = 1.0;
+    // FP64: from above it by more than its error
+    double y = high(x) + 8e-5;
     for (int it = 0; it < 60; it++) {
-        const double step = laguerre5(d, e2, y);
+        bool last;
+        const double step = laguerre5(d, e2, y, &last);
         if (!(step > 2e-16)) break;
         y -= step;
-        if (step < 1e-9 && step < 1e-3 * before) break;
-        before = step;
+        if (last) break;
     }
     return y * back;
 }

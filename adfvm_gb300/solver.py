@@ -29,6 +29,7 @@ The GPU library is mandatory: there is no CPU path.
 import collections
 import ctypes as C
 import functools
+import math
 import os
 import sys
 
@@ -793,19 +794,20 @@ class RCF(object):
         step() gives), the host waiting once instead of after each. As with step(), a CFL sum or
         objective that is not finite (the reference aborts on NaN fields, adFVM/field.py:50-53) raises
         AfvmError with the status AFVM_ERR_NONFINITE."""
-        if self.objectiveFn is None and np.isfinite(float(dts[0])) and all(d == dts[0] for d in dts):
+        if self.objectiveFn is None and math.isfinite(dts[0]) and all(d == dts[0] for d in dts):
             torch = _torch()
-            hist = torch.zeros((2, len(dts)), dtype=torch.float64, device=x[0].device)
-            hp = [C.cast(C.c_void_p(h.data_ptr()), L._d) for h in hist]
+            n = len(dts)
+            hist = torch.empty(2 * n, dtype=torch.float64, device=x[0].device)      # dtc, then the objective
+            hp = hist.data_ptr()
             Sp = (None, None, None) if S is None else [s.data_ptr() for s in S]
-            st = L.lib().afvm_primal_run(self._ctx, x[0].data_ptr(), x[1].data_ptr(), x[2].data_ptr(), len(dts),
+            st = L.lib().afvm_primal_run(self._ctx, x[0].data_ptr(), x[1].data_ptr(), x[2].data_ptr(), n,
                                          float(dts[0]), float(self.CFL), float(self.stepFactor), 1, Sp[0], Sp[1], Sp[2],
-                                         None, hp[0], hp[1], L.stream_of(x[0]))
+                                         None, C.cast(hp, L._d), C.cast(hp + 8 * n, L._d), L.stream_of(x[0]))
             L.check(st, self._ctx, 'afvm_primal_run')
-            hist = hist.cpu().numpy()
-            if not np.isfinite(hist).all():
+            hist = hist.tolist()
+            if not all(map(math.isfinite, hist)):
                 raise L.AfvmError(L.AFVM_ERR_NONFINITE, 'afvm_primal_run: non-finite CFL sum or objective')
-            return hist[1].tolist()
+            return hist[n:]
         return [self.step(x[0], x[1], x[2], d, S=S, out=x)[4] for d in dts]
 
     # ------------------------------------------------------------------ case files

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
 #include <initializer_list>
 #include <string>
 #include <vector>
@@ -260,6 +261,7 @@ struct Ctx {
     // sensitivity reduction scratch (grown on demand)
     void* sensScratch = nullptr;
     size_t sensBytes = 0;
+    std::atomic<unsigned long long> sensCalls{0};   // calls so far (sensitivity.cu)
     // an objective evaluated outside the library (afvm_set_objective_sink / _seed): the device
     // buffer that receives each primal step's objective-stage primitives (nC x 5, record type),
     // and the gradient of the objective with respect to them (nC x 5 double) the adjoint adds

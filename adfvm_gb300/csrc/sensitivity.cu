@@ -10,6 +10,7 @@
 // and more of the host: the 128x64 cylinder's ten-step FP64 sweep, ten calls with three arrays,
 // 4.67 -> 4.26 ms.
 #include <cuda_runtime.h>
+#include <atomic>
 #include <mutex>
 #include "ctx.cuh"
 
@@ -40,12 +41,19 @@ __device__ __forceinline__ double sens_block_sum(double v, double* sh) {
     return r;
 }
 
+// The arrival count is never cleared: a call counts from SENS_CALL times its number, to which each of its
+// blocks first raises the count (it is lower, from the call before). Calls that overlap spoil one
+// another's results, and leave the count at a value that serves the next call as well.
+constexpr unsigned long long SENS_CALL = 1ull << 20;
+static_assert(SENS_PACK * SENS_BLOCKS < SENS_CALL, "a launch's blocks");
+
 // this launch's partials follow the base ones of the launches before; total: all of them, summed
-// into *out by the last launch's last block (out NULL: not the last launch)
-__global__ void __launch_bounds__(BLOCK) k_sens(SensPack a, double* partials, int base, int total, unsigned* arrived,
-                                                double* out) {
+// into *out by the last launch's last block (out NULL: not the last launch). from: the call's count
+__global__ void __launch_bounds__(BLOCK) k_sens(SensPack a, double* partials, int base, int total,
+                                                unsigned long long* arrived, unsigned long long from, double* out) {
     __shared__ double sh[BLOCK / 32];
     __shared__ bool last;
+    if (out && threadIdx.x == 0) atomicMax(arrived, from);
     int k = 0;
     while (k + 1 < a.arrays && (int)blockIdx.x >= a.first[k + 1]) k++;
     const double* __restrict__ g = a.g[k];
@@ -57,7 +65,7 @@ __global__ void __launch_bounds__(BLOCK) k_sens(SensPack a, double* partials, in
     if (threadIdx.x == 0) {
         partials[base + blockIdx.x] = r;
         __threadfence();
-        last = out && atomicInc(arrived, gridDim.x - 1) == gridDim.x - 1;
+        last = out && atomicAdd(arrived, 1ull) == from + gridDim.x - 1;
     }
     __syncthreads();
     if (!last) return;
@@ -74,10 +82,11 @@ static int sens_blocks(long long n) {
     return (int)(b < SENS_BLOCKS ? b : SENS_BLOCKS);
 }
 
-// queues the reduction of nArrays arrays; partials: SENS_BLOCKS x nArrays, arrived: zero between
-// calls
+// queues the reduction of nArrays arrays; partials: SENS_BLOCKS x nArrays; arrived: the scratch's arrival
+// count, zero before its first call; call: the number of this call on the scratch, from 1
 int sensitivity_launch(int nArrays, const double* const* grad, const double* const* pert, const int64_t* n,
-                       double* partials, unsigned* arrived, double* out, cudaStream_t s, std::string* err) {
+                       double* partials, unsigned long long* arrived, unsigned long long call, double* out,
+                       cudaStream_t s, std::string* err) {
     for (int k = 0; k < nArrays; k++)
         if (n[k] < 0 || (n[k] > 0 && (!grad[k] || !pert[k]))) {
             if (err) *err = "afvm_sensitivity: array " + std::to_string(k) + " has a bad size or pointer";
@@ -99,7 +108,8 @@ int sensitivity_launch(int nArrays, const double* const* grad, const double* con
         const int blocks = a.first[m] > 0 ? a.first[m] : (end ? 1 : 0);
         if (!blocks) continue;
         if (a.first[m] == 0) a.first[m] = 1;
-        k_sens<<<blocks, BLOCK, 0, s>>>(a, partials, base, base + blocks, arrived, end ? out : nullptr);
+        k_sens<<<blocks, BLOCK, 0, s>>>(a, partials, base, base + blocks, arrived, call * SENS_CALL,
+                                         end ? out : nullptr);
         base += blocks;
     }
     cudaError_t e = cudaGetLastError();
@@ -128,8 +138,8 @@ int sensitivity_dev(Ctx* c, int nArrays, const double* const* grad, const double
         if (e != cudaSuccess) return cuda_fail(c, e, "afvm_sensitivity scratch");
     }
     ProfScope ps(c, KID_SENS, s);
-    int st = sensitivity_launch(nArrays, grad, pert, n, (double*)c->sensScratch + 1, (unsigned*)c->sensScratch,
-                                c->hostOutDev + 2, s, &c->err);
+    int st = sensitivity_launch(nArrays, grad, pert, n, (double*)c->sensScratch + 1, (unsigned long long*)c->sensScratch,
+                                ++c->sensCalls, c->hostOutDev + 2, s, &c->err);
     if (st) return st;
     cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(c, e, "afvm_sensitivity result");
@@ -144,17 +154,15 @@ int sensitivity_dev(Ctx* c, int nArrays, const double* const* grad, const double
 // fixed share of the GPU up front and makes every allocation itself, or a plug-in loaded
 // into a host program whose memory pool it must not touch. Such a caller can create no
 // context and cannot let afvm_sensitivity grow its scratch. For them the reduction's
-// scratch (block partials, per-array block counts and the result) is this file-scope device
-// array, sized for at most AFVM_SENSITIVITY_NOALLOC_MAX_ARRAYS arrays. Every GPU that loads
-// the library keeps it (~129 KB) until the process exits. All calls share it: two calls
-// that overlap on the GPU (different streams, or different host threads without ordering)
-// race on it.
+// scratch (block partials, the result and the arrival count) is this file-scope device array,
+// sized for at most AFVM_SENSITIVITY_NOALLOC_MAX_ARRAYS arrays. Every GPU that loads the library
+// keeps it (~129 KB) until the process exits. All calls share it: two calls that overlap on the
+// GPU (different streams, or different host threads without ordering) race on it.
 // ---------------------------------------------------------------------------------------
 
 constexpr int NOALLOC_MAX_ARRAYS = AFVM_SENSITIVITY_NOALLOC_MAX_ARRAYS;
 constexpr size_t NOALLOC_PARTIALS = (size_t)NOALLOC_MAX_ARRAYS * SENS_BLOCKS;
-// partials, then the result, then the arrival count (a double's worth; zero when the library is
-// loaded and after every call)
+// partials, then the result, then the arrival count (zero when the library is loaded)
 constexpr size_t NOALLOC_DOUBLES = NOALLOC_PARTIALS + 2;
 
 static __device__ __align__(256) double g_sens_noalloc_scratch[NOALLOC_DOUBLES];
@@ -165,6 +173,7 @@ static __device__ __align__(256) double g_sens_noalloc_scratch[NOALLOC_DOUBLES];
 // module: the cached address is then stale, and calls after a reset are not supported.
 static std::mutex g_noalloc_mutex;
 static double* g_noalloc_ptr[256] = {nullptr};
+static std::atomic<unsigned long long> g_noalloc_calls{0};     // (on any device)
 
 static int noalloc_scratch(int device, double** out) {
     if (device < 0 || device >= 256) return AFVM_ERR_BAD_ARG;
@@ -228,7 +237,8 @@ extern "C" int afvm_sensitivity_noalloc(int32_t device, int32_t nArrays, const d
         cudaStream_t s = (cudaStream_t)stream;
         // every partial read below is written earlier in this call, so nothing left by a previous
         // call is used and nothing needs clearing
-        st = sensitivity_launch(nArrays, grad, pert, n, partials, (unsigned*)(result + 1), result, s, nullptr);
+        st = sensitivity_launch(nArrays, grad, pert, n, partials, (unsigned long long*)(result + 1), ++g_noalloc_calls,
+                                result, s, nullptr);
         if (st == AFVM_OK && (cudaStreamSynchronize(s) != cudaSuccess ||
                               cudaMemcpy(out, result, sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess)) {
             cudaGetLastError();

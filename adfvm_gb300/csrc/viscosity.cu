@@ -46,7 +46,7 @@ constexpr int VT = 128;                    // threads a block of the kernels her
 // Adds the K values of every thread of the block and, in the last block of the grid to arrive,
 // the blocks' sums: true there in thread 0, with the grid's sums in out (the order of every
 // addition is fixed). partials: K x gridDim.x; arrived: zero before the first launch and after
-// each.
+// each (cleared at the start of a call).
 template <int K>
 __device__ __forceinline__ bool grid_sums(const double* v, double* partials, unsigned* arrived, double* out) {
     __shared__ double sh[K * VT];
@@ -411,13 +411,13 @@ int adjoint_viscosity_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, in
         const size_t words = 2 * (size_t)c->nC + 2 * (size_t)c->nF + 4 * 5 * n + 2 * n + 6 * n + 10 * (size_t)nb + 64 + 3 * n;
         int st = ctx_alloc(c, (void**)&c->viscWork, sizeof(double) * words);
         if (st) return st;
-        // (the arrival count; every kernel leaves it zero)
-        cudaError_t e = cudaMemsetAsync(c->viscWork, 0, sizeof(double) * 64, s);
-        if (e != cudaSuccess) return cuda_fail(c, e, "adjoint viscosity work");
     }
     double* sc = c->viscWork;                // 64 scalars: the CG's, the norm's factor, the arrival count
     double* fac = sc + 40;
     unsigned* arrived = (unsigned*)(sc + 48);
+    // (every kernel leaves the arrival count zero, unless calls on this context overlapped)
+    cudaError_t cleared = cudaMemsetAsync(arrived, 0, sizeof(unsigned), s);
+    if (cleared != cudaSuccess) return cuda_fail(c, cleared, "adjoint viscosity work");
     double* M = sc + 64;                     // nC: the viscosity before its scaling (nIC values)
     double* snd = M + c->nC;                 // nC: sound speeds
     double* DT = snd + c->nC;                // nF

@@ -433,7 +433,8 @@ int afvm_adjoint_energy(afvm_ctx* ctx, const void* rhoa, const void* rhoUa, cons
  * the array's device address (cudaGetSymbolAddress) with that device current and caches
  * it, so make that first call before any stream capture; the cached address does not
  * survive cudaDeviceReset. Calls share the array: calls that overlap on the GPU race and
- * must be ordered by the caller. Blocks until the result is in *out (host); calls no
+ * must be ordered by the caller (an overlap spoils the results of the calls in it, of no later
+ * call). Blocks until the result is in *out (host); calls no
  * allocator. */
 #define AFVM_SENSITIVITY_NOALLOC_MAX_ARRAYS 16
 int afvm_sensitivity_noalloc(int32_t device, int32_t nArrays, const double* const* grad,

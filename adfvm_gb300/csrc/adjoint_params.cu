@@ -16,6 +16,8 @@
 //   k_param_cell  cells: the 1/V of the Green-Gauss gradient and the kinetic-energy objective.
 // Every output element is written by one thread, so the sums are deterministic. FP64 contexts.
 #include <cuda_runtime.h>
+#include <algorithm>
+#include <string>
 #include "facedev.cuh"
 
 namespace afvm {
@@ -53,14 +55,44 @@ __device__ __forceinline__ void ghost_bar(const MeshDev<R>& m, const Phys& P, co
     }
 }
 
-// The FP64 pipe binds. Untaped (meshes up to the small-grid limit): about 750 FP64 instructions a
-// face; the face flux is evaluated once, into a tape in registers and local memory that its VJP
-// reads; two blocks a SM hold more of it in registers than the compiler's choice (768 -> 605 us a
-// launch of 317,955 faces). TAPED: the flux and its forward values come from k_flux, whose evaluation
-// serves k_adj_flux as well: with k_adj_flux and the evaluation 272 + 605 -> 136 + 180 + 419 us a stage (two blocks
-// a SM 426). Products on the integer pipes (soft64.cuh) gave 601 for 605: the serial chains are too long
-// for so few warps. One kernel for the face records and these gradients would take 609 + 83 us, but
-// the records' last bits would depend on whether gradients are wanted.
+// the forward values and fluxes of n faces from f0 on, as k_flux forms them for large meshes (the same
+// bits), into a tape and flux records of these faces alone
+__global__ void __launch_bounds__(FLUX_BLOCK, 3)
+    k_param_forward(const __grid_constant__ MeshDev<double> m, const __grid_constant__ Phys P,
+                    const double* __restrict__ rec, int f0, int n, int inviscid, double* __restrict__ fflux,
+                    double* __restrict__ tape) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, f = f0 + i;
+    if (i >= n) return;
+    const int kind = face_at<double>(m, f).kind;
+    if (kind == FACE_BOUNDARY) return;      // (k_param_face evaluates it)
+    double* out = fflux + (size_t)i * FREC;
+    unsigned most = 0;
+    soft_flag() = 0;
+    {
+        FaceIn<sd> in;
+        sd F[5], maxaF;
+        load_face<double>(m, rec, f, in, &most);
+        face_flux<sd>(P, kind, inviscid != 0, in, F, maxaF, TapeStore<double, sd>{tape + i, (size_t)n});
+        for (int k = 0; k < 5; k++) out[k] = raw(F[k]);
+    }
+    if (__builtin_expect(most >= SOFT_LIMIT || soft_flag() != 0, 0)) {
+        FaceIn<double> in;
+        double F[5], maxaF;
+        load_face<double>(m, rec, f, in);
+        face_flux<double>(P, kind, inviscid != 0, in, F, maxaF, TapeStore<double>{tape + i, (size_t)n});
+        for (int k = 0; k < 5; k++) out[k] = F[k];
+    }
+}
+
+// n faces from f0 on; fflux and tape (TAPED) hold these faces alone. The FP64 pipe binds. Untaped
+// (meshes up to the small-grid limit, and gradients of boundary inputs alone): about 750 FP64
+// instructions a face; the face flux is evaluated once, into a tape in registers and local memory
+// that its VJP reads; two blocks a SM hold more of it in registers than the compiler's choice (768 ->
+// 605 us a launch of 317,955 faces). TAPED: the flux and its forward values come from k_flux, whose
+// evaluation serves k_adj_flux as well: with k_adj_flux and the evaluation 272 + 605 -> 136 + 180 +
+// 419 us a stage (two blocks a SM 426). Products on the integer pipes (soft64.cuh) gave 601 for 605: the
+// serial chains are too long for so few warps. One kernel for the face records and these gradients
+// would take 609 + 83 us, but the records' last bits would depend on whether gradients are wanted.
 template <typename R, typename S, bool TAPED>
 __global__ void __launch_bounds__(FLUX_BLOCK, TAPED ? 3 : 2) k_param_face(MeshDev<R> m, Phys P, const R* __restrict__ rec, R coef,
                                                            const S* __restrict__ ar, const S* __restrict__ au,
@@ -68,9 +100,10 @@ __global__ void __launch_bounds__(FLUX_BLOCK, TAPED ? 3 : 2) k_param_face(MeshDe
                                                            const R* __restrict__ cbar, int inviscid, int dragStage,
                                                            int objStart, int objN, double obja,
                                                            const double* __restrict__ objSeed, ParamDev pd,
-                                                           const R* __restrict__ fflux, const R* __restrict__ tape) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= m.nF) return;
+                                                           int f0, int n, const R* __restrict__ fflux,
+                                                           const R* __restrict__ tape) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, f = f0 + i;
+    if (i >= n) return;
     const bool internal = f < m.nIF;
     const int kind = internal ? FACE_INTERNAL : (int)m.fkind[f - m.nIF];
     const int iP = m.own[f], iN = m.nbr[f];
@@ -97,8 +130,8 @@ __global__ void __launch_bounds__(FLUX_BLOCK, TAPED ? 3 : 2) k_param_face(MeshDe
         face_flux<R>(P, kind, inviscid != 0, in, F, maxaF);
         face_vjp<R>(P, kind, inviscid != 0, in, Fb, b, &geo);
     } else if (TAPED) {
-        for (int k = 0; k < 5; k++) F[k] = fflux[(size_t)f * FREC + k];
-        face_vjp_t<R>(P, kind, inviscid != 0, in, TapeLoad<R>{tape + f, (size_t)m.nF}, Fb, b, &geo);
+        for (int k = 0; k < 5; k++) F[k] = fflux[(size_t)i * FREC + k];
+        face_vjp_t<R>(P, kind, inviscid != 0, in, TapeLoad<R>{tape + i, (size_t)n}, Fb, b, &geo);
     } else {
         TapeLocal<R, true> t;
         face_flux<R>(P, kind, inviscid != 0, in, F, maxaF, t);
@@ -235,23 +268,47 @@ __global__ void __launch_bounds__(BLOCK) k_param_cell(MeshDev<R> m, Phys P, cons
     vol[c] += vb;
 }
 
+// whether the gradients take the faces' forward values from a tape
+static bool soft_params(const Ctx* c, const ParamDev& pd) {
+    return use_soft(c, c->nF) && (pd.areas || pd.volL || pd.volR || pd.dlt || pd.nrm || pd.du || pd.lw || pd.qw);
+}
+
+// The faces whose tape is made at a time where there is none of a whole stage: one wave of
+// k_param_face (31 MB).
+constexpr int PARAM_CHUNK = 3 * 152 * FLUX_BLOCK;
+
+int prepare_params(Ctx* c) {
+    if (c->paramChunk || !use_soft(c, c->nF)) return AFVM_OK;
+    return ctx_alloc(c, (void**)&c->paramChunk, sizeof(double) * (FREC + TAPE) * (size_t)PARAM_CHUNK);
+}
+
 bool param_tapes(Ctx* c, const ParamDev& pd, bool tape, cudaStream_t s) {
-    if (!use_soft(c, c->nF)) return false;
-    if (!pd.areas && !pd.volL && !pd.volR && !pd.dlt && !pd.nrm && !pd.du && !pd.lw && !pd.qw) return false;
+    if (!soft_params(c, pd)) return false;
     if (tape || c->paramTape) return true;
     // made with the first gradients, unless the stream is being captured: a whole step's where that
-    // takes no more than a quarter of the free memory, else one stage's
+    // takes no more than a quarter of the free memory and PARAM_TAPE_MOST, else one stage's. Without
+    // one the gradients are the same bits and take longer (an adjoint step with mesh gradients of 47^3
+    // cells: 2.58 ms, with one stage's 2.89, with none 3.41).
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     size_t free = 0, total = 0;
-    const size_t whole = sizeof(double) * (3 * FREC * (size_t)c->nF + tape_elements(c));
-    const size_t one = sizeof(double) * TAPE * (size_t)c->nF;
     if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
-        cudaMemGetInfo(&free, &total) != cudaSuccess || one > free / 4) {
+        cudaMemGetInfo(&free, &total) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    c->paramTapeWhole = whole <= free / 4;
-    return ctx_alloc(c, (void**)&c->paramTape, c->paramTapeWhole ? whole : one) == AFVM_OK;
+    const size_t most = std::min(free / 4, c->paramTapeMost);
+    const std::string err = c->err;
+    for (bool whole : {true, false}) {
+        const size_t bytes = sizeof(double) * (whole ? 3 * FREC * (size_t)c->nF + tape_elements(c) : TAPE * (size_t)c->nF);
+        if (bytes > most) continue;
+        if (ctx_alloc(c, (void**)&c->paramTape, bytes) == AFVM_OK) {
+            c->paramTapeWhole = whole;
+            return true;
+        }
+        c->paramTape = nullptr;
+        c->err = err;        // (no error of the call)
+    }
+    return false;
 }
 
 template <typename R, typename S>
@@ -261,12 +318,26 @@ void launch_param_grads(Ctx* c, const ParamDev& pd, const R* rec, R coef, const 
     const Phys& P = c->phys;
     int inviscid = (P.muModel == AFVM_MU_CONSTANT && P.mu0 == 0.0) ? 1 : 0;
     ProfScope ps(c, KID_ADJ_MISC, s);
-    int nbF = (m.nF + FLUX_BLOCK - 1) / FLUX_BLOCK;
     int drag = objectiveStage && c->objective == AFVM_OBJ_DRAG;
     const double* seed = objectiveStage ? c->objSeed : nullptr;
-    auto k = tape ? k_param_face<R, S, true> : k_param_face<R, S, false>;
-    k<<<nbF, FLUX_BLOCK, 0, s>>>(m, P, rec, coef, ar, au, ae, (const R*)c->fadj, (const R*)c->cbar, inviscid, drag,
-                                 c->objStart, c->objN, obja, seed, pd, flux, tape);
+    auto faces = [&](auto kernel, int f0, int n, const R* ff, const R* t) {
+        kernel<<<(n + FLUX_BLOCK - 1) / FLUX_BLOCK, FLUX_BLOCK, 0, s>>>(
+            m, P, rec, coef, ar, au, ae, (const R*)c->fadj, (const R*)c->cbar, inviscid, drag, c->objStart, c->objN,
+            obja, seed, pd, f0, n, ff, t);
+    };
+    if (tape) {
+        faces(k_param_face<R, S, true>, 0, m.nF, flux, tape);
+    } else if (soft_params(c, pd)) {
+        double* const t = c->paramChunk + (size_t)FREC * PARAM_CHUNK;
+        for (int f0 = 0; f0 < m.nF; f0 += PARAM_CHUNK) {
+            const int n = std::min(PARAM_CHUNK, m.nF - f0);
+            k_param_forward<<<(n + FLUX_BLOCK - 1) / FLUX_BLOCK, FLUX_BLOCK, 0, s>>>(m, P, rec, f0, n, inviscid,
+                                                                                   c->paramChunk, t);
+            faces(k_param_face<R, S, true>, f0, n, c->paramChunk, t);
+        }
+    } else {
+        faces(k_param_face<R, S, false>, 0, m.nF, nullptr, nullptr);
+    }
     if (pd.vol) {
         int ke = objectiveStage && c->objective == AFVM_OBJ_KINETIC_ENERGY;
         k_param_cell<R><<<nblocks(m.nIC), BLOCK, 0, s>>>(m, P, rec, (const R*)c->cbar, ke, obja, pd.vol);

@@ -1066,6 +1066,7 @@ int afvm_adjoint_step_params(afvm_ctx* ctx, const void* rho, const void* rhoU, c
         c->gdirn = (uint8_t*)p;
     }
     pd.gdirn = c->gdirn;
+    if ((st = prepare_params(c))) return st;
     // the outputs are the step's gradients: cleared, then summed over the three stages
     const size_t nF = c->nF, nIF = c->nIF, nIC = c->nIC;
     const std::pair<double*, size_t> outs[] = {{pd.areas, nF}, {pd.volL, nF}, {pd.volR, nIF}, {pd.wts, nF},

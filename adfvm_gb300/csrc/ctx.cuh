@@ -211,6 +211,10 @@ struct VaneDev {
     double n0, n1, n2, ptin, Tw, a, b, rw2;   // rw2 = 1 / sum_f A_f w_f
 };
 
+// the most memory a context keeps for the mesh gradients (paramTape): a whole step's tape up to about 6
+// million cells, one stage's up to 22 million
+constexpr size_t PARAM_TAPE_MOST = size_t(32) << 30;
+
 struct Ctx {
     int precision;            // AFVM_FP64 / AFVM_FP32
     int device;
@@ -248,9 +252,12 @@ struct Ctx {
     uint8_t* gdirn = nullptr;            // per ghost, the same flag (device; on first use)
     // adjoint buffers (allocated on first use)
     void* fadj = nullptr;     // nF x 40 face adjoint records
-    // for the mesh gradients (adjoint_params.cu): a step's flux records and tape, or one stage's face tape
+    // for the mesh gradients (adjoint_params.cu): a step's flux records and tape, or one stage's face tape;
+    // the flux records and tape of some faces, where there is neither
     double* paramTape = nullptr;
+    double* paramChunk = nullptr;
     bool paramTapeWhole = false;
+    size_t paramTapeMost = PARAM_TAPE_MOST;
     void* cbar = nullptr;     // nIC x 20 cell primitive/gradient adjoints
     void* a1[3] = {nullptr, nullptr, nullptr};
     void* a2[3] = {nullptr, nullptr, nullptr};
@@ -356,10 +363,11 @@ int adjoint_step_dev(Ctx* c, const S* rho, const S* rhoU, const S* rhoE, double 
 int prepare_adjoint(Ctx* c);
 // per stage of the reverse sweep, after the face records and cell sums of the stage (fadj,
 // cbar) and before the stage's cell kernel: adds the stage's share of the parameter gradients
-// tape, flux: the stage's face tape and flux records (NULL: neither)
+// tape, flux: the stage's face tape and flux records (NULL: neither). After prepare_params.
 template <typename R, typename S>
 void launch_param_grads(Ctx* c, const ParamDev& pd, const R* rec, R coef, const S* ar, const S* au, const S* ae,
                         bool objectiveStage, double obja, cudaStream_t s, const R* tape, const R* flux);
+int prepare_params(Ctx* c);
 // whether the gradients are to be formed from face tapes (tape: the step's own is given), with
 // paramTape made where it is needed
 bool param_tapes(Ctx* c, const ParamDev& pd, bool tape, cudaStream_t s);

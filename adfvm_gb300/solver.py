@@ -673,7 +673,9 @@ class RCF(object):
         forward recompute. tape: the tape_buffer() the same step filled; skips the face
         flux's re-evaluation inside the VJP. params: 'mesh' or ('BCs', field, patch, key) -
         also the gradients with respect to those parameters (afvm_adjoint_step_params, FP64
-        contexts), returned as a fifth item: a list of float64 CUDA tensors of param_shapes()."""
+        contexts), returned as a fifth item: a list of float64 CUDA tensors of param_shapes().
+        The first call for them may allocate up to 32 GiB and a quarter of the free memory (11 GB
+        at 128^3), kept until close(); the results do not depend on it."""
         torch = _torch()
         stream = L.stream_of(rho)
         if out is None:

@@ -381,7 +381,13 @@ typedef struct afvm_param_grad {
 /* afvm_adjoint_step_tape that also returns the parameter gradients described by *pg. AFVM_FP64
  * contexts (AFVM_ERR_UNSUPPORTED otherwise, and for the vane objective's heat-transfer term);
  * AFVM_ERR_BAD_ARG for a patch / field without an input (zeroGradient, cyclic, symmetryPlane,
- * or a CBC_TOTAL_PT direction that is the face normals - a mesh input). */
+ * or a CBC_TOTAL_PT direction that is the face normals - a mesh input).
+ * Memory: on meshes of more than 155,648 faces the first call allocates 31 MB, and the first one for mesh
+ * gradients that is not being captured a buffer for a step's face values besides: 1,608 bytes a face and
+ * 480 a cell (11 GB at 128^3) where that is at most a quarter of the free memory and 32 GiB, else 488
+ * bytes a face under the same limits, else none. Both are kept until afvm_ctx_destroy and counted in
+ * afvm_ctx_device_bytes. The results are the same bits with either buffer and with none; with less
+ * memory the call takes longer. */
 int afvm_adjoint_step_params(afvm_ctx* ctx, const void* rho, const void* rhoU, const void* rhoE, double dt,
                              const void* S_rho, const void* S_rhoU, const void* S_rhoE, const void* stages,
                              const void* tape, const void* rhoNa, const void* rhoUNa, const void* rhoENa,

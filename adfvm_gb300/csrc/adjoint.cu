@@ -242,7 +242,8 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 12 : 5)
 
 // The same with products, reciprocals and square roots on the integer pipes (soft64.cuh), FP64.
 // Of 323 FP64 instructions a face of the taped VJP 233 are left: 3.71 -> 2.86 ms a launch of
-// 6,340,608 faces (the FP64 pipe 84 % busy; 2.3 ms when it never waited). The forward values
+// 6,340,608 faces (the FP64 pipe 84 % busy, 232 bytes a thread spilled at 168 registers; 2.3 ms when the
+// pipe never waited). The forward values
 // come through shared memory: read from global memory where they are used, the same kernel takes
 // 3.05 ms at 168 registers and 3.07 ms at 128 (four blocks a SM). Untaped, the forward writes
 // them there instead of holding 61 values in registers: 3 x 521 -> 3 x 310 us for 317,955

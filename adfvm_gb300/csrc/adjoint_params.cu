@@ -90,9 +90,10 @@ __global__ void __launch_bounds__(FLUX_BLOCK, 3)
 // that its VJP reads; two blocks a SM hold more of it in registers than the compiler's choice (768 ->
 // 605 us a launch of 317,955 faces). TAPED: the flux and its forward values come from k_flux, whose
 // evaluation serves k_adj_flux as well: with k_adj_flux and the evaluation 272 + 605 -> 136 + 180 +
-// 419 us a stage (two blocks a SM 426). Products on the integer pipes (soft64.cuh) gave 601 for 605: the
-// serial chains are too long for so few warps. One kernel for the face records and these gradients
-// would take 609 + 83 us, but the records' last bits would depend on whether gradients are wanted.
+// 419 us a stage (two blocks a SM 426; at three, 556 bytes a thread are spilled into 740 of loads).
+// Untaped products on the integer pipes (soft64.cuh) gave 601 for 605: the serial chains are too long for
+// so few warps. One kernel for the face records and these gradients would take 609 + 83 us, but the
+// records' last bits would depend on whether gradients are wanted.
 template <typename R, typename S, bool TAPED>
 __global__ void __launch_bounds__(FLUX_BLOCK, TAPED ? 3 : 2) k_param_face(MeshDev<R> m, Phys P, const R* __restrict__ rec, R coef,
                                                            const S* __restrict__ ar, const S* __restrict__ au,

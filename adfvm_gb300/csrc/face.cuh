@@ -642,8 +642,9 @@ AFVM_HD void viscous_geo_vjp(const Phys& P, R TL, R TR, const R* UL, const R* UR
 }
 
 // VFIRST: the viscous part before the Riemann part, as FP32 and mixed contexts take them. The other
-// order holds 16 adjoints fewer across the Riemann part (the FP64 VJP spills 4 bytes a thread at 168
-// registers instead of 352); the sums of the face states' adjoints round differently.
+// order holds 16 adjoints fewer across the Riemann part (at 168 registers the taped FP64 VJP of small
+// meshes, k_adj_flux, spills 4 bytes a thread instead of 352; k_adj_flux_soft of large ones stores 232
+// and loads 244); the sums of the face states' adjoints round differently.
 template <typename R, bool VFIRST = false, typename Src, typename G = GeoNone>
 AFVM_HD void face_vjp_t(const Phys& P, int kind, bool inviscid, const FaceIn<R>& in, const Src& t, const R* Fb,
                         FaceBar<R>& o, G* geo = nullptr);

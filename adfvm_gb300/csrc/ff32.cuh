@@ -4,8 +4,8 @@
 // instruction (a conversion too) holds its pipe for 16 clocks of an SM, an FP32 one for a quarter of a
 // clock: the primitives' 21 in double kept the pipe busy for 50 to 60 % of k_prim and k_update, the
 // gradient's 40 for half of k_adj_cell2. At 128^3: the objective stage's k_adj_cell2 about 200 -> 160 us,
-// k_update 119 -> 115; k_prim stays at 72 us there (most warps hold a value that the double form has to
-// settle; without that test, 53).
+// k_update 119 -> 115; k_prim 80 -> 52 us on the benchmark's state, and 72 with or without the pairs
+// on a perturbed one, most of whose warps hold a value that the double form has to settle.
 // The sums and products are the error-free transformations of Knuth and Dekker (T. J. Dekker, A
 // floating-point technique for extending the available precision, Numer. Math. 18 (1971)): with
 // u = 2^-24 a sum of pairs below errs by at most 3 u^2 of its operands' sizes, of a pair and a float by u^2 of

@@ -323,7 +323,8 @@ __device__ __noinline__ void flux_face_again(const MeshDev<R>& m, const Phys& P,
 // pipe binds either form; of 298 FP64 instructions a face (52 DADD, 90 DMUL, 156 DFMA) 183 are
 // left (50 DADD, 133 DFMA): 3.47 -> 2.33 ms a taped launch of 6,340,608 faces, 1.85 ms when the
 // pipe never waited (it is 81 % busy: three warps a sub-partition, whose integer chains are
-// serial; 128 registers for four spill more than they hide, 2.42 ms, 255 for two 2.46).
+// serial; 168 registers spill about 300 bytes a thread into 376 of loads, 128 registers for four warps
+// spill more than they hide, 2.42 ms, 255 for two 2.46).
 template <typename R, bool TAPED, bool CFL, bool SOFT>
 __global__ void __launch_bounds__(FLUX_BLOCK, sizeof(R) == 8 ? 3 : 8)
     k_flux(const __grid_constant__ MeshDev<R> m, const __grid_constant__ Phys P, const R* __restrict__ rec,
@@ -405,8 +406,8 @@ __device__ __forceinline__ void step_end(const StepEnd& e) {
 // with a sixth warp for the CFL sum. SOFT (FP64, use_soft): the FP64 pipe binds; the gather's 30
 // products of about 105 FP64 instructions a cell go to the integer pipes (soft64.cuh; the same bits),
 // and four blocks a SM then hide their latency: 392 -> 304 us at 128^3, 171 -> 136 at 96^3, 62 -> 50 at
-// 64^3 (two blocks 322, 143, 55; three 301, 136, 54). A cell with a flux of 2^64 or more gathers again with
-// the hardware's.
+// 64^3 (two blocks 322, 143, 55; three 301, 136, 54); at 64 registers it spills 220
+// to 290 bytes a thread. A cell with a flux of 2^64 or more gathers again with the hardware's.
 template <typename R, typename S, int STAGE, bool SPLIT, bool SOFT>
 __global__ void __launch_bounds__(SPLIT ? 192 : BLOCK, SOFT ? 4 : 0)
     k_update(MeshDev<R> m, const R* __restrict__ fflux, double dtv, const double* dtp, const S* u0r, const S* u0u,

@@ -27,8 +27,8 @@
 // its 5 or 10 dot products through shared memory (about 8 FP64 instructions a warp and product
 // instead of 12 in every warp). An iteration is three kernels.
 // Vectors are interleaved, five components a cell: a neighbour's are in two sectors instead of five.
-// 262,144 cells in FP64, four iterations: 3.27 -> 0.80 ms (k_visc_cell 2.13 -> 0.30, an iteration
-// 198 -> 72 us: q = A p 57 + 10 -> 30, update 84 + 17.5 + 2 -> 31, direction 27.5 -> 11).
+// 262,144 cells in FP64, four iterations: 3.27 -> 0.89 ms (k_visc_cell 2.13 -> 0.31, an iteration
+// 198 -> 87 us: q = A p 57 + 10 -> 44, update 84 + 17.5 + 2 -> 32, direction 27.5 -> 11).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <algorithm>
